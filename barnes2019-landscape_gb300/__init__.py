@@ -378,7 +378,8 @@ class FastScape_RBP:
               "order_kernel", "erode_kernel", "accum_kernel")
 
     def phase_times(self, reset: bool = False):
-        """Device milliseconds per timer in TIMERS (fs_get_phase_times)."""
+        """Device milliseconds per timer in TIMERS (fs_get_phase_times, which
+        says what the timestep's kernels put under these names)."""
         out = np.zeros(len(self.TIMERS), np.float64)
         check(library().fs_get_phase_times(self._m, _p(out, C.c_double), int(reset)))
         return out

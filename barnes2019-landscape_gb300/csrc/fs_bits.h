@@ -133,6 +133,56 @@ FS_BITS_FN uint64_t add_pos_rn_bits(uint64_t x, uint64_t y) {
   return ((uint64_t)(ea - 1) << 52) + r;
 }
 
+// RN(x + c) for c accepted by add_pos_operand with a biased exponent of at
+// most 1900 and x > 0 in c's binade or one up to 52 above: half the steps of
+// add_pos_rn_bits. The aligned c is truncated without a sticky bit: the exact
+// sum lies in [s, s + 1), and every rounding threshold is a multiple of 2^8
+// of these units, so s rounds like the exact sum unless s is itself such a
+// multiple after bits were shifted out. Returns 0 then, and for other x (the
+// caller adds otherwise).
+FS_BITS_FN uint64_t add_const_rn_bits(uint64_t x, uint64_t c) {
+  const int ex = (int)(x >> 52), d = ex - (int)(c >> 52);
+  if ((unsigned)d > 52u) return 0;  // a negative x, Inf and NaN among them
+  constexpr uint64_t kFrac = (1ull << 52) - 1, kOne = 1ull << 52;
+  const uint64_t mc = ((c & kFrac) | kOne) << 10, sh = mc >> d;
+  const uint64_t s = (((x & kFrac) | kOne) << 10) + sh;
+  if ((s & 0xFF) == 0 && sh << d != mc) return 0;
+  const int up = (int)(s >> 63), n = 10 + up;
+  const uint64_t r = (s + ((1u << (n - 1)) - 1u) + ((uint32_t)(s >> n) & 1u)) >> n;
+  return ((uint64_t)(ex + up - 1) << 52) + r;
+}
+
+// RN(num/D) in magnitude, with q0's sign, from q0 = RN(num * R) up to sign, R =
+// RN(1/D), D >= 1: q0 is within 2^-52 (1 + 2^-52) of num/D relatively. The
+// residual |num| - |q0|*|D| is exact in integer arithmetic, in units of
+// ulp(q0)*ulp(D): r = mn*2^k - mq*md with mn, mq, md the significands
+// (implicit bit set) and k = en - eq - ed + 1075 from the biased exponents,
+// which is 52 or 53; |r| < 2.01 md < 2^55, so the difference modulo 2^64 is r
+// itself, and mn*2^k modulo 2^64 is num's low word alone, shifted. As num/D =
+// q0 + (r/md) ulp(q0) in magnitude, the correctly rounded quotient is q0 when
+// 2|r| < md, and one or two ulp further from or nearer to 0 when md < 2|r| <
+// 3md or 3md < 2|r| < 5md (away from the ends of q0's binade, where the
+// spacing changes; a quotient is never a rounding midpoint). 0 where this
+// does not decide (the caller divides).
+FS_BITS_FN uint64_t quotient_tabled_bits(uint64_t q0, uint64_t num, uint64_t D) {
+  constexpr uint64_t kMant = (1ull << 52) - 1, kHidden = 1ull << 52;
+  const int eq = (int)((uint32_t)(q0 >> 52) & 0x7FFu), en = (int)((uint32_t)(num >> 52) & 0x7FFu);
+  const int ed = (int)(uint32_t)(D >> 52);  // a negative D fails the check below
+  const int k = en - eq - ed + 1075;
+  const uint64_t m = q0 & kMant;
+  if ((unsigned)(eq - 64) > 1916u || (unsigned)(ed - 1023) > 1020u || (unsigned)(k - 52) > 1u ||
+      m - 2 > kMant - 4)
+    return 0;
+  const uint64_t md = (D & kMant) | kHidden;
+  const uint64_t top = (uint64_t)((uint32_t)num << (k - 32)) << 32;
+  const long long r = (long long)(top - (m | kHidden) * md);
+  const uint64_t a2 = (uint64_t)(r < 0 ? -r : r) << 1;
+  if (a2 < md) return q0;
+  const uint64_t n = a2 < 3 * md ? 1 : 2;
+  if (a2 == md || a2 == 3 * md || a2 >= 5 * md) return 0;
+  return r > 0 ? q0 + n : q0 - n;
+}
+
 FS_BITS_FN int clz64(uint64_t x) {
 #if defined(__CUDA_ARCH__)
   return __clzll((long long)x);

@@ -16,7 +16,7 @@
 namespace fs {
 
 // Batch-wide control block. `err` holds the first error status of the
-// current fs_step call; the words from `bar` on are reset before every
+// current fs_step call; the words from `amb` on are reset before every
 // timestep.
 struct Ctl {
   int err;                 // FS_OK or first FS_ERR_* seen by any kernel
@@ -25,22 +25,23 @@ struct Ctl {
                            // capacity was met; the timestep stopped before
                            // touching h
   int steps_done;          // timesteps completed in the current fs_step call
-  int abort_r;             // realization that raised abort_k
+  int abort_r;             // realization (of the batch) that raised abort_k
   int pad0[3];
-  unsigned long long walk_ns[3];  // accumulated walk time: ordering,
-                                  // accumulation, erosion (block 0's clock)
-  // --- reset before every timestep (from `bar` on) ---
-  unsigned int bar;        // grid-barrier arrival counter (k_order)
+  // --- reset before every timestep (from `amb` on) ---
   int amb;                 // cells queued by the receiver filter
-  unsigned int bar2;       // grid-barrier arrival counter (k_erode)
+  unsigned int bar;        // grid-barrier arrival counter (k_order)
   unsigned int bar3;       // grid-barrier arrival counter (k_accum)
+  int left;                // cells still to erode in trees that leave their
+                           // tile (k_tile_queue), or tiles finished (resident)
+  unsigned int qtail, qhead;  // pushes to and pops from the tile queue
+  int progress;            // moves now and then while resident tiles get further
 };
-constexpr size_t kCtlResetOffset = offsetof(Ctl, bar);
+constexpr size_t kCtlResetOffset = offsetof(Ctl, amb);
 constexpr size_t kCtlResetBytes = sizeof(Ctl) - kCtlResetOffset;
 constexpr size_t kCtlCallResetBytes = 5 * sizeof(int);  // err .. abort_r
 
-// Per-realization counters written by the kernels; `top` and `lvlcnt` are
-// reset before every timestep.
+// Per-realization counters of the level order; `top` and `lvlcnt` are reset
+// before every ordering.
 struct RealCtl {
   int top;                 // pits appended to level 0 (after the rings)
   int lvlcnt[3];           // rotating per-level append counters
@@ -60,20 +61,23 @@ struct RealDesc {
   double tol;
   long long tol_bits;      // bits of tol (magnitude compares as integers)
   float tol_lo_f;          // an FP32 value <= tol*(1-2^-20)
+  uint32_t tol_q_hi, tol_y_hi;  // upper words at most tol*(1-2^-8)'s and
+                                // tol*2^39's (steps surely below tol)
   float g_orth, g_diag, gmax;  // FP32 1/dr for the receiver filter
   double dr_orth, dr_diag;
   double rdr_orth_n, rdr_diag_n;  // -RN(1/dr) for the tabled receiver
                                   // slope division; 0: divide in IEEE FP64
   const double *tab;       // erosion table, kTabStride doubles per count
   int tab_cap;             // counts k < tab_cap are in the table
-  int pad;
+  int tile0;               // first of its walk tiles
+  int id;                  // its number in the batch
 };
 
 // A 2-D tile of one realization for the stencil kernels.
 struct Tile {
   int r;                   // realization
   int x0, y0;              // grid coordinates of the tile's first cell
-  int pad;
+  int ntx;                 // walk tiles: tiles per row of the realization
 };
 
 // Receiver code of an interior cell without a lower neighbour. The ABI
@@ -121,6 +125,54 @@ enum NMode : int {
   kNTwo = 2,      // pow(x,2) = x*x, pow(x,1) = x
 };
 
+// Walk tiles: the grid cut into rectangles of 64 x 32 cells from its first
+// cell on (fs_tile.cu). Every realization owns ntx*nty of them, row by row;
+// tile t's cells are numbered c = 64*y + x inside it. Cells on a tile's edge
+// that trade water with other tiles are named by their perimeter slot: 0..63
+// the top row, 64..127 the bottom row, 128..159 the left and 160..191 the
+// right column (corners belong to the rows). A tile's sinks are its cells
+// through which water of other tiles leaves it: slot s for the exit cell at
+// slot s, 192 + s for the cell above a root that the water entering at slot s
+// (and at other slots) ends in.
+constexpr int kWalkW = 64, kWalkH = 32;
+constexpr int kWalkCells = kWalkW * kWalkH;
+constexpr int kSlots = 2 * kWalkW + 2 * kWalkH;
+// Cell codes inside a tile: 0..7 the direction of a receiver inside the
+// tile, kCodeExit | direction of one outside, kCodeRoot no receiver,
+// kCodeOutside past the grid's edge.
+constexpr int kCodeRoot = 8, kCodeOutside = 9, kCodeExit = 16;
+
+struct TileBufs {
+  const Tile *tiles;       // every walk tile of the batch
+  const int32_t *list;     // the tiles of this launch (null: all, in order)
+  int n;                   // how many
+  int total;               // tiles of the batch (queue capacity)
+  const RealDesc *desc;    // every realization (not only the active ones)
+  uint8_t *code;           // [t][2048] cell codes
+  uint32_t *planes;        // [t][4][64] bit planes of the directions' three
+                           // bits and of "has a receiver", 32 cells a word
+  uint16_t *local;         // [t][2048] cells drained inside the tile
+  uint32_t *inflow;        // [t][192] cells drained from other tiles, by slot
+  unsigned long long *sink;  // [t][384] cells << 16 | edges still to come in
+  uint32_t *link;          // [t][192] slot -> sink, and that exit's target
+  uint32_t *start;         // [t][192] exits that wait for nothing
+  int32_t *nstart;         // [t] how many
+  unsigned long long *done;  // [t][32] rows of cells whose elevation is final
+  int32_t *state;          // [t] kTileQueued | kTileAgain
+  int32_t *queue;          // [total] ring of queued tiles + 1, 0 where empty
+  uint32_t *count;         // drainage count per cell (grid layout)
+};
+// Bytes of one tile in the arrays above (12 KB), before rounding.
+constexpr size_t kWalkTileBytes = kWalkCells * (1 + 2) + 256 * 4 + kSlots * (4 + 16 + 4 + 4) +
+                                  kWalkH * 8 + 4 + 4 + 4;
+// Bytes of the per-tile arrays, and their pointers inside one allocation of
+// tile_bytes(total) bytes (256-byte aligned).
+size_t tile_bytes(size_t total);
+void tile_carve(TileBufs *b, void *base, size_t total);
+// Walk tiles of realization r appended to out (capacity cap), as
+// append_tiles.
+int append_walk_tiles(int r, int W, int H, Tile *out, int cap);
+
 // Arrays indexed by position i in the level order (the reference's stack):
 //   ent[i]   cell index (local); level 0 starts with the two rings (fixed)
 //            followed by the pits of this timestep; each level lists the
@@ -155,8 +207,8 @@ struct StepArgs {
                            // launch choice)
   int erode_generic;       // 1: the reference's Newton loop literally, for
                            // every n (a test of the fast paths)
-  int stamp;               // 1: accumulate phase times into ctl->walk_ns
   unsigned long long timeout_ns;
+  TileBufs tb;
 };
 
 // Largest batch one walk launch handles.
@@ -172,34 +224,39 @@ cudaError_t launch_receivers_fast(const StepArgs &a, cudaStream_t s,
                                   const CUtensorMap *hmap = nullptr);
 bool make_receiver_map(CUtensorMap *m, const double *h, int W, int H);
 cudaError_t launch_donors_level0(const StepArgs &a, cudaStream_t s);
-// The level walk: k_order with order_bps blocks per SM (2 or 3; each has
-// its own register budget), k_accum with accum_bps, then (when a.do_erode)
-// k_erode with erode_bps blocks per SM; cooperative launches over `sms` SMs.
-cudaError_t launch_walk(const StepArgs &a, int sms, int order_bps, int accum_bps,
-                        int erode_bps, cudaStream_t s);
-cudaError_t launch_order(const StepArgs &a, int sms, int bps, cudaStream_t s);  // k_order
-cudaError_t launch_accum(const StepArgs &a, int sms, int bps, cudaStream_t s);  // k_accum
-cudaError_t launch_erode(const StepArgs &a, int sms, int bps, cudaStream_t s);  // k_erode
+// The level order: k_order and k_accum with bps blocks per SM, cooperative
+// launches over `sms` SMs.
+cudaError_t launch_order(const StepArgs &a, int sms, int bps, cudaStream_t s);
+cudaError_t launch_accum(const StepArgs &a, int sms, int bps, cudaStream_t s);
 int walk_threads();
-// k_erode: var 0 FP64 subtractions, 1 integer subtractions (n = 1, 2), 2 the
-// reference's loop literally
-const void *walk_kernel_ptr(int nmode, bool single, int var = 0);
-const void *order_kernel_ptr(bool single, int bps);     // k_order for bps 2 or 3
-const void *accum_kernel_ptr(bool single);              // k_accum
-constexpr int kAccumMaxBps = 4;                         // k_accum's register budget
+const void *order_kernel_ptr(bool single);
+const void *accum_kernel_ptr(bool single);
+constexpr int kAccumMaxBps = 4;      // k_accum's register budget
 cudaError_t prepare_walk_kernels();  // dynamic shared memory limit
-// The per-realization walk (batches of many small realizations): one CTA of
-// cta_threads(erode) threads per realization (blocks CTAs in all, looping over
-// the realizations); launch_cta_order orders and accumulates,
-// launch_cta_erode uplifts and erodes (skipped on an abort or error).
-int cta_threads(bool erode);
-const void *cta_order_ptr();
-const void *cta_erode_ptr(int nmode, int var);
-cudaError_t launch_cta_order(const StepArgs &a, int blocks, cudaStream_t s);
-cudaError_t launch_cta_erode(const StepArgs &a, int blocks, cudaStream_t s);
+// The tile walk (fs_tile.cu): drainage inside the tiles, drainage between
+// them, and the counts alone or the erosion. `resident` and `queued` are the
+// blocks that k_tile_resident and k_tile_queue can keep on the GPU at once.
+struct TileRoom {
+  int resident = 0, queued = 0;
+};
+cudaError_t launch_tile_drain(const StepArgs &a, cudaStream_t s);
+cudaError_t launch_tile_links(const StepArgs &a, cudaStream_t s);
+cudaError_t launch_tile_counts(const StepArgs &a, cudaStream_t s);
+cudaError_t launch_tile_erode(const StepArgs &a, const TileRoom &room, cudaStream_t s);
+cudaError_t launch_tile_rest(const StepArgs &a, const TileRoom &room, cudaStream_t s);
+// Raises the kernels' shared-memory limits and counts the room for the n mode
+// on a GPU of sms SMs.
+cudaError_t prepare_tile_kernels(int nmode, int sms, TileRoom *room);
+// The per-realization walk (batches of many small realizations): one CTA per
+// realization orders and accumulates, then uplifts and erodes (skipped on an
+// abort or error).
+cudaError_t launch_cta_order(const StepArgs &a, int sms, cudaStream_t s);
+cudaError_t launch_cta_erode(const StepArgs &a, int sms, cudaStream_t s);
 cudaError_t launch_check_finite(const double *h, long long n, Ctl *ctl, cudaStream_t s);
 cudaError_t launch_philox_field(double *h, int W, int H, uint64_t seed, cudaStream_t s);
 cudaError_t launch_place_rings(int32_t *ent, int W, int H, cudaStream_t s);
+// Codes of a grid without receivers: -1 on the rings, kPit inside.
+cudaError_t launch_no_receivers(int8_t *rec, int W, int H, cudaStream_t s);
 cudaError_t launch_test_wait(Ctl *ctl, int blocks, unsigned long long timeout_ns,
                              cudaStream_t s);
 
@@ -220,7 +277,7 @@ cudaError_t launch_dfs_order(const DfsArgs &d, const int32_t *lvl_host, int nlev
                              int32_t *scratch, int32_t *out, cudaStream_t s);
 
 // Host helpers shared by the entry points.
-float tol_lower_float(double tol);
+void set_tolerance(RealDesc *d, double tol);  // every field that tol fills
 // -RN(1/dr) when the tabled division covers dr (1 <= dr <= 2^60), else 0.
 double neg_recip_dr(double dr);
 int ring_cells(int W, int H);

@@ -1,23 +1,23 @@
 // fs_kernels.cu -- sm_103a kernels of the FastScape timestep, over a batch
 // of realizations (a single model is a batch of one).
 //
-// One timestep = six launches on the stream:
-//   1. k_receivers_filter  D8 steepest descent over the interior
-//      + k_receivers_fixup (fastscape_RB.cpp:160-182): FP32 proof of the
-//                          receiver, FP64 reference formula for the cells
-//                          the proof cannot settle
-//   2. k_donors_level0     donor masks (pull form of fastscape_RB.cpp:188-203)
-//                          and the level-0 frontier (fastscape_RB.cpp:221-227)
-//   3. k_order             persistent cooperative kernel: level-by-level
-//                          ordering (:229-251)
-//   4. k_accum             persistent cooperative kernel: flow accumulation
-//                          back down the levels (:262-279); uplifts the pits
-//   5. k_erode             persistent cooperative kernel: uplift (:285-296)
-//                          and the implicit erosion solved upward from base
-//                          level (:306-328, in the level order of
-//                          fastscape_RB+P.cpp:319-350).
-//   In the three walk kernels all realizations walk their levels in lock
-//   step, so one grid barrier per level serves the whole batch.
+// A timestep starts with k_receivers_filter + k_receivers_fixup: D8 steepest
+// descent over the interior (fastscape_RB.cpp:160-182), an FP32 proof of the
+// receiver and the FP64 reference formula for the cells the proof cannot
+// settle. Its other kernels, from the receivers on, are the tile walk
+// (fs_tile.cu).
+//
+// For callers that ask for the drainage network -- levels, donor masks, the
+// depth-first order -- the reference's level order is built from a timestep's
+// receivers:
+//   k_donors_level0  donor masks (pull form of fastscape_RB.cpp:188-203) and
+//                    the level-0 frontier (fastscape_RB.cpp:221-227)
+//   k_order          persistent cooperative kernel: level-by-level ordering
+//                    (:229-251)
+//   k_accum          persistent cooperative kernel: flow accumulation back
+//                    down the levels (:262-279), by position in the order
+//   All realizations walk their levels in lock step, so one grid barrier per
+//   level serves the whole batch.
 //
 // Floating point follows the reference's operation order exactly; the whole
 // file is compiled with -fmad=false so no multiply-add is contracted, every
@@ -33,124 +33,18 @@
 
 #include "fastscape_gb300.h"
 #include "fs_bits.h"
+#include "fs_device.h"
 #include "fs_internal.h"
 
 namespace fs {
 
 namespace {
 
-constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWalkThreads = 512;
 constexpr int kWalkWarps = kWalkThreads / 32;
 constexpr int kPer = 8;   // entries per thread per expansion chunk (measured best of 4..16)
 constexpr int kLevelCache = 2048;  // level offsets a single grid's walk keeps in shared memory
 constexpr int kChunk = kPer * kWalkThreads;
-constexpr int kNewtonMaxIt = 1000;
-
-__device__ __forceinline__ unsigned long long globaltimer_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ int ld_volatile_i32(const int *p) {
-  return *reinterpret_cast<const volatile int *>(p);
-}
-
-__device__ __forceinline__ void raise_err(Ctl *ctl, int code, int phase) {
-  if (atomicCAS(&ctl->err, 0, code) == 0) ctl->err_detail = phase;
-}
-
-__device__ __forceinline__ bool stopped(const Ctl *ctl) {
-  return (ld_volatile_i32(&ctl->err) | ld_volatile_i32(&ctl->abort_k)) != 0;
-}
-
-__device__ __forceinline__ void red_release_add_u32(unsigned *p, unsigned v) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Grid-wide barrier of a cooperative launch. The arrival counter only grows
-// during a launch (reset by the host before it), so barrier number `epoch`
-// completes when bar reaches epoch*gridDim.x. Arrival: the block barrier
-// orders the block's writes before thread 0's release reduction; wait:
-// thread 0's acquire loads see every block's release, and the closing block
-// barrier orders the rest of the block after them (the release/acquire
-// pattern of the CUTLASS grid barrier). Every wait is bounded by
-// `timeout_ns` of wall time; on timeout, or when another block has raised
-// an error (the error word is polled every 16 spins), it returns false and
-// the caller leaves the kernel.
-__device__ bool grid_barrier(Ctl *ctl, unsigned *bar, unsigned &epoch,
-                             unsigned long long timeout_ns) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ++epoch;
-    const unsigned target = epoch * gridDim.x;
-    red_release_add_u32(bar, 1u);
-    int ok = 1;
-    const unsigned long long t0 = globaltimer_ns();
-    unsigned spins = 0;
-    while (ld_acquire_u32(bar) < target) {
-      ++spins;
-      if ((spins & 15u) == 0 && ld_volatile_i32(&ctl->err) != 0) { ok = 0; break; }
-      if ((spins & 255u) == 0 && globaltimer_ns() - t0 > timeout_ns) {
-        raise_err(ctl, FS_ERR_TIMEOUT, kPhaseBarrier);
-        ok = 0;
-        break;
-      }
-      __nanosleep(64);
-    }
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
-// nshift[k] (fastscape_RB.cpp:137) for a run-time k without a local array:
-// dx+1 and dy+1 of the 8 directions packed two bits per direction
-// (W, NW, N, NE, E, SE, S, SW).
-__device__ __forceinline__ int nbr_off(int k, int W) {
-  const int dx = ((0x1A90 >> (2 * k)) & 3) - 1;
-  const int dy = ((0xA901 >> (2 * k)) & 3) - 1;
-  return dy * W + dx;
-}
-
-// Exclusive block scan of one int per thread; t is the thread's linear index
-// in the block and nthreads the block size (a multiple of 32, at most 1024).
-// Returns the prefix and the block total.
-__device__ __forceinline__ int block_excl_scan(int v, int &total, int t, int nthreads) {
-  __shared__ int s_w[32];
-  const int lane = t & 31, wid = t >> 5;
-  const int nw = nthreads >> 5;
-  int incl = v;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const int x = __shfl_up_sync(kFull, incl, d);
-    if (lane >= d) incl += x;
-  }
-  if (lane == 31) s_w[wid] = incl;
-  __syncthreads();
-  if (wid == 0) {
-    int w = lane < nw ? s_w[lane] : 0;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int x = __shfl_up_sync(kFull, w, d);
-      if (lane >= d) w += x;
-    }
-    if (lane < nw) s_w[lane] = w;  // inclusive warp prefix
-  }
-  __syncthreads();
-  total = s_w[nw - 1];
-  const int before = wid ? s_w[wid - 1] : 0;
-  __syncthreads();  // s_w may be reused by the caller's next scan
-  return before + incl - v;
-}
 
 // Exclusive prefix over realizations of count(r) into s_pre[0..n]; the walk
 // kernel's block-wide view of how a level's work splits across the batch.
@@ -181,136 +75,6 @@ __device__ __forceinline__ int find_real(const int *s_pre, int n, int g) {
     if (s_pre[mid] <= g) lo = mid; else hi = mid;
   }
   return lo;
-}
-
-__device__ __forceinline__ long long abs_bits(double x) {
-  return __double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll;
-}
-
-// FP64 add / multiply of bit patterns held in integer registers. Keeping
-// elevations as integers between the FP64 instructions avoids the FP64
-// moves the compiler otherwise emits for merges, selects and negations of
-// doubles (each an instruction on this part's narrow FP64 pipe).
-__device__ __forceinline__ uint64_t fadd_bits(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("{\n\t.reg .f64 x, y;\n\tmov.b64 x, %1;\n\tmov.b64 y, %2;\n\t"
-      "add.rn.f64 x, x, y;\n\tmov.b64 %0, x;\n\t}"
-      : "=l"(r)
-      : "l"(a), "l"(b));
-  return r;
-}
-
-__device__ __forceinline__ uint64_t fmul_bits(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("{\n\t.reg .f64 x, y;\n\tmov.b64 x, %1;\n\tmov.b64 y, %2;\n\t"
-      "mul.rn.f64 x, x, y;\n\tmov.b64 %0, x;\n\t}"
-      : "=l"(r)
-      : "l"(a), "l"(b));
-  return r;
-}
-
-constexpr uint64_t kSignBit = 0x8000000000000000ull;
-
-// FP64 addition in a branch taken by few cells: volatile, so that the
-// compiler does not execute it speculatively for the others.
-__device__ __forceinline__ uint64_t fadd_bits_volatile(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm volatile(
-      "{\n\t.reg .f64 x, y;\n\tmov.b64 x, %1;\n\tmov.b64 y, %2;\n\t"
-      "add.rn.f64 x, x, y;\n\tmov.b64 %0, x;\n\t}"
-      : "=l"(r)
-      : "l"(a), "l"(b));
-  return r;
-}
-
-// The erosion's FP64 pipe is its bottleneck while its integer pipes idle, so
-// some of its additions run in integer arithmetic (fs_bits.h, each
-// bit-identical to the hardware's RN operation on the operands it accepts;
-// the rest take the FP64 addition).
-//
-// The uplift h + U*dt of an eroded cell: two positive normal operands (every
-// cell of a landscape above base level). Off the cell's critical path (it
-// does not wait for the receiver's elevation), so always worth it.
-__device__ __forceinline__ uint64_t uplift_bits(uint64_t h, uint64_t udt) {
-  if (add_pos_operand(h) && add_pos_operand(udt)) return add_pos_rn_bits(h, udt);
-  return fadd_bits_volatile(h, udt);
-}
-
-// RN(x - y) of a cell's and its receiver's elevation: the exact integer
-// difference when y >= x/2 (sub_near_bits), else in FP64.
-__device__ __forceinline__ uint64_t sub_near(uint64_t x, uint64_t y) {
-  if (add_pos_operand(x) && add_pos_operand(y) && x > y) {
-    const uint64_t r = sub_near_bits(x, y);
-    if (r) return r;
-  }
-  return fadd_bits_volatile(x, y ^ kSignBit);
-}
-
-// RN(x - y) of an elevation and its erosion: in integer arithmetic when y's
-// exponent is at least 2 below x's (sub_far_bits), else in FP64.
-__device__ __forceinline__ uint64_t sub_far(uint64_t x, uint64_t y) {
-  if (add_pos_operand(x) && add_pos_operand(y)) {
-    const uint64_t r = sub_far_bits(x, y);
-    if (r) return r;
-  }
-  return fadd_bits_volatile(x, y ^ kSignBit);
-}
-
-// RN(x - y) for any two elevations: the exact integer difference when both
-// are positive normal and within a factor 2 of each other (Sterbenz), else
-// in FP64.
-__device__ __forceinline__ uint64_t sub_sterbenz(uint64_t x, uint64_t y) {
-  if (add_pos_operand(x) && add_pos_operand(y) && x != y) {
-    const bool gt = x > y;
-    const uint64_t r = sub_near_bits(gt ? x : y, gt ? y : x);
-    if (r) return gt ? r : (r ^ kSignBit);
-  }
-  return fadd_bits_volatile(x, y ^ kSignBit);
-}
-
-// -RN(num/D) on bit patterns, given Rn = -R, R = RN(1/D), in one FP64
-// operation. q0n = RN(num*Rn) = -RN(num*R) (RN is symmetric), within
-// 2^-52 (1 + 2^-52) of num/D relatively when num, q0, D and 1/D are normal.
-// The residual |num| - |q0|*|D| is then exact in integer arithmetic, in
-// units of ulp(q0)*ulp(D): r = mn*2^k - mq*mD with mn, mq, mD the
-// significands (implicit bit set) and k = en - eq - eD + 1075 from the
-// biased exponents; |r| < 2.01 mD < 2^55, so the difference taken modulo
-// 2^64 (the low halves of the 106-bit products) is r itself. In magnitude
-// num/D = q0 + (r/mD) ulp(q0), so the correctly rounded quotient is q0 when
-// 2|r| < mD and q0 one ulp further from or nearer to 0 when mD < 2|r| < 3mD
-// (q0 not a power of two, so the spacing is ulp(q0) on both sides; a
-// quotient is never a rounding midpoint, and the equalities fall back).
-// tests/native/division_check.cpp replays this on the host against the
-// IEEE division, near rounding midpoints included. It replaces Markstein's
-// correction q1 = RN(q0 + r0*R) with r0 = num - q0*D by a fused
-// multiply-add (P. Markstein, IBM J. Res. Dev. 34(1), 1990), which cost two
-// more FP64 operations on the erosion's FP64 pipe. Anything else takes the
-// IEEE division, volatile PTX in a branch; the numerator and result stay in
-// integer registers.
-__device__ __forceinline__ uint64_t neg_div_rn_bits(uint64_t numb, double D, double Rn) {
-  constexpr uint64_t kMant = (1ull << 52) - 1, kHidden = 1ull << 52;
-  const uint64_t q0b = (uint64_t)__double_as_longlong(__longlong_as_double(numb) * Rn);
-  const uint64_t Db = (uint64_t)__double_as_longlong(D);
-  const int eq = (int)((q0b << 1) >> 53);
-  const int en = (int)((numb << 1) >> 53);
-  const int ed = (int)((Db << 1) >> 53);
-  const int k = en - eq - ed + 1075;
-  if ((unsigned)(eq - 64) <= 1980u - 64u && (unsigned)(en - 1) <= 2045u &&
-      (unsigned)(ed - 1) <= 2043u && (unsigned)(k - 48) <= 12u && (q0b << 12) != 0) {
-    const uint64_t mq = (q0b & kMant) | kHidden, mn = (numb & kMant) | kHidden,
-                   md = (Db & kMant) | kHidden;
-    const long long r = (long long)((mn << k) - mq * md);
-    const uint64_t a2 = (uint64_t)(r < 0 ? -r : r) << 1;
-    if (a2 < md) return q0b;
-    if (a2 > md && a2 < 3 * md) return r > 0 ? q0b + 1 : q0b - 1;
-  }
-  uint64_t r;
-  asm volatile(
-      "{\n\t.reg .f64 x, y;\n\tmov.b64 x, %1;\n\tmov.b64 y, %2;\n\t"
-      "div.rn.f64 x, x, y;\n\tmov.b64 %0, x;\n\t}"
-      : "=l"(r)
-      : "l"(numb), "l"(Db));
-  return r ^ kSignBit;
 }
 
 // ---------------------------------------------------------------------------
@@ -814,283 +578,6 @@ __global__ void __launch_bounds__(256) k_donors_level0(StepArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// 3. Erosion of one cell and the division it needs.
-// ---------------------------------------------------------------------------
-
-// Correctly rounded num/D for D > 0 given R = RN(1/D), without the FP64
-// divide routine: Markstein's correction q1 = q0 + (num - q0*D)*R with
-// fused multiply-adds (P. Markstein, IBM J. Res. Dev. 34(1), 1990), then an
-// exact check of the remainder r1 = num - q1*D: q1 is accepted only if
-// |r1| < D*ulp(q1)/2 (then |num/D - q1| < ulp(q1)/2, so q1 = RN(num/D)),
-// q1 is not a power of two (where the spacing below halves) and its
-// exponent is far from the subnormal/overflow range. Anything else -- zero
-// numerators included -- takes the IEEE division. 4 FP64 operations against
-// ~7.5 for the divide routine on this part.
-__device__ __forceinline__ double div_rn(double num, double D, double R) {
-  const double q0 = num * R;
-  const double r0 = fma(-q0, D, num);
-  const double q1 = fma(r0, R, q0);
-  const double r1 = fma(-q1, D, num);
-  const long long qb = abs_bits(q1);
-  const int e = (int)(qb >> 52);
-  if (e >= 64 && e <= 1980 && (qb & 0x000FFFFFFFFFFFFFll) != 0) {
-    const long long thr = __double_as_longlong(D) + ((long long)(e - 1076) << 52);
-    if (abs_bits(r1) < thr) return q1;
-  }
-  return num / D;
-}
-
-// pow(x, n) and pow(x, n-1) for the Newton update of fastscape_RB.cpp:322.
-template <int NMODE>
-__device__ __forceinline__ void powers(double x, double neq, double &pn, double &pn1) {
-  if (NMODE == kNOne) {
-    pn = x;
-    pn1 = 1.0;
-  } else if (NMODE == kNTwo) {
-    pn = x * x;
-    pn1 = x;
-  } else {
-    pn = pow(x, neq);
-    pn1 = pow(x, neq - 1.0);
-  }
-}
-
-// The fields of a table record the n = 1 erosion reads up front.
-struct TabN1 {
-  uint64_t fact, D, Rn;
-};
-
-__device__ __forceinline__ TabN1 load_tab_n1(const unsigned long long *Tb) {
-  return TabN1{__ldg(Tb + 0), __ldg(Tb + 1), __ldg(Tb + 3)};
-}
-
-// True when |RN(x - y)| <= tol is proven for x = RN(y - q), y the previous
-// iterate and qn = -q: |RN(x - y)| <= (|q| + 2^-51(|y|+|q|))(1+2^-53), and
-// an FP32 test on truncated magnitudes (each within 2^-23 relative, flushed
-// below 2^-126) with 2^-21 of slack proves it for almost every cell without
-// the subtraction.
-__device__ __forceinline__ bool step_below_tol(uint64_t qn, uint64_t y, const RealDesc &d) {
-  const float qf = fabsf(trunc_bits_to_float(qn));
-  const float yf = fabsf(trunc_bits_to_float(y));
-  return qf * (1.f + 0x1p-21f) + yf * 0x1p-48f <= d.tol_lo_f;
-}
-
-// RN(x + y), y = -q with |q| far below x > 0 (a Newton correction): in
-// integer arithmetic when the operands allow, else in FP64.
-__device__ __forceinline__ uint64_t add_correction(uint64_t x, uint64_t y) {
-  return (y & kSignBit) ? sub_far(x, y ^ kSignBit) : uplift_bits(x, y);
-}
-
-// RN(x / y) of bit patterns on the FP64 pipe.
-// IEEE division in a branch taken by few cells (volatile: not executed
-// speculatively for the others).
-__device__ __forceinline__ uint64_t fdiv_bits_volatile(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm volatile(
-      "{\n\t.reg .f64 x, y;\n\tmov.b64 x, %1;\n\tmov.b64 y, %2;\n\t"
-      "div.rn.f64 x, x, y;\n\tmov.b64 %0, x;\n\t}"
-      : "=l"(r)
-      : "l"(a), "l"(b));
-  return r;
-}
-
-__device__ __forceinline__ uint64_t ffma_bits(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("{\n\t.reg .f64 x, y, z;\n\tmov.b64 x, %1;\n\tmov.b64 y, %2;\n\tmov.b64 z, %3;\n\t"
-      "fma.rn.f64 x, x, y, z;\n\tmov.b64 %0, x;\n\t}"
-      : "=l"(r)
-      : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
-// RN(num/den) on bit patterns for a denominator with no tabled reciprocal
-// (the n = 2 erosion's), in three FP64 operations: the IEEE FP32 reciprocal
-// of |den| truncated to FP32 (within 1.5*2^-23 of 1/|den|), one Newton step
-// r1 = r0 + r0*(1 - |den|*r0) by fused multiply-adds (within ~2^-44.8),
-// q0 = RN(|num|*r1) (within ~2^8.2 ulp of the quotient), and the rounding
-// from the exact integer residual (round_quotient_bits, fs_bits.h). Newton's
-// iteration for the reciprocal and the residual check are the published
-// methods (e.g. P. Markstein, IBM J. Res. Dev. 34(1), 1990);
-// tests/native/division_check.cpp replays the sequence on the host against
-// the IEEE division. Operands outside [2^-99, 2^102) and the rare cases the
-// rounding leaves open take the IEEE division.
-__device__ __forceinline__ uint64_t fdiv_rn_bits(uint64_t nb, uint64_t db) {
-  const uint64_t an = nb & ~kSignBit, ad = db & ~kSignBit;
-  if ((unsigned)((int)(an >> 52) - 924) <= 200u && (unsigned)((int)(ad >> 52) - 924) <= 200u) {
-    const uint32_t rb = __float_as_uint(__frcp_rn(trunc_bits_to_float(ad)));
-    // widen the positive normal FP32 reciprocal to FP64 bits
-    const uint64_t r0 = ((uint64_t)((rb >> 23) + 896) << 52) | ((uint64_t)(rb & 0x7FFFFFu) << 29);
-    const uint64_t e = ffma_bits(ad ^ kSignBit, r0, 0x3FF0000000000000ull);  // 1 - |den| r0
-    const uint64_t r1 = ffma_bits(r0, e, r0);
-    const uint64_t q = round_quotient_bits(an, ad, fmul_bits(an, r1));
-    if (q) return q | ((nb ^ db) & kSignBit);
-  }
-  return fdiv_bits_volatile(nb, db);
-}
-
-// RN(x - y) for any operands: in integer arithmetic when both are positive
-// normal (sub_near_bits within a factor 2, sub_far_bits from an exponent gap
-// of 2) or x is positive and y negative (add_pos_rn_bits), else in FP64.
-__device__ __forceinline__ uint64_t sub_gen(uint64_t x, uint64_t y) {
-  if (add_pos_operand(x)) {
-    if (add_pos_operand(y)) {
-      if (x != y) {
-        const bool gt = x > y;
-        const uint64_t hi = gt ? x : y, lo = gt ? y : x;
-        const uint64_t r = ((int)(hi >> 52) - (int)(lo >> 52) >= 2) ? sub_far_bits(hi, lo)
-                                                                     : sub_near_bits(hi, lo);
-        if (r) return gt ? r : (r ^ kSignBit);
-      }
-    } else if (add_pos_operand(y ^ kSignBit)) {
-      return add_pos_rn_bits(x, y ^ kSignBit);
-    }
-  }
-  return fadd_bits_volatile(x, y ^ kSignBit);
-}
-
-// Erosion of one cell for n = 2 (fastscape_RB.cpp:315-326; pow(x,2) as x*x,
-// pow(x,1) = x) on bit patterns, iterate by iterate in the reference's
-// operation order: x' = RN(x - RN(num/den)) with
-//   num = RN(RN(x - h0) + RN(fact*RN(RN(x-hn)^2))),
-//   den = RN(1 + RN(RN(fact*n)*RN(x-hn))),
-// RN(fact*n) hoisted (the reference's grouping), the first iterate's
-// x - h0 = +0 dropped, and |x' - x| <= tol proven in FP32 for most
-// iterates without the subtraction. With ISUB the subtractions run in
-// integer arithmetic.
-template <bool ISUB>
-__device__ __forceinline__ uint64_t erode_cell_n2(const RealDesc &d, double neq, Ctl *ctl,
-                                                  uint64_t factb, uint64_t h0, uint64_t hn) {
-  auto sub = [](uint64_t x, uint64_t y) { return ISUB ? sub_gen(x, y) : fadd_bits(x, y ^ kSignBit); };
-  constexpr uint64_t kOne = 0x3FF0000000000000ull;
-  const uint64_t fact2 = fmul_bits(factb, (uint64_t)__double_as_longlong(neq));
-  uint64_t x = h0;
-  for (int it = 1;; ++it) {
-    const uint64_t dx = sub(x, hn);
-    const uint64_t fpn = fmul_bits(factb, fmul_bits(dx, dx));
-    uint64_t num;
-    if (it == 1) {
-      num = (fpn << 1) == 0 ? 0 : fpn;  // RN(+0 + fpn)
-    } else {
-      const uint64_t a = sub(x, h0);
-      num = ISUB ? sub_gen(fpn, a ^ kSignBit) : fadd_bits(a, fpn);
-    }
-    const uint64_t den = fadd_bits(kOne, fmul_bits(fact2, dx));
-    const uint64_t q = fdiv_rn_bits(num, den);
-    const uint64_t xn = sub(x, q);
-    if (step_below_tol(q ^ kSignBit, x, d)) return xn;
-    const uint64_t df = sub(xn, x);
-    x = xn;
-    // fabs(diff) > tol as an integer compare (a NaN diff stops the loop)
-    const long long m = (long long)(df & ~kSignBit);
-    if (!(m > d.tol_bits && m <= 0x7FF0000000000000ll)) return x;
-    if (it >= kNewtonMaxIt) {
-      raise_err(ctl, FS_ERR_NEWTON, kPhaseErode);
-      return x;
-    }
-  }
-}
-
-// Erosion of one cell for n = 1 (fastscape_RB.cpp:315-326) on bit
-// patterns: h0 the uplifted elevation, hn the receiver's final elevation,
-// t the table record of the cell's drainage count and direction class
-// (fact, D = 1 + fact, -1/D; Tb the record itself for 1/D).
-//
-// The reference's loop for n = 1 (pow(x,1) = x, pow(x,0) = 1):
-//   x' = RN(x - RN(RN(RN(x - h0) + RN(fact*RN(x - hn))) / D)),
-//   stop when |RN(x' - x)| <= tol.
-// First iterate (x = h0): RN(h0 - h0) = +0, so x1 = RN(h0 - RN(RN(fact*
-// RN(h0-hn)) / D)). Cells whose erosion exceeds tol take a second iterate,
-// unrolled here too; its residual num2 is often exactly 0 (then x2 = x1).
-// Rarer third iterates follow the generic loop. With ISUB the subtractions
-// of elevations run in integer arithmetic: that relieves the FP64 pipe but
-// lengthens the cell's dependency chain after the receiver's elevation
-// arrives, which pays where the pipe, not latency, limits the erosion (the
-// autotuner decides per workload).
-template <bool ISUB>
-__device__ __forceinline__ uint64_t erode_cell_n1(const RealDesc &d, Ctl *ctl,
-                                                  const unsigned long long *Tb, TabN1 t,
-                                                  uint64_t h0, uint64_t hn) {
-  const uint64_t factb = t.fact;
-  const double D = __longlong_as_double(t.D), Rn = __longlong_as_double(t.Rn);
-  const uint64_t dh = ISUB ? sub_near(h0, hn) : fadd_bits(h0, hn ^ kSignBit);
-  const uint64_t num = fmul_bits(factb, dh);
-  const uint64_t qn = neg_div_rn_bits(num, D, Rn);  // -q
-  const uint64_t x1 = ISUB ? sub_far(h0, qn ^ kSignBit) : fadd_bits(h0, qn);
-  if (step_below_tol(qn, h0, d)) return x1;
-  // diff = RN(x1 - h0); |diff| > tol as an integer compare of the
-  // magnitudes' bits (a NaN diff stops the loop, as fabs(NaN) > tol is false)
-  const uint64_t a = ISUB ? sub_sterbenz(x1, h0) : fadd_bits(x1, h0 ^ kSignBit);
-  auto more = [&](uint64_t df) {
-    const long long m = (long long)(df & ~kSignBit);
-    return m > d.tol_bits && m <= 0x7FF0000000000000ll;
-  };
-  if (!more(a)) return x1;
-  // second iterate: num2 = RN(a + RN(fact * RN(x1 - hn)))
-  const uint64_t b = ISUB ? sub_sterbenz(x1, hn) : fadd_bits(x1, hn ^ kSignBit);
-  const uint64_t c = fmul_bits(factb, b);
-  const uint64_t num2 = ISUB ? sub_sterbenz(c, a ^ kSignBit) : fadd_bits(a, c);
-  if ((num2 << 1) == 0) return x1;  // RN(0/D) = +0 and x1 - 0 = x1: diff = 0
-  // The correction is a residual of x1's rounding: x2 is x1 or a neighbour,
-  // decided from an FP32 estimate of the quotient (newton_step_in_spacing),
-  // and a step of at most one spacing <= tol ends the loop.
-  if (add_pos_operand(x1)) {
-    const float qe = __fdividef(fabsf(trunc_bits_to_float(num2)), trunc_bits_to_float(t.D));
-    int step;
-    float ulp;
-    if (newton_step_in_spacing(num2, t.D, x1, qe, &step, &ulp) && ulp <= d.tol_lo_f)
-      return x1 + (uint64_t)(int64_t)step;
-  }
-  const uint64_t q2n = neg_div_rn_bits(num2, D, Rn);
-  const uint64_t x2 = ISUB ? add_correction(x1, q2n) : fadd_bits(x1, q2n);
-  if (step_below_tol(q2n, x1, d)) return x2;
-  // third and later iterates: the reference's loop in FP64
-  const double R = __longlong_as_double(__ldg(Tb + 2));
-  const double fact = __longlong_as_double(factb), h0d = __longlong_as_double(h0),
-               hnd = __longlong_as_double(hn);
-  double x = __longlong_as_double(x2);
-  double diff = x - __longlong_as_double(x1), hp = x;
-  int it = 2;
-  while (more((uint64_t)__double_as_longlong(diff))) {
-    const double n3 = (x - h0d) + fact * (x - hnd);
-    x -= div_rn(n3, D, R);
-    diff = x - hp;
-    hp = x;
-    if (++it >= kNewtonMaxIt) {
-      raise_err(ctl, FS_ERR_NEWTON, kPhaseErode);
-      break;
-    }
-  }
-  return (uint64_t)__double_as_longlong(x);
-}
-
-// Erosion of one cell for n != 1: fastscape_RB.cpp:315-326 with h0 the
-// uplifted elevation, hn the receiver's final elevation and T the table
-// record of the cell's drainage count and direction class (T[0] = fact).
-template <int NMODE>
-__device__ __forceinline__ double erode_cell(const RealDesc &d, double neq, Ctl *ctl,
-                                             const double *T, double h0, double hn) {
-  const double fact = T[0];
-  double hnew, hp, diff;
-  int it;
-  hnew = h0;
-  hp = h0;
-  diff = 2 * d.tol;
-  it = 0;
-  while (fabs(diff) > d.tol) {
-    double pn, pn1;
-    powers<NMODE>(hnew - hn, neq, pn, pn1);
-    hnew -= (hnew - h0 + fact * pn) / (1. + fact * neq * pn1);
-    diff = hnew - hp;
-    hp = hnew;
-    if (++it >= kNewtonMaxIt) {
-      raise_err(ctl, FS_ERR_NEWTON, kPhaseErode);
-      break;
-    }
-  }
-  return hnew;
-}
-
-// ---------------------------------------------------------------------------
 // 4. Persistent level walker (cooperative launch).
 //
 // The ordering is kept as arrays indexed by position in the level order
@@ -1123,15 +610,6 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_order(StepArgs a) {
   auto real_of = [&](int g) -> int { return SINGLE ? 0 : find_real(s_pre, nreal, g); };
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const bool stamp = a.stamp && tid == 0;
-  unsigned long long t_prev = stamp ? globaltimer_ns() : 0;
-  auto lap = [&](int slot) {
-    if (stamp) {
-      const unsigned long long t = globaltimer_ns();
-      atomicAdd(&ctl->walk_ns[slot], t - t_prev);
-      t_prev = t;
-    }
-  };
 
   // ---- ordering: fastscape_RB.cpp:229-251 -------------------------------
   // Level k+1 = the donors of level k. A block expands a chunk of kChunk
@@ -1323,7 +801,6 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_order(StepArgs a) {
       return;
     }
   }
-  lap(0);
 }
 
 // Accumulation (fastscape_RB.cpp:262-279) level by level back down to base
@@ -1350,8 +827,6 @@ __global__ void __launch_bounds__(kWalkThreads, 4) k_accum(StepArgs a) {
   const int nthreads = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   const int warp_global = tid >> 5, nwarps = nthreads >> 5;
-  const bool stamp = a.stamp && tid == 0;
-  const unsigned long long t_start = stamp ? globaltimer_ns() : 0;
   if (threadIdx.x == 0) s_maxlev = 0;
   __syncthreads();
   for (int r = threadIdx.x; r < nreal; r += kWalkThreads) {
@@ -1472,9 +947,6 @@ __global__ void __launch_bounds__(kWalkThreads, 4) k_accum(StepArgs a) {
           if (ok[u]) {
             const RealDesc &d = desc(rr[u]);
             atomicAdd(&a.acc[d.off + pp[u]], v[u]);
-            if (a.do_erode && v[u] >= (uint32_t)d.tab_cap) {
-              if (atomicMax(&ctl->abort_k, (int)v[u]) < (int)v[u]) ctl->abort_r = rr[u];
-            }
           }
           continue;
         }
@@ -1499,236 +971,22 @@ __global__ void __launch_bounds__(kWalkThreads, 4) k_accum(StepArgs a) {
         if (ok[u]) {
           const RealDesc &d = desc(rr[u]);
           if (tail) atomicAdd(&a.acc[d.off + p], run);
-          if (a.do_erode && v[u] >= (uint32_t)d.tab_cap) {
-            if (atomicMax(&ctl->abort_k, (int)v[u]) < (int)v[u]) ctl->abort_r = rr[u];
-          }
         }
       }
     }
     if (Lv > 1) ngroups = level_groups(Lv - 1);
     if (!grid_barrier(ctl, &ctl->bar3, epoch, a.timeout_ns)) return;
   }
-  // Level 0: counts final. With no table exceeded, uplift the pits (level 0
-  // past the rings; fastscape_RB.cpp:291-295) -- the erosion kernel reads
-  // them after the kernel boundary.
-  if (a.do_erode && ld_volatile_i32(&ctl->abort_k) == 0) {
-    __syncthreads();  // every warp is done with the last level's ranges
-    for (int r = threadIdx.x; r < nreal; r += kWalkThreads) {
-      s_lo[r] = desc(r).nring;
-      s_hi[r] = __ldcg(&a.lvl_off[desc(r).lvl_base + 1]);
-    }
-    __syncthreads();
-    const int np = block_prefix(nreal, [&](int r) { return s_hi[r] - s_lo[r]; }, s_pre);
-    for (int g = tid; g < np; g += nthreads) {
-      const int r = real_of(g);
-      const RealDesc &d = desc(r);
-      unsigned long long *hh = reinterpret_cast<unsigned long long *>(a.h + d.off);
-      const int c = __ldcg(&a.ent[d.off + s_lo[r] + (g - s_pre[r])]);
-      hh[c] = fadd_bits(__ldcg(&hh[c]), (uint64_t)__double_as_longlong(d.u_dt));
-    }
-  }
-  if (stamp) atomicAdd(&ctl->walk_ns[1], globaltimer_ns() - t_start);
-}
-
-// Uplift and erosion (fastscape_RB.cpp:285-296, :306-328) level by level
-// from base level, after k_order has placed the levels and the drainage
-// counts (and uplifted the pits). A kernel of its own: the ordering and
-// accumulation run with more resident threads than the register-hungry FP64
-// erosion allows.
-// VAR 0: subtractions of elevations on the FP64 pipe; 1: in integer
-// arithmetic (n = 1, 2); 2: the reference's Newton loop literally, for every
-// n (a test of the fast paths).
-template <int NMODE, bool SINGLE, int VAR>
-__global__ void __launch_bounds__(kWalkThreads, 2) k_erode(StepArgs a) {
-  constexpr bool ISUB = VAR == 1, GENERIC = VAR == 2;
-  extern __shared__ int smem[];
-  const int nreal = a.nreal;
-  int *s_lo = smem;
-  int *s_hi = s_lo + nreal;
-  int *s_nlev = s_hi + nreal;
-  int *s_pre = s_nlev + nreal;
-  __shared__ int s_maxlev;
-  unsigned epoch = 0;
-  Ctl *ctl = a.ctl;
-  if (stopped(ctl)) return;
-  RealDesc d0;
-  if (SINGLE) d0 = a.desc[0];
-  auto desc = [&](int r) -> const RealDesc & { return SINGLE ? d0 : a.desc[r]; };
-  auto real_of = [&](int g) -> int { return SINGLE ? 0 : find_real(s_pre, nreal, g); };
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  const int offk0 = SINGLE ? nbr_off(lane & 7, d0.W) : 0;
-  const int warp_global = tid >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-  const bool stamp = a.stamp && tid == 0;
-  const unsigned long long t_start = stamp ? globaltimer_ns() : 0;
-  if (threadIdx.x == 0) s_maxlev = 0;
-  __syncthreads();
-  for (int r = threadIdx.x; r < nreal; r += kWalkThreads) {
-    s_nlev[r] = __ldcg(&a.rctl[r].nlevels);
-    atomicMax(&s_maxlev, s_nlev[r]);
-  }
-  __syncthreads();
-  const int maxlev = s_maxlev;
-
-  // Level Lv of every realization as [lo_of(r), hi_of(r)) (empty past its
-  // depth), and the prefix of its 32-entry groups over the batch. A batch
-  // of one copies its level table into shared memory once (one load per
-  // entry and block) and takes each level's range from there into
-  // registers: no block barrier, scan or global load per level.
-  __shared__ int s_off[kLevelCache + 1];
-  if (SINGLE) {
-    const int n = min(maxlev, kLevelCache) + 1;
-    for (int k = threadIdx.x; k < n; k += kWalkThreads) s_off[k] = __ldcg(&a.lvl_off[d0.lvl_base + k]);
-    __syncthreads();
-  }
-  int lv_lo = 0, lv_hi = 0;
-  auto lo_of = [&](int r) -> int { return SINGLE ? lv_lo : s_lo[r]; };
-  auto hi_of = [&](int r) -> int { return SINGLE ? lv_hi : s_hi[r]; };
-  auto pre_of = [&](int r) -> int { return SINGLE ? 0 : s_pre[r]; };
-  auto level_groups = [&](int Lv) -> int {
-    if (SINGLE) {
-      if (Lv < kLevelCache) {
-        lv_lo = s_off[Lv];
-        lv_hi = s_off[Lv + 1];
-      } else {  // deeper than the cache: one load per block
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          s_lo[0] = __ldcg(&a.lvl_off[d0.lvl_base + Lv]);
-          s_hi[0] = __ldcg(&a.lvl_off[d0.lvl_base + Lv + 1]);
-        }
-        __syncthreads();
-        lv_lo = s_lo[0];
-        lv_hi = s_hi[0];
-      }
-      return (lv_hi - lv_lo + 31) >> 5;
-    }
-    __syncthreads();  // every warp is done with the previous ranges
-    for (int r = threadIdx.x; r < nreal; r += kWalkThreads) {
-      if (Lv < s_nlev[r]) {
-        const int b = desc(r).lvl_base;
-        s_lo[r] = __ldcg(&a.lvl_off[b + Lv]);
-        s_hi[r] = __ldcg(&a.lvl_off[b + Lv + 1]);
-      } else {
-        s_lo[r] = s_hi[r] = 0;
-      }
-    }
-    __syncthreads();
-    return block_prefix(nreal, [&](int r) { return (s_hi[r] - s_lo[r] + 31) >> 5; }, s_pre);
-  };
-
-  // ---- uplift + erosion: fastscape_RB.cpp:285-296 and :306-328 in the
-  // level order of fastscape_RB+P.cpp:319-350. Eroded cells are uplifted on
-  // their first read (uplift of every interior cell precedes erosion in the
-  // reference; a cell's h is read first by its own erosion, its receiver's
-  // h is final).
-  // A warp erodes one 32-entry group per iteration, in a software pipeline:
-  // the entries (cell, receiver direction, drainage count) of the group two
-  // iterations ahead and the elevations of the next group are loaded before
-  // this group's erosion, so the chain entry -> elevation -> erosion of one
-  // group overlaps the erosion of the groups before it. The next level's
-  // ranges and first groups -- entries and the cells' own elevations, which
-  // this level does not change -- are loaded before the level's barrier;
-  // after it only the receivers' elevations remain to be gathered.
-  int ngroups = 0;  // groups of the level being eroded
-  struct Entry {
-    int c, dir, r;
-    uint32_t k;
-    bool ok;
-  };
-  struct Heights {
-    uint64_t hc, hn;  // bit patterns in integer registers (see fadd_bits)
-  };
-  auto load_entry = [&](int g) -> Entry {
-    Entry e{0, 0, 0, 0u, false};
-    if (g < ngroups) {
-      const int r = real_of(g);
-      const int i = lo_of(r) + 32 * (g - pre_of(r)) + lane;
-      e.r = r;
-      if (i < hi_of(r)) {
-        const int off = desc(r).off;
-        e.ok = true;
-        e.c = __ldcg(&a.ent[off + i]);
-        e.dir = __ldcg(&a.pdir[off + i]);
-        e.k = __ldcg(&a.acc[off + i]);
-      }
-    }
-    return e;
-  };
-  auto gather_hc = [&](const Entry &e) -> uint64_t {
-    return e.ok ? __ldcg(reinterpret_cast<const unsigned long long *>(a.h + desc(e.r).off) + e.c)
-                : 0ull;
-  };
-  auto gather_hn = [&](const Entry &e) -> uint64_t {
-    // a group lies in one realization: lane k < 8 holds direction k's offset
-    const int offk = SINGLE ? offk0 : nbr_off(lane & 7, desc(e.r).W);
-    const int ro = __shfl_sync(kFull, offk, e.dir & 7);
-    return e.ok ? __ldcg(reinterpret_cast<const unsigned long long *>(a.h + desc(e.r).off) +
-                         e.c + ro)
-                : 0ull;
-  };
-  const int gstride = nwarps;
-  Entry e1{}, e2{};
-  Heights h1{0, 0};
-  bool ahead = false;  // e1, e2 and h1.hc already hold this level's first groups
-  for (int Lv = 1; Lv < maxlev; ++Lv) {
-    if (!ahead) {
-      ngroups = level_groups(Lv);
-      e1 = load_entry(warp_global);
-      e2 = load_entry(warp_global + gstride);
-      h1.hc = gather_hc(e1);
-    }
-    h1.hn = gather_hn(e1);
-    for (int g = warp_global; g < ngroups; g += gstride) {
-      const Entry e = e1;
-      const Heights hg = h1;
-      e1 = e2;
-      e2 = load_entry(g + 2 * gstride);
-      h1.hc = gather_hc(e1);
-      h1.hn = gather_hn(e1);
-      if (e.ok) {
-        const RealDesc &d = desc(e.r);
-        const size_t rec_at = (size_t)e.k * kTabStride + 4 * (e.dir & 1);
-        const uint64_t udt = (uint64_t)__double_as_longlong(d.u_dt);
-        const uint64_t h0 = uplift_bits(hg.hc, udt);
-        uint64_t hnew;
-        if (NMODE == kNOne && !GENERIC) {
-          const unsigned long long *Tb = reinterpret_cast<const unsigned long long *>(d.tab) + rec_at;
-          hnew = erode_cell_n1<ISUB>(d, ctl, Tb, load_tab_n1(Tb), h0, hg.hn);
-        } else if (NMODE == kNTwo && !GENERIC) {
-          hnew = erode_cell_n2<ISUB>(d, a.neq, ctl,
-                                     __ldg(reinterpret_cast<const unsigned long long *>(d.tab) + rec_at),
-                                     h0, hg.hn);
-        } else {
-          hnew = (uint64_t)__double_as_longlong(
-              erode_cell<NMODE>(d, a.neq, ctl, d.tab + rec_at, __longlong_as_double(h0),
-                                __longlong_as_double(hg.hn)));
-        }
-        if (((hnew >> 52) & 0x7FF) == 0x7FF)  // Inf or NaN
-          raise_err(ctl, FS_ERR_NONFINITE, kPhaseErode);
-        reinterpret_cast<unsigned long long *>(a.h + d.off)[e.c] = hnew;
-      }
-    }
-    ahead = Lv + 1 < maxlev;
-    if (ahead) {
-      ngroups = level_groups(Lv + 1);  // reads only the finished level table
-      e1 = load_entry(warp_global);
-      e2 = load_entry(warp_global + gstride);
-      h1.hc = gather_hc(e1);
-    }
-    if (Lv + 1 < maxlev && !grid_barrier(ctl, &ctl->bar2, epoch, a.timeout_ns)) return;  }
-  if (stamp) atomicAdd(&ctl->walk_ns[2], globaltimer_ns() - t_start);
-  if (tid == 0) atomicAdd(&ctl->steps_done, 1);
 }
 
 // ---------------------------------------------------------------------------
-// Per-realization level walk for batches of many small realizations. The
-// grid-wide walk above pays a grid barrier per level for the whole batch,
-// and long runs grow hundreds of levels of a few thousand cells each; here
-// one CTA walks one realization's levels with block barriers only (several
-// realizations per SM), with the same arrays, the same per-cell arithmetic
-// and the same level ids, counts and elevations bit for bit (the order of
-// entries within a level may differ from the grid walk's, which its atomics
-// leave free as well).
+// Per-realization level walk, the timestep of batches of many small
+// realizations late in a long run, whose tiles do not fit the GPU at once.
+// There the tile walk (fs_tile.cu) finds narrow levels, some 30 cells of a
+// tile, and revisits each tile five times from its queue (256 realizations of
+// eroded 512^2: 9.4 ms); one CTA that walks a whole realization's levels, some
+// 1000 cells wide, with block barriers only, keeps its threads busy. Same
+// per-cell arithmetic, counts and elevations bit for bit.
 //   k_cta_order_accum: level ordering (fastscape_RB.cpp:213-254: level k+1 =
 //     the donors of level k, each entry's donors contiguous in direction
 //     order) and the accumulation back down the levels (fastscape_RB.cpp:
@@ -1737,12 +995,14 @@ __global__ void __launch_bounds__(kWalkThreads, 2) k_erode(StepArgs a) {
 //     next kernel leaves every elevation unchanged and the timestep is redone.
 //   k_cta_erode: uplift of the pits, then uplift + erosion level by level
 //     (fastscape_RB.cpp:285-328 in the level order of fastscape_RB+P.cpp:
-//     319-350), exactly as k_accum's tail and k_erode do.
+//     319-350).
+// The CTAs are as wide as the batch leaves room for: a batch of up to two
+// realizations per SM gives each 1024 threads for the ordering (512 for the
+// erosion), one of more than four 256 (128), so that the realizations walk
+// at once and the latency of one's levels is hidden by the others'.
 // ---------------------------------------------------------------------------
-constexpr int kCtaThreads = 256;       // ordering CTAs (32 registers: 8 per SM)
-constexpr int kCtaErodeThreads = 128;  // erosion CTAs (at most 72 registers: 7 per SM)
-
-__global__ void __launch_bounds__(kCtaThreads, 8) k_cta_order_accum(StepArgs a) {
+template <int T>
+__global__ void __launch_bounds__(T, 2048 / T) k_cta_order_accum(StepArgs a) {
   Ctl *ctl = a.ctl;
   if (stopped(ctl)) return;
   const int t = threadIdx.x;
@@ -1766,7 +1026,7 @@ __global__ void __launch_bounds__(kCtaThreads, 8) k_cta_order_accum(StepArgs a) 
     bool ovf = false;
     for (;;) {
       int next = hi;
-      for (int cs = lo; cs < hi; cs += kCtaThreads) {
+      for (int cs = lo; cs < hi; cs += T) {
         const int i = cs + t;
         int cell = 0;
         unsigned m = 0;
@@ -1776,7 +1036,7 @@ __global__ void __launch_bounds__(kCtaThreads, 8) k_cta_order_accum(StepArgs a) 
           acc[i] = 1u;  // the cell itself; donors add theirs below
         }
         int total;
-        const int excl = block_excl_scan(__popc(m), total, t, kCtaThreads);
+        const int excl = block_excl_scan(__popc(m), total, t, T);
         if (next + total > d.size) {  // block-uniform
           ovf = true;
           break;
@@ -1816,8 +1076,8 @@ __global__ void __launch_bounds__(kCtaThreads, 8) k_cta_order_accum(StepArgs a) 
       const int l1 = Lv + 1 <= kLevelCache ? s_lvl[Lv + 1] : __ldcg(&lvl[Lv + 1]);
       // two entries per thread load before their pushes (which go one level
       // down, so they cannot change the counts read here)
-      for (int i = l0 + t; i < l1; i += 2 * kCtaThreads) {
-        const int i2 = i + kCtaThreads;
+      for (int i = l0 + t; i < l1; i += 2 * T) {
+        const int i2 = i + T;
         const uint32_t v = __ldcg(&acc[i]);
         const int q = __ldcg(&par[i]);
         const uint32_t v2 = i2 < l1 ? __ldcg(&acc[i2]) : 0u;
@@ -1826,7 +1086,7 @@ __global__ void __launch_bounds__(kCtaThreads, 8) k_cta_order_accum(StepArgs a) 
         if (i2 < l1) atomicAdd(&acc[q2], v2);
         const uint32_t vm = v > v2 ? v : v2;
         if (a.do_erode && vm >= (uint32_t)d.tab_cap) {
-          if (atomicMax(&ctl->abort_k, (int)vm) < (int)vm) ctl->abort_r = r;
+          if (atomicMax(&ctl->abort_k, (int)vm) < (int)vm) ctl->abort_r = d.id;
         }
       }
       __syncthreads();  // this level's counts are final before the next reads them
@@ -1834,16 +1094,13 @@ __global__ void __launch_bounds__(kCtaThreads, 8) k_cta_order_accum(StepArgs a) 
   }
 }
 
-// The erosion walk keeps two entries per thread in flight (as k_erode does):
+// The erosion walk keeps two entries per thread in flight:
 // the entry after next is loaded and the next one's own elevation gathered
 // while a cell erodes; only the receiver's elevation waits for the level
 // below, and the next level's first entries are loaded before the barrier
-// (a cell's own elevation is written only in its own level). Its CTAs are
-// small so that a batch's realizations walk at once (7 per SM, 1064 on 152
-// SMs): the walk is bound by the latency of each level, hidden across
-// realizations.
-template <int NMODE, int VAR>
-__global__ void __launch_bounds__(kCtaErodeThreads, 7) k_cta_erode(StepArgs a) {
+// (a cell's own elevation is written only in its own level).
+template <int NMODE, int VAR, int T>
+__global__ void __launch_bounds__(T, T == 128 ? 7 : 1024 / T) k_cta_erode(StepArgs a) {
   constexpr bool ISUB = VAR == 1, GENERIC = VAR == 2;
   Ctl *ctl = a.ctl;
   if (stopped(ctl)) return;  // an error, or a count beyond a table: nothing changes
@@ -1864,7 +1121,7 @@ __global__ void __launch_bounds__(kCtaErodeThreads, 7) k_cta_erode(StepArgs a) {
     const uint64_t udt = (uint64_t)__double_as_longlong(d.u_dt);
     // the pits (level 0 after the rings) are uplifted, not eroded
     const int p1 = __ldcg(&lvl[1]);
-    for (int i = d.nring + t; i < p1; i += kCtaErodeThreads) {
+    for (int i = d.nring + t; i < p1; i += T) {
       const int c = __ldcg(&ent[i]);
       hh[c] = fadd_bits(__ldcg(&hh[c]), udt);
     }
@@ -1883,16 +1140,16 @@ __global__ void __launch_bounds__(kCtaErodeThreads, 7) k_cta_erode(StepArgs a) {
       return e.ok ? __ldcg(&hh[e.c + nbr_off(e.dir & 7, d.W)]) : 0ull;
     };
     int lo = p1, hi = nlev > 1 ? __ldcg(&lvl[2]) : p1;
-    Entry e1 = load_entry(lo + t, hi), e2 = load_entry(lo + t + kCtaErodeThreads, hi);
+    Entry e1 = load_entry(lo + t, hi), e2 = load_entry(lo + t + T, hi);
     uint64_t hc1 = gather_hc(e1);
     __syncthreads();  // the pits are uplifted
     for (int Lv = 1; Lv < nlev; ++Lv) {
       uint64_t hn1 = gather_hn(e1);
-      for (int i = lo + t; i < hi; i += kCtaErodeThreads) {
+      for (int i = lo + t; i < hi; i += T) {
         const Entry e = e1;
         const uint64_t hc = hc1, hn = hn1;
         e1 = e2;
-        e2 = load_entry(i + 2 * kCtaErodeThreads, hi);
+        e2 = load_entry(i + 2 * T, hi);
         hc1 = gather_hc(e1);
         hn1 = gather_hn(e1);
         const uint64_t h0 = uplift_bits(hc, udt);
@@ -1917,7 +1174,7 @@ __global__ void __launch_bounds__(kCtaErodeThreads, 7) k_cta_erode(StepArgs a) {
         lo = hi;
         hi = __ldcg(&lvl[Lv + 2]);
         e1 = load_entry(lo + t, hi);
-        e2 = load_entry(lo + t + kCtaErodeThreads, hi);
+        e2 = load_entry(lo + t + T, hi);
         hc1 = gather_hc(e1);
       }
       __syncthreads();  // this level's elevations are final before the next reads them
@@ -1992,6 +1249,15 @@ __global__ void k_place_rings(int32_t *ent, int W, int H) {
       c = (H - 2) * W + (i - top - 4 * mid_rows);
     }
     ent[i] = c;
+  }
+}
+
+// rec of a grid without receivers: -1 on the rings, kPit inside.
+__global__ void k_no_receivers(int8_t *rec, int W, int H) {
+  const int size = W * H;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < size; i += gridDim.x * blockDim.x) {
+    const int y = i / W, x = i - y * W;
+    rec[i] = (int8_t)(x >= 2 && y >= 2 && x < W - 2 && y < H - 2 ? kPit : FS_NO_FLOW);
   }
 }
 
@@ -2127,29 +1393,7 @@ size_t walk_smem_bytes(int nreal) { return sizeof(int) * (4 * (size_t)nreal + 1)
 
 int walk_threads() { return kWalkThreads; }
 
-template <int NMODE, bool SINGLE>
-const void *erode_ptr(int var) {
-  if (var == 1) return reinterpret_cast<const void *>(&k_erode<NMODE, SINGLE, 1>);
-  if (var == 2) return reinterpret_cast<const void *>(&k_erode<NMODE, SINGLE, 2>);
-  return reinterpret_cast<const void *>(&k_erode<NMODE, SINGLE, 0>);
-}
-
-const void *walk_kernel_ptr(int nmode, bool single, int var) {
-  if (nmode == kNGeneral) var = var == 2 ? 2 : 0;  // no integer variant
-  if (single) {
-    if (nmode == kNOne) return erode_ptr<kNOne, true>(var);
-    if (nmode == kNTwo) return erode_ptr<kNTwo, true>(var);
-    return erode_ptr<kNGeneral, true>(var);
-  }
-  if (nmode == kNOne) return erode_ptr<kNOne, false>(var);
-  if (nmode == kNTwo) return erode_ptr<kNTwo, false>(var);
-  return erode_ptr<kNGeneral, false>(var);
-}
-
-const void *order_kernel_ptr(bool single, int bps) {
-  if (bps >= 3)
-    return single ? reinterpret_cast<const void *>(&k_order<true, 3>)
-                  : reinterpret_cast<const void *>(&k_order<false, 3>);
+const void *order_kernel_ptr(bool single) {
   return single ? reinterpret_cast<const void *>(&k_order<true, 2>)
                 : reinterpret_cast<const void *>(&k_order<false, 2>);
 }
@@ -2162,20 +1406,11 @@ const void *accum_kernel_ptr(bool single) {
 cudaError_t prepare_walk_kernels() {
   const int bytes = (int)walk_smem_bytes(kMaxReal);
   for (int single = 0; single < 2; single++) {
-    for (int nm = 0; nm < 3; nm++) {
-      for (int var = 0; var < 3; var++) {
-        cudaError_t e = cudaFuncSetAttribute(walk_kernel_ptr(nm, single != 0, var),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return e;
-      }
-    }
-    for (int bps = 2; bps <= 3; bps++) {
-      cudaError_t e = cudaFuncSetAttribute(order_kernel_ptr(single != 0, bps),
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-      if (e != cudaSuccess) return e;
-    }
-    cudaError_t e = cudaFuncSetAttribute(accum_kernel_ptr(single != 0),
+    cudaError_t e = cudaFuncSetAttribute(order_kernel_ptr(single != 0),
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(accum_kernel_ptr(single != 0),
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -2185,11 +1420,20 @@ double neg_recip_dr(double dr) {
   return dr >= 1.0 && dr <= 0x1p60 ? -(1.0 / dr) : 0.0;
 }
 
-float tol_lower_float(double tol) {
+void set_tolerance(RealDesc *d, double tol) {
+  d->tol = tol;
+  std::memcpy(&d->tol_bits, &tol, sizeof(double));
   const double t = tol * (1.0 - 0x1p-20);
   float f = (float)t;
   while ((double)f > t) f = nextafterf(f, 0.f);
-  return f;
+  d->tol_lo_f = f;
+  auto upper = [](double x) {  // x >= 0: a double whose upper word is below x's is below x
+    uint64_t b;
+    std::memcpy(&b, &x, sizeof(b));
+    return (uint32_t)(b >> 32);
+  };
+  d->tol_q_hi = upper(tol * (1.0 - 0x1p-8));
+  d->tol_y_hi = upper(tol * 0x1p39);
 }
 
 int ring_cells(int W, int H) {
@@ -2289,16 +1533,7 @@ cudaError_t launch_donors_level0(const StepArgs &a, cudaStream_t s) {
 cudaError_t launch_order(const StepArgs &a, int sms, int bps, cudaStream_t s) {
   StepArgs args = a;
   void *params[] = {&args};
-  return cudaLaunchCooperativeKernel(order_kernel_ptr(a.nreal == 1, bps), dim3(sms * bps),
-                                     dim3(kWalkThreads), params, walk_smem_bytes(a.nreal), s);
-}
-
-cudaError_t launch_erode(const StepArgs &a, int sms, int bps, cudaStream_t s) {
-  StepArgs args = a;
-  void *params[] = {&args};
-  return cudaLaunchCooperativeKernel(walk_kernel_ptr(a.nmode, a.nreal == 1,
-                                                     a.erode_generic ? 2 : a.erode_isub ? 1 : 0),
-                                     dim3(sms * bps),
+  return cudaLaunchCooperativeKernel(order_kernel_ptr(a.nreal == 1), dim3(sms * bps),
                                      dim3(kWalkThreads), params, walk_smem_bytes(a.nreal), s);
 }
 
@@ -2309,44 +1544,40 @@ cudaError_t launch_accum(const StepArgs &a, int sms, int bps, cudaStream_t s) {
                                      dim3(kWalkThreads), params, walk_smem_bytes(a.nreal), s);
 }
 
-const void *cta_erode_ptr(int nmode, int var) {
-  switch (nmode) {
-    case kNOne:
-      return var == 2 ? reinterpret_cast<const void *>(&k_cta_erode<kNOne, 2>)
-             : var == 1 ? reinterpret_cast<const void *>(&k_cta_erode<kNOne, 1>)
-                        : reinterpret_cast<const void *>(&k_cta_erode<kNOne, 0>);
-    case kNTwo:
-      return var == 2 ? reinterpret_cast<const void *>(&k_cta_erode<kNTwo, 2>)
-             : var == 1 ? reinterpret_cast<const void *>(&k_cta_erode<kNTwo, 1>)
-                        : reinterpret_cast<const void *>(&k_cta_erode<kNTwo, 0>);
-    default:
-      return reinterpret_cast<const void *>(&k_cta_erode<kNGeneral, 2>);
-  }
+// Threads of a CTA by the realizations an SM has to hold.
+int cta_width(int nreal, int sms) {
+  const int per = (nreal + sms - 1) / sms;
+  return per <= 2 ? 2 : per <= 4 ? 1 : 0;
 }
 
-int cta_threads(bool erode) { return erode ? kCtaErodeThreads : kCtaThreads; }
+template <int NMODE, int VAR>
+const void *cta_erode_ptr(int width) {
+  return width == 2   ? reinterpret_cast<const void *>(&k_cta_erode<NMODE, VAR, 512>)
+         : width == 1 ? reinterpret_cast<const void *>(&k_cta_erode<NMODE, VAR, 256>)
+                      : reinterpret_cast<const void *>(&k_cta_erode<NMODE, VAR, 128>);
+}
 
-const void *cta_order_ptr() { return reinterpret_cast<const void *>(&k_cta_order_accum); }
-
-cudaError_t launch_cta_order(const StepArgs &a, int blocks, cudaStream_t s) {
-  k_cta_order_accum<<<blocks, kCtaThreads, 0, s>>>(a);
+cudaError_t launch_cta_order(const StepArgs &a, int sms, cudaStream_t s) {
+  switch (cta_width(a.nreal, sms)) {
+    case 2: k_cta_order_accum<1024><<<a.nreal, 1024, 0, s>>>(a); break;
+    case 1: k_cta_order_accum<512><<<a.nreal, 512, 0, s>>>(a); break;
+    default: k_cta_order_accum<256><<<a.nreal, 256, 0, s>>>(a);
+  }
   return cudaGetLastError();
 }
 
-cudaError_t launch_cta_erode(const StepArgs &a, int blocks, cudaStream_t s) {
+cudaError_t launch_cta_erode(const StepArgs &a, int sms, cudaStream_t s) {
   StepArgs args = a;
   void *params[] = {&args};
-  const int var = a.erode_generic ? 2 : a.erode_isub ? 1 : 0;
-  return cudaLaunchKernel(cta_erode_ptr(a.nmode, var), dim3(blocks), dim3(kCtaErodeThreads), params, 0,
-                          s);
-}
-
-cudaError_t launch_walk(const StepArgs &a, int sms, int order_bps, int accum_bps,
-                        int erode_bps, cudaStream_t s) {
-  cudaError_t e = launch_order(a, sms, order_bps, s);
-  if (e == cudaSuccess) e = launch_accum(a, sms, accum_bps, s);
-  if (e != cudaSuccess || !a.do_erode) return e;
-  return launch_erode(a, sms, erode_bps, s);
+  const int w = cta_width(a.nreal, sms), var = a.erode_generic ? 2 : a.erode_isub ? 1 : 0;
+  const void *k = a.nmode == kNOne ? (var == 2   ? cta_erode_ptr<kNOne, 2>(w)
+                                      : var == 1 ? cta_erode_ptr<kNOne, 1>(w)
+                                                 : cta_erode_ptr<kNOne, 0>(w))
+                  : a.nmode == kNTwo ? (var == 2   ? cta_erode_ptr<kNTwo, 2>(w)
+                                        : var == 1 ? cta_erode_ptr<kNTwo, 1>(w)
+                                                   : cta_erode_ptr<kNTwo, 0>(w))
+                                     : cta_erode_ptr<kNGeneral, 2>(w);
+  return cudaLaunchKernel(k, dim3(a.nreal), dim3(w == 2 ? 512 : w == 1 ? 256 : 128), params, 0, s);
 }
 
 cudaError_t launch_check_finite(const double *h, long long n, Ctl *ctl, cudaStream_t s) {
@@ -2367,6 +1598,12 @@ cudaError_t launch_philox_field(double *h, int W, int H, uint64_t seed, cudaStre
 
 cudaError_t launch_place_rings(int32_t *ent, int W, int H, cudaStream_t s) {
   k_place_rings<<<64, 256, 0, s>>>(ent, W, H);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_no_receivers(int8_t *rec, int W, int H, cudaStream_t s) {
+  const long long blocks = ((long long)W * H + 255) / 256;
+  k_no_receivers<<<(int)(blocks < 4096 ? blocks : 4096), 256, 0, s>>>(rec, W, H);
   return cudaGetLastError();
 }
 

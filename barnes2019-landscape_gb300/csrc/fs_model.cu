@@ -8,18 +8,19 @@
 //   h       double[C]           elevation (the only state carried between
 //                               timesteps, as in the reference)
 //   rec     int8[C]             receiver direction code, -1 rings, -2 pits
-//   mask    uint8[C]            donor mask (bit k: neighbour k drains here)
-//   ent     int32[C]            cells grouped by level (the reference's stack)
-//   pdir    uint8[C]            receiver direction by level position
-//   acc     uint32[C]           drainage cell counts by level position
-//                               (accum = acc*cell_area)
-//   par     int32[C]            receiver's position by level position
+//   count   uint32[C]           drainage cell counts (accum = count*cell_area)
 //   amb     int32[C], amb_r     cells queued for the FP64 receiver fix-up
-//   lvl_off int32[C+2n]         level offsets, size_r+2 per realization
+//   tile_mem                    the tile walk's arrays (fs_internal.h, TileBufs),
+//                               12 KB per 64 x 32 cells
+//   ent, pdir, acc, par, lvl_off, mask
+//                               the level order and donor masks, which the
+//                               timestep does without: written when a caller
+//                               asks for levels, masks or the depth-first order
 //   tab_r   double[8*cap_r]     erosion table of realization r per drainage
 //                               count k < cap_r (fs_internal.h); grows on
 //                               demand
-//   desc, rctl, ctl, tiles      descriptors, counters, status, stencil tiles
+//   desc, rctl, ctl, tiles      descriptors, counters, status, stencil and
+//                               walk tiles
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -115,20 +116,26 @@ struct fs_batch {
   fs::RealDesc *d_desc = nullptr;
   fs::RealCtl *d_rctl = nullptr, *h_rctl = nullptr;
   fs::Ctl *d_ctl = nullptr, *h_ctl = nullptr;
-  fs::Tile *d_rtiles = nullptr, *d_dtiles = nullptr;
+  fs::Tile *d_rtiles = nullptr, *d_dtiles = nullptr, *d_wtiles = nullptr;
   int nrtiles = 0, ndtiles = 0;
+  uint32_t *count = nullptr;
+  void *tile_mem = nullptr;
+  fs::TileBufs tb{};             // over tile_mem, all tiles
+  std::vector<int> tile0;        // first walk tile of each realization, and the total
+  fs::TileRoom room;             // blocks of the tile kernels that fit the GPU
+  bool network_stale = true;     // the level order is older than the receivers
+  std::vector<char> count_stale; // and `count`, per realization
+  std::vector<char> stepped;     // realizations that a timestep or analysis included
   std::vector<fs::RealDesc> desc;
   std::vector<double *> tab;
   std::vector<int> tab_cap;
-  int walk_occ = 1, walk_sms = 1, walk_bps = 2;  // k_erode blocks per SM: limit, SMs, in use
-  int order_max = 2, order_bps = 2;              // k_order blocks per SM: limit (2 or 3), in use
+  int walk_sms = 1;
+  int order_bps = 2;                             // k_order blocks per SM
   int accum_bps = 1;                             // k_accum blocks per SM
-  int erode_isub = 0;                            // k_erode's integer subtractions (n = 1)
-  // per-realization walk (one CTA per realization, block barriers only):
-  // used when cta_walk and the launch covers more than one realization;
-  // resident CTAs per SM of its ordering and erosion kernels (by variant)
+  int erode_isub = 0;                            // the erosion's integer subtractions (n = 1, 2)
+  // per-realization walk: used when cta_walk, the launch covers more than one
+  // realization and their tiles do not all fit the GPU at once
   bool cta_walk = false;
-  int cta_occ_order = 1, cta_occ_erode[3] = {1, 1, 1};
   // a single grid's receiver filter may stage its tiles by TMA (rmap_ok:
   // the map exists; rtma: in use; the autotuner decides)
   CUtensorMap rmap;
@@ -145,16 +152,16 @@ struct fs_batch {
   std::vector<cudaEvent_t> ev;
   double phase_ms[FS_NUM_TIMERS] = {};  // event timers (indices 0-3, 7, 8)
   // Active subset (fs_batch_set_active): act_n > 0 steps only the
-  // realizations act_idx through their own descriptor, counter and tile
-  // arrays (the per-cell arrays are shared); act_n == 0 steps all.
+  // realizations act_idx through descriptors and tile lists of their own
+  // (the per-cell arrays are shared); act_n == 0 steps all.
   int act_n = 0;
   std::vector<int> act_idx;
   fs::RealDesc *d_desc_act = nullptr;
   fs::RealCtl *d_rctl_act = nullptr;
-  int *d_act_idx = nullptr;
   fs::Tile *d_rtiles_act = nullptr, *d_dtiles_act = nullptr;
-  int nrt_act = 0, ndt_act = 0, act_cap = 0, act_tiles_cap[2] = {0, 0};
-  int act_walk_bps = 0, act_order_bps = 0, act_accum_bps = 0;
+  int32_t *d_wlist_act = nullptr;  // their walk tiles
+  int nrt_act = 0, ndt_act = 0, nwt_act = 0, act_cap = 0, act_tiles_cap[2] = {0, 0},
+      wlist_act_cap = 0;
 };
 
 struct fs_model {
@@ -181,8 +188,8 @@ void free_batch(fs_batch *b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
   void *bufs[] = {b->h, b->rec_alloc, b->mask, b->pdir, b->ent, b->par, b->amb, b->amb_r,
                   b->lvl, b->acc, b->d_desc, b->d_rctl, b->d_ctl, b->d_rtiles, b->d_dtiles,
-                  b->d_desc_act, b->d_rctl_act, b->d_act_idx, b->d_rtiles_act,
-                  b->d_dtiles_act};
+                  b->d_wtiles, b->count, b->tile_mem, b->d_desc_act, b->d_rctl_act,
+                  b->d_rtiles_act, b->d_dtiles_act, b->d_wlist_act};
   for (void *x : bufs) cudaFree(x);
   for (double *t : b->tab) cudaFree(t);
   if (b->h_ctl) cudaFreeHost(b->h_ctl);
@@ -277,6 +284,7 @@ fs::StepArgs step_args(const fs_batch *b, int do_erode) {
   a.nrtiles = b->nrtiles;
   a.dtiles = b->d_dtiles;
   a.ndtiles = b->ndtiles;
+  a.tb = b->tb;
   if (b->act_n > 0) {
     a.desc = b->d_desc_act;
     a.rctl = b->d_rctl_act;
@@ -285,13 +293,14 @@ fs::StepArgs step_args(const fs_batch *b, int do_erode) {
     a.nrtiles = b->nrt_act;
     a.dtiles = b->d_dtiles_act;
     a.ndtiles = b->ndt_act;
+    a.tb.list = b->d_wlist_act;
+    a.tb.n = b->nwt_act;
   }
   a.nmode = b->nmode;
   a.neq = b->neq;
   a.do_erode = do_erode;
   a.erode_isub = b->erode_isub;
   a.erode_generic = b->erode_generic ? 1 : 0;
-  a.stamp = b->timing == 1 ? 1 : 0;
   a.timeout_ns = b->timeout_ns;
   return a;
 }
@@ -300,41 +309,38 @@ const CUtensorMap *receiver_map(const fs_batch *b) {
   return b->rtma && b->rmap_ok && b->n == 1 ? &b->rmap : nullptr;
 }
 
-// The per-realization walk runs when chosen and the launch covers more than
-// one realization (a single grid keeps the grid-wide walk).
-bool use_cta(const fs_batch *b, const fs::StepArgs &a) { return b->cta_walk && a.nreal > 1; }
+cudaError_t reset_ctl(fs_batch *b) {
+  return cudaMemsetAsync(reinterpret_cast<char *>(b->d_ctl) + fs::kCtlResetOffset, 0,
+                         fs::kCtlResetBytes, b->stream);
+}
 
-// CTAs of a per-realization walk kernel: every realization at once where
-// they fit, else as many as are resident (each loops over realizations).
-int cta_blocks(const fs_batch *b, const fs::StepArgs &a, bool erode) {
-  const int var = a.erode_generic ? 2 : a.erode_isub ? 1 : 0;
-  const int occ = erode ? b->cta_occ_erode[var] : b->cta_occ_order;
-  const int resident = b->walk_sms * std::max(occ, 1);
-  return std::max(1, std::min(a.nreal, resident));
+// The per-realization walk runs when chosen, for more than one realization
+// whose tiles the GPU cannot hold at once (resident tiles are faster: 8
+// realizations of eroded 512^2 0.35 against 1.6 ms).
+bool use_cta(const fs_batch *b, const fs::StepArgs &a) {
+  return b->cta_walk && a.nreal > 1 && a.do_erode && a.tb.n > b->room.resident;
 }
 
 // The launches of one timestep (no synchronization).
 cudaError_t launch_step(fs_batch *b, const fs::StepArgs &a) {
-  cudaError_t e = cudaMemsetAsync(reinterpret_cast<char *>(b->d_ctl) + fs::kCtlResetOffset, 0,
-                                  fs::kCtlResetBytes, b->stream);
-  if (e == cudaSuccess)
+  cudaError_t e = reset_ctl(b);
+  const bool cta = use_cta(b, a);
+  if (cta && e == cudaSuccess)
     e = cudaMemsetAsync(a.rctl, 0, sizeof(fs::RealCtl) * a.nreal, b->stream);
   if (e == cudaSuccess)
     e = b->exact_receivers ? fs::launch_receivers_exact(a, b->stream)
                            : fs::launch_receivers_fast(a, b->stream, receiver_map(b));
-  if (e == cudaSuccess) e = fs::launch_donors_level0(a, b->stream);
-  if (e == cudaSuccess) {
-    if (use_cta(b, a)) {
-      e = fs::launch_cta_order(a, cta_blocks(b, a, false), b->stream);
-      if (e == cudaSuccess && a.do_erode)
-        e = fs::launch_cta_erode(a, cta_blocks(b, a, true), b->stream);
-    } else if (b->act_n > 0) {
-      e = fs::launch_walk(a, b->walk_sms, b->act_order_bps, b->act_accum_bps, b->act_walk_bps,
-                          b->stream);
-    } else {
-      e = fs::launch_walk(a, b->walk_sms, b->order_bps, b->accum_bps, b->walk_bps, b->stream);
-    }
+  if (cta) {
+    if (e == cudaSuccess) e = fs::launch_donors_level0(a, b->stream);
+    if (e == cudaSuccess) e = fs::launch_cta_order(a, b->walk_sms, b->stream);
+    if (e == cudaSuccess) e = fs::launch_cta_erode(a, b->walk_sms, b->stream);
+    return e;
   }
+  if (e == cudaSuccess) e = fs::launch_tile_drain(a, b->stream);
+  if (e == cudaSuccess) e = fs::launch_tile_links(a, b->stream);
+  if (e == cudaSuccess && !a.do_erode) return fs::launch_tile_counts(a, b->stream);
+  if (e == cudaSuccess) e = fs::launch_tile_erode(a, b->room, b->stream);
+  if (e == cudaSuccess) e = fs::launch_tile_rest(a, b->room, b->stream);
   return e;
 }
 
@@ -347,51 +353,57 @@ int ensure_events(fs_batch *b, size_t n) {
   return FS_OK;
 }
 
-// Events per timed timestep: start, after the receivers, after the donors,
-// after the ordering, after the accumulation (the next timestep's start, or
-// the final event, closes the erosion kernel).
+// Events per timed timestep: start, after the receivers, after the drainage
+// inside the tiles, after the drainage between them, after the erosion of the
+// trees rooted in their tile, or of all resident tiles (the next timestep's
+// start, or the final event, closes the queue's).
 constexpr int kEvPerStep = 5;
 
 // One timestep with the phase events ev[5i..5i+5] around its launches.
 int timed_step(fs_batch *b, const fs::StepArgs &a, int i) {
   cudaEvent_t *ev = &b->ev[kEvPerStep * i];
   FS_CUDA(cudaEventRecord(ev[0], b->stream));
-  FS_CUDA(cudaMemsetAsync(reinterpret_cast<char *>(b->d_ctl) + fs::kCtlResetOffset, 0,
-                          fs::kCtlResetBytes, b->stream));
-  FS_CUDA(cudaMemsetAsync(a.rctl, 0, sizeof(fs::RealCtl) * a.nreal, b->stream));
+  FS_CUDA(reset_ctl(b));
+  const bool cta = use_cta(b, a);
+  if (cta) FS_CUDA(cudaMemsetAsync(a.rctl, 0, sizeof(fs::RealCtl) * a.nreal, b->stream));
   FS_CUDA(b->exact_receivers ? fs::launch_receivers_exact(a, b->stream)
                              : fs::launch_receivers_fast(a, b->stream, receiver_map(b)));
   FS_CUDA(cudaEventRecord(ev[1], b->stream));
-  FS_CUDA(fs::launch_donors_level0(a, b->stream));
-  FS_CUDA(cudaEventRecord(ev[2], b->stream));
-  const bool act = b->act_n > 0;
-  if (use_cta(b, a)) {
-    // ordering + accumulation in one kernel (reported as the ordering's),
-    // then the erosion
-    FS_CUDA(fs::launch_cta_order(a, cta_blocks(b, a, false), b->stream));
+  if (cta) {
+    // ordering + accumulation in one kernel, then the erosion
+    FS_CUDA(fs::launch_donors_level0(a, b->stream));
+    FS_CUDA(cudaEventRecord(ev[2], b->stream));
+    FS_CUDA(fs::launch_cta_order(a, b->walk_sms, b->stream));
     FS_CUDA(cudaEventRecord(ev[3], b->stream));
+    FS_CUDA(fs::launch_cta_erode(a, b->walk_sms, b->stream));
     FS_CUDA(cudaEventRecord(ev[4], b->stream));
-    FS_CUDA(fs::launch_cta_erode(a, cta_blocks(b, a, true), b->stream));
     return FS_OK;
   }
-  FS_CUDA(fs::launch_order(a, b->walk_sms, act ? b->act_order_bps : b->order_bps, b->stream));
+  FS_CUDA(fs::launch_tile_drain(a, b->stream));
+  FS_CUDA(cudaEventRecord(ev[2], b->stream));
+  FS_CUDA(fs::launch_tile_links(a, b->stream));
   FS_CUDA(cudaEventRecord(ev[3], b->stream));
-  FS_CUDA(fs::launch_accum(a, b->walk_sms, act ? b->act_accum_bps : b->accum_bps, b->stream));
+  FS_CUDA(fs::launch_tile_erode(a, b->room, b->stream));
   FS_CUDA(cudaEventRecord(ev[4], b->stream));
-  FS_CUDA(fs::launch_erode(a, b->walk_sms, act ? b->act_walk_bps : b->walk_bps, b->stream));
+  FS_CUDA(fs::launch_tile_rest(a, b->room, b->stream));
   return FS_OK;
 }
 
 int harvest_events(fs_batch *b, int k) {
   FS_CUDA(cudaEventSynchronize(b->ev[kEvPerStep * k]));
-  // receivers, donors, k_order, k_accum, k_erode
-  static const int slot[kEvPerStep] = {0, 1, 7, 9, 8};
+  // receivers, k_tile_drain, k_tile_links, k_tile_resident or k_tile_rooted, the rest; the
+  // last three also fill the walk's split
+  static const int slot[kEvPerStep] = {0, 1, 7, 8, 9};
+  static const int split[kEvPerStep] = {0, 0, 4, 6, 5};
   for (int i = 0; i < k; i++)
     for (int j = 0; j < kEvPerStep; j++) {
       float ms = 0;
       FS_CUDA(cudaEventElapsedTime(&ms, b->ev[kEvPerStep * i + j], b->ev[kEvPerStep * i + j + 1]));
       b->phase_ms[slot[j]] += ms;
-      if (j >= 2) b->phase_ms[2] += ms;  // the level walk: its three kernels
+      if (j >= 2) {  // the walk: its three kernels
+        b->phase_ms[2] += ms;
+        b->phase_ms[split[j]] += ms;
+      }
     }
   float tot = 0;
   FS_CUDA(cudaEventElapsedTime(&tot, b->ev[0], b->ev[kEvPerStep * k]));
@@ -440,28 +452,6 @@ int read_rctl(const fs_batch *b) {
                           b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
   return FS_OK;
-}
-
-// Copies the active subset's per-realization counters (levels found,
-// cells placed) back to the realizations' own entries.
-__global__ void k_scatter_rctl(const fs::RealCtl *__restrict__ src, const int *__restrict__ idx,
-                               int n, fs::RealCtl *__restrict__ dst) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[idx[i]] = src[i];
-}
-
-cudaError_t launch_scatter_rctl(fs_batch *b) {
-  k_scatter_rctl<<<(b->act_n + 127) / 128, 128, 0, b->stream>>>(b->d_rctl_act, b->d_act_idx,
-                                                                b->act_n, b->d_rctl);
-  return cudaGetLastError();
-}
-
-// Per-cell drainage counts of one realization from the walk's
-// position-indexed arrays: counts[ent[i]] = acc[i].
-__global__ void k_drainage_counts(const int32_t *__restrict__ ent, const uint32_t *__restrict__ acc,
-                                  int size, uint32_t *__restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < size; i += gridDim.x * blockDim.x)
-    out[ent[i]] = acc[i];
 }
 
 // Initial erosion tables of every realization (counts below min(65536,
@@ -513,16 +503,6 @@ int init_tables(fs_batch *b) {
   return FS_OK;
 }
 
-// Blocks per SM of a cooperative walk kernel: `want`, or fewer when fewer are
-// resident with `smem` bytes of shared memory.
-int resident_bps(const void *kernel, size_t smem, int want, int *out) {
-  int occ = 0;
-  FS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, fs::walk_threads(), smem));
-  if (occ < 1) return set_error(FS_ERR_CUDA, "walk kernel cannot be resident");
-  *out = std::min(occ, want);
-  return FS_OK;
-}
-
 // Selects the realizations the next timesteps advance (n = 0: all).
 int set_active(fs_batch *b, int n, const int *idx) {
   if (n < 0 || n > b->n) return set_error(FS_ERR_ARG, "active count %d out of [0, %d]", n, b->n);
@@ -544,6 +524,7 @@ int set_active(fs_batch *b, int n, const int *idx) {
   }
   std::vector<fs::RealDesc> desc(n);
   std::vector<fs::Tile> rt, dt;
+  std::vector<int32_t> wl;
   for (int i = 0; i < n; i++) {
     const int r = idx[i];
     desc[i] = b->desc[r];
@@ -555,18 +536,17 @@ int set_active(fs_batch *b, int n, const int *idx) {
                                        static_cast<int>(v.size() - at));
       v.resize(at + std::max(got, 0));
     }
+    for (int t = b->tile0[r]; t < b->tile0[r + 1]; t++) wl.push_back(t);
   }
+  b->act_n = 0;  // until every list below is in place
   if (n > b->act_cap) {
     cudaFree(b->d_desc_act);
     cudaFree(b->d_rctl_act);
-    cudaFree(b->d_act_idx);
     b->d_desc_act = nullptr;
     b->d_rctl_act = nullptr;
-    b->d_act_idx = nullptr;
     b->act_cap = 0;
     FS_CUDA(cudaMalloc(&b->d_desc_act, n * sizeof(fs::RealDesc)));
     FS_CUDA(cudaMalloc(&b->d_rctl_act, n * sizeof(fs::RealCtl)));
-    FS_CUDA(cudaMalloc(&b->d_act_idx, n * sizeof(int)));
     b->act_cap = n;
   }
   fs::Tile **tiles[2] = {&b->d_rtiles_act, &b->d_dtiles_act};
@@ -576,41 +556,87 @@ int set_active(fs_batch *b, int n, const int *idx) {
       cudaFree(*tiles[k]);
       *tiles[k] = nullptr;
       b->act_tiles_cap[k] = 0;
-      FS_CUDA(cudaMalloc(tiles[k], std::max<size_t>(1, ntile[k]) * sizeof(fs::Tile)));
+      FS_CUDA(cudaMalloc(tiles[k], ntile[k] * sizeof(fs::Tile)));
       b->act_tiles_cap[k] = static_cast<int>(ntile[k]);
     }
+  if (static_cast<int>(wl.size()) > b->wlist_act_cap) {
+    cudaFree(b->d_wlist_act);
+    b->d_wlist_act = nullptr;
+    b->wlist_act_cap = 0;
+    FS_CUDA(cudaMalloc(&b->d_wlist_act, wl.size() * sizeof(int32_t)));
+    b->wlist_act_cap = static_cast<int>(wl.size());
+  }
   FS_CUDA(cudaMemcpyAsync(b->d_desc_act, desc.data(), n * sizeof(fs::RealDesc),
                           cudaMemcpyHostToDevice, b->stream));
-  FS_CUDA(cudaMemcpyAsync(b->d_act_idx, idx, n * sizeof(int), cudaMemcpyHostToDevice, b->stream));
   if (!rt.empty())
     FS_CUDA(cudaMemcpyAsync(b->d_rtiles_act, rt.data(), rt.size() * sizeof(fs::Tile),
                             cudaMemcpyHostToDevice, b->stream));
   if (!dt.empty())
     FS_CUDA(cudaMemcpyAsync(b->d_dtiles_act, dt.data(), dt.size() * sizeof(fs::Tile),
                             cudaMemcpyHostToDevice, b->stream));
+  FS_CUDA(cudaMemcpyAsync(b->d_wlist_act, wl.data(), wl.size() * sizeof(int32_t),
+                          cudaMemcpyHostToDevice, b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
-  // a subset of one runs the single-grid kernels, which may hold fewer
-  // blocks per SM than the batch kernels the launch shape was tuned for
-  const bool single = n == 1;
-  const size_t smem = fs::walk_smem_bytes(n);
-  if (int st = resident_bps(fs::walk_kernel_ptr(b->nmode, single, b->erode_isub ? 1 : 0), smem,
-                           b->walk_bps, &b->act_walk_bps))
-    return st;
-  if (int st = resident_bps(fs::order_kernel_ptr(single, b->order_bps), smem, b->order_bps,
-                           &b->act_order_bps))
-    return st;
-  if (b->act_order_bps < b->order_bps) {
-    // the 3-block ordering form is compiled for exactly 3 blocks per SM
-    if (int st = resident_bps(fs::order_kernel_ptr(single, 2), smem, 2, &b->act_order_bps))
-      return st;
-  }
-  if (int st = resident_bps(fs::accum_kernel_ptr(single), smem, b->accum_bps,
-                           &b->act_accum_bps))
-    return st;
   b->nrt_act = static_cast<int>(rt.size());
   b->ndt_act = static_cast<int>(dt.size());
+  b->nwt_act = static_cast<int>(wl.size());
   b->act_idx.assign(idx, idx + n);
   b->act_n = n;
+  return FS_OK;
+}
+
+// The counts of the realizations that the next launches cover: stale or not.
+void mark_counts(fs_batch *b, char stale) {
+  if (b->act_n > 0)
+    for (int r : b->act_idx) b->count_stale[r] = stale;
+  else
+    std::fill(b->count_stale.begin(), b->count_stale.end(), stale);
+}
+
+// The realizations the next launches cover have receivers of their own now.
+void mark_stepped(fs_batch *b) {
+  b->have_step = true;
+  if (b->act_n > 0)
+    for (int r : b->act_idx) b->stepped[r] = 1;
+  else
+    std::fill(b->stepped.begin(), b->stepped.end(), 1);
+}
+
+// Drainage counts per cell, and the donor masks and level order, of every
+// realization's last receivers (fastscape_RB.cpp:188-279), for the callers
+// that ask for them: the timestep itself keeps its counts in the tiles and
+// needs no order.
+int ensure_counts(const fs_batch *cb, int r) {
+  fs_batch *b = const_cast<fs_batch *>(cb);
+  if (!b->count_stale[r]) return FS_OK;
+  fs::StepArgs a = step_args(b, 0);
+  a.tb = b->tb;  // every realization, active or not
+  FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, fs::kCtlCallResetBytes, b->stream));
+  FS_CUDA(fs::launch_tile_drain(a, b->stream));
+  FS_CUDA(fs::launch_tile_links(a, b->stream));
+  FS_CUDA(fs::launch_tile_counts(a, b->stream));
+  if (int st = collect_status(b)) return st;
+  std::fill(b->count_stale.begin(), b->count_stale.end(), 0);
+  return FS_OK;
+}
+
+int ensure_network(const fs_batch *cb) {
+  fs_batch *b = const_cast<fs_batch *>(cb);
+  if (!b->network_stale) return FS_OK;
+  fs::StepArgs a = step_args(b, 0);
+  a.desc = b->d_desc;  // every realization, active or not
+  a.rctl = b->d_rctl;
+  a.nreal = b->n;
+  a.dtiles = b->d_dtiles;
+  a.ndtiles = b->ndtiles;
+  FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, fs::kCtlCallResetBytes, b->stream));
+  FS_CUDA(cudaMemsetAsync(&b->d_ctl->bar, 0, sizeof(fs::Ctl) - offsetof(fs::Ctl, bar), b->stream));
+  FS_CUDA(cudaMemsetAsync(b->d_rctl, 0, sizeof(fs::RealCtl) * b->n, b->stream));
+  FS_CUDA(fs::launch_donors_level0(a, b->stream));
+  FS_CUDA(fs::launch_order(a, b->walk_sms, b->order_bps, b->stream));
+  FS_CUDA(fs::launch_accum(a, b->walk_sms, b->accum_bps, b->stream));
+  if (int st = collect_status(b)) return st;
+  b->network_stale = false;
   return FS_OK;
 }
 
@@ -655,14 +681,15 @@ int batch_step(fs_batch *b, int k) {
         b->phase_ms[3] += tot;
       }
     }
-    if (b->act_n > 0) FS_CUDA(launch_scatter_rctl(b));
+    b->network_stale = true;
+    mark_counts(b, 1);
     if (int st = collect_status(b)) return st;
     const int completed = b->h_ctl->steps_done;
+    if (completed > 0) mark_stepped(b);
     done += completed;
     b->steps += completed;
-    if (completed > 0) b->have_step = true;
     if (b->h_ctl->abort_k > 0) {
-      const int ar = b->act_n > 0 ? b->act_idx[b->h_ctl->abort_r] : b->h_ctl->abort_r;
+      const int ar = b->h_ctl->abort_r;
       if (int st = grow_table(b, ar, b->h_ctl->abort_k)) return st;
       if (b->act_n > 0)
         for (int i = 0; i < b->act_n; i++)
@@ -737,6 +764,7 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
   b->nmode = nmode_of(b->neq);
   cudaGetDevice(&b->device);
   long long o = 0, lb = 0;
+  std::vector<fs::Tile> wt;  // walk tiles
   for (int r = 0; r < n; r++) {
     b->W.push_back(widths[r]);
     b->H.push_back(heights[r]);
@@ -747,7 +775,17 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
     b->p.push_back(params[r]);
     o += b->size.back();
     lb += b->size.back() + 2;
+    b->tile0.push_back(static_cast<int>(wt.size()));
+    const size_t at = wt.size();
+    wt.resize(at + static_cast<size_t>(widths[r] / fs::kWalkW + 1) * (heights[r] / fs::kWalkH + 1));
+    wt.resize(at + fs::append_walk_tiles(r, widths[r], heights[r], wt.data() + at,
+                                         static_cast<int>(wt.size() - at)));
   }
+  b->tile0.push_back(static_cast<int>(wt.size()));
+  if (wt.size() >= (1u << 24))  // k_tile_pull's 32-bit indices; 200 GB of tiles
+    return fail(set_error(FS_ERR_NOMEM, "%zu walk tiles", wt.size()));
+  b->stepped.assign(n, 0);
+  b->count_stale.assign(n, 1);
   b->lvl_total = lb;
   b->tab.assign(n, nullptr);
   b->tab_cap.assign(n, 0);
@@ -763,6 +801,9 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
       !cu(cudaMalloc(&b->amb_r, C * sizeof(int32_t)), "cudaMalloc(amb_r)") ||
       !cu(cudaMalloc(&b->acc, C * sizeof(uint32_t)), "cudaMalloc(acc)") ||
       !cu(cudaMalloc(&b->lvl, static_cast<size_t>(lb) * sizeof(int32_t)), "cudaMalloc(lvl)") ||
+      !cu(cudaMalloc(&b->count, C * sizeof(uint32_t)), "cudaMalloc(count)") ||
+      !cu(cudaMalloc(&b->tile_mem, fs::tile_bytes(wt.size())), "cudaMalloc(tiles)") ||
+      !cu(cudaMalloc(&b->d_wtiles, wt.size() * sizeof(fs::Tile)), "cudaMalloc(wtiles)") ||
       !cu(cudaMalloc(&b->d_desc, n * sizeof(fs::RealDesc)), "cudaMalloc(desc)") ||
       !cu(cudaMalloc(&b->d_rctl, n * sizeof(fs::RealCtl)), "cudaMalloc(rctl)") ||
       !cu(cudaMalloc(&b->d_ctl, sizeof(fs::Ctl)), "cudaMalloc(ctl)") ||
@@ -770,9 +811,18 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
       !cu(cudaMallocHost(&b->h_rctl, n * sizeof(fs::RealCtl)), "cudaMallocHost(rctl)"))
     return fail(*status);
   b->rec = b->rec_alloc + fs::kRecPad;
+  fs::tile_carve(&b->tb, b->tile_mem, wt.size());
+  b->tb.tiles = b->d_wtiles;
+  b->tb.list = nullptr;
+  b->tb.n = static_cast<int>(wt.size());
+  b->tb.desc = b->d_desc;
+  b->tb.count = b->count;
   // Rings keep NO_FLOW forever (fastscape_RB.cpp:361-362) and ring-0 cells
   // never have donors: receivers and masks are written for the interior only.
-  if (!cu(cudaMemsetAsync(b->rec, 0xff, C, b->stream), "memset(rec)") ||
+  if (!cu(cudaMemcpyAsync(b->d_wtiles, wt.data(), wt.size() * sizeof(fs::Tile),
+                          cudaMemcpyHostToDevice, b->stream),
+          "upload(wtiles)") ||
+      !cu(cudaMemsetAsync(b->count, 0, C * sizeof(uint32_t), b->stream), "memset(count)") ||
       !cu(cudaMemsetAsync(b->mask, 0, C, b->stream), "memset(mask)") ||
       !cu(cudaMemsetAsync(b->acc, 0, C * sizeof(uint32_t), b->stream), "memset(acc)") ||
       !cu(cudaMemsetAsync(b->lvl, 0, static_cast<size_t>(lb) * sizeof(int32_t), b->stream),
@@ -792,10 +842,10 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
     d.off = b->off[r];
     d.lvl_base = b->lvl_base[r];
     d.nring = b->nring[r];
+    d.tile0 = b->tile0[r];
+    d.id = r;
     d.u_dt = p.ueq * p.dt;
-    d.tol = p.tol;
-    std::memcpy(&d.tol_bits, &p.tol, sizeof(double));
-    d.tol_lo_f = fs::tol_lower_float(p.tol);
+    fs::set_tolerance(&d, p.tol);
     d.g_orth = static_cast<float>(1.0 / p.dr_orth);
     d.g_diag = static_cast<float>(1.0 / p.dr_diag);
     d.gmax = std::max(d.g_orth, d.g_diag);
@@ -840,7 +890,8 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
   // Rings 0 and 1 are the head of level 0 in every timestep; initial fields.
   std::vector<double> host;
   for (int r = 0; r < n; r++) {
-    if (!cu(fs::launch_place_rings(b->ent + b->off[r], b->W[r], b->H[r], b->stream), "rings"))
+    if (!cu(fs::launch_place_rings(b->ent + b->off[r], b->W[r], b->H[r], b->stream), "rings") ||
+        !cu(fs::launch_no_receivers(b->rec + b->off[r], b->W[r], b->H[r], b->stream), "receivers"))
       return fail(*status);
     const uint64_t seed = seeds ? seeds[r] : 0;
     double *hr = b->h + b->off[r];
@@ -861,46 +912,24 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
       return fail(*status);
     }
   }
-  int occ = 0;
   if (!cu(fs::prepare_walk_kernels(), "walk smem attribute") ||
       !cu(cudaDeviceGetAttribute(&b->walk_sms, cudaDevAttrMultiProcessorCount, b->device), "attr") ||
-      !cu(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fs::walk_kernel_ptr(b->nmode, n == 1),
-                                                        fs::walk_threads(),
-                                                        fs::walk_smem_bytes(n)),
-          "occupancy"))
+      !cu(fs::prepare_tile_kernels(b->nmode, b->walk_sms, &b->room), "tile kernels"))
     return fail(*status);
-  if (occ < 1) return fail(set_error(FS_ERR_CUDA, "walk kernel cannot be resident"));
+  if (b->room.queued < 1) return fail(set_error(FS_ERR_CUDA, "tile kernel cannot be resident"));
   b->rmap_ok = n == 1 && fs::make_receiver_map(&b->rmap, b->h, b->W[0], b->H[0]);
-  b->walk_occ = occ;
-  b->walk_bps = std::min(occ, 2);
-  if (!cu(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->cta_occ_order, fs::cta_order_ptr(),
-                                                        fs::cta_threads(false), 0),
-          "occupancy"))
-    return fail(*status);
-  for (int v = 0; v < 3; v++)
-    if (!cu(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &b->cta_occ_erode[v], fs::cta_erode_ptr(b->nmode, v), fs::cta_threads(true), 0),
-            "occupancy"))
-      return fail(*status);
-  // k_order: the variant with 3 blocks per SM is available where all three
-  // fit (a large batch's shared memory may not allow it); the 2-block one is
-  // the default, the autotuner's choice on every single grid measured (1000²
-  // to 10000², where 3 blocks per SM took ~25% longer: 0.205 against 0.149 ms
-  // per ordering at 4000²).
-  for (int bps = 3; bps >= 2; bps--) {
+  // k_order at two blocks per SM: three took ~25% longer on every single
+  // grid measured (1000² to 10000²: 0.205 against 0.149 ms per ordering at
+  // 4000²).
+  {
     int o = 0;
-    if (!cu(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fs::order_kernel_ptr(n == 1, bps),
+    if (!cu(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fs::order_kernel_ptr(n == 1),
                                                           fs::walk_threads(),
                                                           fs::walk_smem_bytes(n)),
             "occupancy"))
       return fail(*status);
-    if (o >= bps) {
-      b->order_max = bps;
-      break;
-    }
-    if (bps == 2) return fail(set_error(FS_ERR_CUDA, "order kernel cannot be resident"));
+    if (o < b->order_bps) return fail(set_error(FS_ERR_CUDA, "order kernel cannot be resident"));
   }
-  b->order_bps = 2;
   {
     int o = 0;
     if (!cu(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fs::accum_kernel_ptr(n == 1),
@@ -950,15 +979,14 @@ int get_accumulation(const fs_batch *b, int r, double *out) {
   if (!out) return set_error(FS_ERR_ARG, "out is NULL");
   if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
   DeviceGuard dg(b->device);
+  if (int st = ensure_counts(b, r)) return st;
   const int n = b->size[r];
-  std::vector<uint32_t> acc(n);
-  std::vector<int32_t> ent(n);
-  FS_CUDA(cudaMemcpyAsync(acc.data(), b->acc + b->off[r], sizeof(uint32_t) * n,
-                          cudaMemcpyDeviceToHost, b->stream));
-  FS_CUDA(cudaMemcpyAsync(ent.data(), b->ent + b->off[r], sizeof(int32_t) * n,
+  std::vector<uint32_t> k(n);
+  FS_CUDA(cudaMemcpyAsync(k.data(), b->count + b->off[r], sizeof(uint32_t) * n,
                           cudaMemcpyDeviceToHost, b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
-  for (int i = 0; i < n; i++) out[ent[i]] = static_cast<double>(acc[i]) * b->p[r].cell_area;
+  const double area = b->p[r].cell_area;
+  for (int i = 0; i < n; i++) out[i] = static_cast<double>(k[i]) * area;
   return FS_OK;
 }
 
@@ -979,8 +1007,9 @@ int get_levels(const fs_batch *b, int r, int32_t *level_id, int32_t *nlevels) {
   if (int st = check_r(b, r)) return st;
   if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
   DeviceGuard dg(b->device);
+  if (int st = ensure_network(b)) return st;
   if (int st = read_rctl(b)) return st;
-  const int nl = b->h_rctl[r].nlevels;
+  const int nl = b->stepped[r] ? b->h_rctl[r].nlevels : 0;
   if (nlevels) *nlevels = nl;
   if (!level_id) return FS_OK;
   const int n = b->size[r];
@@ -1006,6 +1035,7 @@ int get_stack_dfs(const fs_batch *b, int r, int32_t *stack, int32_t *stack_start
   if (!stack) return set_error(FS_ERR_ARG, "stack is NULL");
   if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
   DeviceGuard dg(b->device);
+  if (int st = ensure_network(b)) return st;
   if (int st = read_rctl(b)) return st;
   const int nl = b->h_rctl[r].nlevels;
   const int n = b->size[r];
@@ -1045,34 +1075,27 @@ int get_donor_mask(const fs_batch *b, int r, uint8_t *mask) {
   if (!mask) return set_error(FS_ERR_ARG, "mask is NULL");
   if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
   DeviceGuard dg(b->device);
+  if (int st = ensure_network(b)) return st;
   FS_CUDA(cudaMemcpyAsync(mask, b->mask + b->off[r], b->size[r], cudaMemcpyDeviceToHost, b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
   return FS_OK;
 }
 
 int get_phase_times(const fs_batch *b, double *ms, int reset) {
-  DeviceGuard dg(b->device);
-  FS_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(fs::Ctl), cudaMemcpyDeviceToHost, b->stream));
-  FS_CUDA(cudaStreamSynchronize(b->stream));
-  if (ms) {
+  if (ms)
     for (int i = 0; i < FS_NUM_TIMERS; i++) ms[i] = b->phase_ms[i];
-    for (int i = 0; i < 3; i++) ms[4 + i] = b->h_ctl->walk_ns[i] * 1e-6;
-  }
-  if (reset) {
+  if (reset)
     for (double &x : const_cast<fs_batch *>(b)->phase_ms) x = 0;
-    FS_CUDA(cudaMemsetAsync(reinterpret_cast<char *>(b->d_ctl) + offsetof(fs::Ctl, walk_ns), 0,
-                            sizeof(b->h_ctl->walk_ns), b->stream));
-    FS_CUDA(cudaStreamSynchronize(b->stream));
-  }
   return FS_OK;
 }
 
-// Autotuner: times each candidate launch configuration -- ordering and
-// erosion blocks per SM with and without the captured graph, then for n = 1
-// or 2 the fastest of these with the erosion's integer subtractions -- on the
-// batch's own state over `probe` timesteps, restoring the elevation after
-// every probe, and keeps the fastest; the level walk is chosen by size.
+// Autotuner: times each candidate launch configuration -- with and without
+// the captured graph, for n = 1 or 2 the faster of these with the erosion's
+// integer subtractions, and a single grid's receiver tiles staged by TMA -- on
+// the batch's own state over `probe` timesteps, restoring the elevation after
+// every probe, and keeps the fastest.
 constexpr int kCtaWalkCells = 1 << 19;
+constexpr int kErodeBps = 2;  // reported as the erosion's blocks per SM
 
 int autotune(fs_batch *b, int probe, int *chosen) {
   DeviceGuard dg(b->device);
@@ -1092,14 +1115,12 @@ int autotune(fs_batch *b, int probe, int *chosen) {
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   float best = 1e30f;
-  int best_bps = b->walk_bps, best_obps = b->order_bps, best_isub = 0;
+  int best_isub = 0;
   bool best_graph = false;
   int st = FS_OK;
   // One probe: a warm-up timestep (which also builds the graph), then
   // `probe` timed ones; the elevation is restored afterwards.
-  auto time_config = [&](int obps, int bps, bool graph, int isub, float *ms) -> int {
-    b->order_bps = obps;
-    b->walk_bps = bps;
+  auto time_config = [&](bool graph, int isub, float *ms) -> int {
     b->use_graph = graph;
     b->erode_isub = isub;
     b->graph_dirty = true;
@@ -1114,23 +1135,17 @@ int autotune(fs_batch *b, int probe, int *chosen) {
     cudaMemcpyAsync(b->h, save, b->cells * sizeof(double), cudaMemcpyDeviceToDevice, b->stream);
     return r;
   };
-  for (int obps = 2; obps <= b->order_max && st == FS_OK; obps++) {
-    for (int bps = 1; bps <= std::min(b->walk_occ, 2) && st == FS_OK; bps++) {
-      for (int gr = 0; gr < 2 && st == FS_OK; gr++) {
-        float ms = 0;
-        if ((st = time_config(obps, bps, gr == 1, 0, &ms)) != FS_OK) break;
-        if (ms < best) {
-          best = ms;
-          best_bps = bps;
-          best_obps = obps;
-          best_graph = gr == 1 && b->use_graph;
-        }
-      }
+  for (int gr = 0; gr < 2 && st == FS_OK; gr++) {
+    float ms = 0;
+    if ((st = time_config(gr == 1, 0, &ms)) != FS_OK) break;
+    if (ms < best) {
+      best = ms;
+      best_graph = gr == 1 && b->use_graph;
     }
   }
   if (st == FS_OK && b->nmode != fs::kNGeneral) {
     float ms = 0;
-    st = time_config(best_obps, best_bps, best_graph, 1, &ms);
+    st = time_config(best_graph, 1, &ms);
     if (st == FS_OK && ms < best) {
       best = ms;
       best_isub = 1;
@@ -1141,49 +1156,27 @@ int autotune(fs_batch *b, int probe, int *chosen) {
   if (st == FS_OK && b->rmap_ok) {
     float ms = 0;
     b->rtma = true;
-    st = time_config(best_obps, best_bps, best_graph, best_isub, &ms);
+    st = time_config(best_graph, best_isub, &ms);
     if (st == FS_OK && ms < best) {
       best = ms;
       best_rtma = true;
     }
   }
   b->rtma = best_rtma;
-  // The per-realization walk is chosen by size, not by the probes: its
-  // advantage (a block barrier per level instead of a grid barrier) grows with
-  // the number of levels, which the probes, run on the batch's current state,
-  // do not see when that state is young. With every realization at most
-  // kCtaWalkCells cells it wins at every depth measured (1024 x 512^2: 13.2 vs
-  // 19.0 ms per timestep over 2000 timesteps); a larger realization walked by
-  // one CTA serialises (a ragged batch up to 2048^2 ran 7x slower). Within the
-  // chosen walk the probes pick the graph.
-  const bool cta_before = b->cta_walk;
-  const bool want_cta = b->n > 1 && *std::max_element(b->size.begin(), b->size.end()) <= kCtaWalkCells;
-  if (want_cta && st == FS_OK) {
-    b->cta_walk = true;
-    best = 1e30f;
-    for (int gr = 0; gr < 2 && st == FS_OK; gr++) {
-      float ms = 0;
-      st = time_config(best_obps, best_bps, gr == 1, best_isub, &ms);
-      if (st == FS_OK && ms < best) {
-        best = ms;
-        best_graph = gr == 1 && b->use_graph;
-      }
-    }
-  }
-  b->cta_walk = st == FS_OK ? want_cta : cta_before;
+  if (st == FS_OK)
+    b->cta_walk =
+        b->n > 1 && *std::max_element(b->size.begin(), b->size.end()) <= kCtaWalkCells;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaStreamSynchronize(b->stream);
   release();
   b->timing = timing;
   b->steps = steps;
-  b->walk_bps = best_bps;
-  b->order_bps = best_obps;
   b->use_graph = best_graph;
   b->erode_isub = best_isub;
   b->graph_dirty = true;
   if (chosen) {
-    chosen[0] = best_bps;
+    chosen[0] = kErodeBps;
     chosen[1] = best_graph ? 1 : 0;
   }
   return st;
@@ -1427,7 +1420,6 @@ int fs_batch_set_timing(fs_batch *b, int enable) {
   if (!b) return set_error(FS_ERR_ARG, "batch is NULL");
   if (enable < 0 || enable > FS_TIMING_CALL)
     return set_error(FS_ERR_ARG, "timing mode must be 0, 1 or 2 (got %d)", enable);
-  if (b->timing != enable) b->graph_dirty = true;  // the walk's clock stamps change
   b->timing = enable;
   return FS_OK;
 }
@@ -1462,7 +1454,7 @@ int fs_batch_launch_config(const fs_batch *b, int *order_bps, int *erode_bps, in
                            int *erode_int_sub) {
   if (!b) return set_error(FS_ERR_ARG, "batch is NULL");
   if (order_bps) *order_bps = b->order_bps;
-  if (erode_bps) *erode_bps = b->walk_bps;
+  if (erode_bps) *erode_bps = kErodeBps;
   if (graph) *graph = b->use_graph ? 1 : 0;
   if (erode_int_sub) *erode_int_sub = b->erode_isub;
   return FS_OK;
@@ -1533,10 +1525,12 @@ int fs_batch_analyze(fs_batch *b) {
   DeviceGuard dg(b->device);
   const fs::StepArgs a = step_args(b, 0);
   FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, fs::kCtlCallResetBytes, b->stream));
+  b->network_stale = true;
+  mark_counts(b, 1);
   FS_CUDA(launch_step(b, a));
-  if (b->act_n > 0) FS_CUDA(launch_scatter_rctl(b));
   if (int st = collect_status(b)) return st;
-  b->have_step = true;
+  mark_counts(b, 0);
+  mark_stepped(b);
   return FS_OK;
 }
 
@@ -1545,10 +1539,9 @@ int fs_batch_drainage_counts(const fs_batch *b, int r, uint32_t *d_counts) {
   if (!d_counts) return set_error(FS_ERR_ARG, "d_counts is NULL");
   if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
   DeviceGuard dg(b->device);
-  const int n = b->size[r];
-  k_drainage_counts<<<std::min((n + 255) / 256, 1024), 256, 0, b->stream>>>(
-      b->ent + b->off[r], b->acc + b->off[r], n, d_counts);
-  FS_CUDA(cudaGetLastError());
+  if (int st = ensure_counts(b, r)) return st;
+  FS_CUDA(cudaMemcpyAsync(d_counts, b->count + b->off[r], sizeof(uint32_t) * b->size[r],
+                          cudaMemcpyDeviceToDevice, b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
   return FS_OK;
 }
@@ -1611,10 +1604,14 @@ int fs_test_order_from_receivers(fs_model *m, const int32_t *dir) {
   FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, sizeof(fs::Ctl), b->stream));
   FS_CUDA(cudaMemsetAsync(b->d_rctl, 0, sizeof(fs::RealCtl) * b->n, b->stream));
   const fs::StepArgs a = step_args(b, 0);
-  FS_CUDA(fs::launch_donors_level0(a, b->stream));
-  FS_CUDA(fs::launch_walk(a, b->walk_sms, b->order_bps, b->accum_bps, b->walk_bps, b->stream));
-  b->have_step = true;
-  return collect_status(b);
+  FS_CUDA(fs::launch_tile_drain(a, b->stream));
+  FS_CUDA(fs::launch_tile_links(a, b->stream));
+  FS_CUDA(fs::launch_tile_counts(a, b->stream));
+  b->network_stale = true;
+  mark_counts(b, 0);
+  mark_stepped(b);
+  if (int st = collect_status(b)) return st;
+  return ensure_network(b);
 }
 
 // Selects the receiver kernel: 1 = the FP64 reference formula for every

@@ -14,9 +14,9 @@
 // Limits and sharing:
 //   * grids of at most FS_NOALLOC_MAX_CELLS cells (width*height); larger
 //     grids are rejected with FS_ERR_ARG;
-//   * the scratch array (~24 MB: receivers, donor masks, level lists and
-//     offsets, receiver positions, drainage counts, the erosion table for
-//     every possible count,
+//   * the scratch array (~50 MB: receivers, drainage counts, the tile walk's
+//     arrays for the most tiles a grid within the limit can have -- a
+//     3-cell-wide one, 2731 -- the erosion table for every possible count,
 //     stencil tiles, descriptors and the control block) lives in the library
 //     image, so every GPU that loads the library holds it until the process
 //     exits;
@@ -47,30 +47,25 @@ namespace {
 
 constexpr size_t kMaxCells = FS_NOALLOC_MAX_CELLS;
 constexpr size_t kTabRecords = kMaxCells + 1;  // counts 0..kMaxCells
-constexpr int kMaxTiles = 4096;                // per stencil kernel
+constexpr int kMaxTiles = 4096;                // receiver tiles
+constexpr size_t kMaxWalkTiles = kMaxCells / 3 / fs::kWalkH + 1;  // 3 cells wide
 constexpr int kMaxDevices = 64;
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
 // Regions of the scratch array, each 256-byte aligned.
 constexpr size_t kOffCtl = 0;
-constexpr size_t kOffRctl = align256(kOffCtl + sizeof(fs::Ctl));
-constexpr size_t kOffDesc = align256(kOffRctl + sizeof(fs::RealCtl));
+constexpr size_t kOffDesc = align256(kOffCtl + sizeof(fs::Ctl));
 constexpr size_t kOffRtiles = align256(kOffDesc + sizeof(fs::RealDesc));
-constexpr size_t kOffDtiles = align256(kOffRtiles + kMaxTiles * sizeof(fs::Tile));
-constexpr size_t kOffTab = align256(kOffDtiles + kMaxTiles * sizeof(fs::Tile));
-constexpr size_t kOffEnt = align256(kOffTab + kTabRecords * fs::kTabStride * sizeof(double));
-constexpr size_t kOffPar = align256(kOffEnt + kMaxCells * sizeof(int32_t));
-constexpr size_t kOffAmb = align256(kOffPar + kMaxCells * sizeof(int32_t));
+constexpr size_t kOffWtiles = align256(kOffRtiles + kMaxTiles * sizeof(fs::Tile));
+constexpr size_t kOffTab = align256(kOffWtiles + kMaxWalkTiles * sizeof(fs::Tile));
+constexpr size_t kOffAmb = align256(kOffTab + kTabRecords * fs::kTabStride * sizeof(double));
 constexpr size_t kOffAmbR = align256(kOffAmb + kMaxCells * sizeof(int32_t));
-constexpr size_t kOffLvl = align256(kOffAmbR + kMaxCells * sizeof(int32_t));
-constexpr size_t kOffAcc = align256(kOffLvl + (kMaxCells + 2) * sizeof(int32_t));
-// rec keeps fs::kRecPad bytes on both sides (read, never written, by the
-// donor kernel); acc before it is not written while that kernel runs.
-constexpr size_t kOffRec = align256(kOffAcc + kMaxCells * sizeof(uint32_t) + fs::kRecPad);
-constexpr size_t kOffMask = align256(kOffRec + kMaxCells + fs::kRecPad);
-constexpr size_t kOffPdir = align256(kOffMask + kMaxCells);
-constexpr size_t kScratchBytes = align256(kOffPdir + kMaxCells);
+constexpr size_t kOffCount = align256(kOffAmbR + kMaxCells * sizeof(int32_t));
+constexpr size_t kOffRec = align256(kOffCount + kMaxCells * sizeof(uint32_t));
+constexpr size_t kOffTiles = align256(kOffRec + kMaxCells);
+constexpr size_t kTileScratch = align256(kMaxWalkTiles * fs::kWalkTileBytes + 16 * 256);
+constexpr size_t kScratchBytes = kOffTiles + kTileScratch;
 
 // The scratch. Host code must not use this name as a device address (on the
 // host it is only a stand-in); the address comes from cudaGetSymbolAddress.
@@ -78,15 +73,12 @@ static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
 // Host copies for the parameters last uploaded: erosion table, tiles.
 static double g_host_tab[kTabRecords * fs::kTabStride];
-static fs::Tile g_host_tiles[2][kMaxTiles];
+static fs::Tile g_host_tiles[2][kMaxTiles];  // receiver and walk tiles
 
 struct DeviceState {
   bool ready = false;
   unsigned char *base = nullptr;  // device address of g_scratch
-  int sms = 0;
-  int erode_bps[3] = {0, 0, 0};  // k_erode blocks per SM for each n mode
-  int order_bps = 2;
-  int accum_bps = 1;
+  fs::TileRoom room[3];          // per n mode
   bool tab_valid = false;
   fs_params tab_params{};
 };
@@ -118,33 +110,15 @@ int setup_device(int dev, DeviceState &d) {
   // first call on this device, or the module was reloaded (the array is
   // zeroed and may sit elsewhere): nothing cached about it holds any more
   d = DeviceState{};
-  e = fs::prepare_walk_kernels();
-  if (e != cudaSuccess) return cuda_fail(e, "walk smem attribute");
+  if (fs::tile_bytes(kMaxWalkTiles) > kTileScratch) return fail(FS_ERR_CUDA, "scratch too small");
   int sms = 0;
   e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
   for (int nm = 0; nm < 3; nm++) {
-    int occ = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fs::walk_kernel_ptr(nm, true),
-                                                      fs::walk_threads(), fs::walk_smem_bytes(1));
-    if (e != cudaSuccess) return cuda_fail(e, "occupancy");
-    if (occ < 1) return fail(FS_ERR_CUDA, "walk kernel cannot be resident");
-    d.erode_bps[nm] = occ < 2 ? occ : 2;
+    e = fs::prepare_tile_kernels(nm, sms, &d.room[nm]);
+    if (e != cudaSuccess) return cuda_fail(e, "tile kernels");
+    if (d.room[nm].queued < 1) return fail(FS_ERR_CUDA, "tile kernel cannot be resident");
   }
-  // k_order at 2 blocks per SM: the autotuner's choice on every single grid
-  // measured (3 blocks per SM took ~25% longer)
-  int occ = 0;
-  d.order_bps = 2;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fs::order_kernel_ptr(true, 2),
-                                                    fs::walk_threads(), fs::walk_smem_bytes(1));
-  if (e != cudaSuccess) return cuda_fail(e, "occupancy");
-  if (occ < 2) return fail(FS_ERR_CUDA, "order kernel cannot be resident");
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fs::accum_kernel_ptr(true),
-                                                    fs::walk_threads(), fs::walk_smem_bytes(1));
-  if (e != cudaSuccess) return cuda_fail(e, "occupancy");
-  if (occ < 1) return fail(FS_ERR_CUDA, "accumulation kernel cannot be resident");
-  d.accum_bps = occ < fs::kAccumMaxBps ? occ : fs::kAccumMaxBps;
-  d.sms = sms;
   d.base = static_cast<unsigned char *>(ptr);
   d.ready = true;
   return FS_OK;
@@ -170,12 +144,12 @@ extern "C" int fs_step_noalloc(double *d_h, int width, int height, const fs_para
       !std::isfinite(p.keq) || !std::isfinite(p.neq) || !std::isfinite(p.meq) ||
       !std::isfinite(p.ueq) || !std::isfinite(p.dt))
     return fail(FS_ERR_ARG, "parameters must be finite, dr and cell_area > 0, tol >= 0");
-  fs::Tile *rt = g_host_tiles[0], *dt = g_host_tiles[1];
+  fs::Tile *rt = g_host_tiles[0], *wt = g_host_tiles[1];
 
   std::lock_guard<std::mutex> lock(g_mutex);
   const int nrt = fs::append_tiles(0, 0, width, height, rt, kMaxTiles);
-  const int ndt = fs::append_tiles(1, 0, width, height, dt, kMaxTiles);
-  if (nrt < 0 || ndt < 0) return fail(FS_ERR_ARG, "grid too elongated for the static tile list");
+  const int nwt = fs::append_walk_tiles(0, width, height, wt, kMaxWalkTiles);
+  if (nrt < 0 || nwt < 0) return fail(FS_ERR_ARG, "grid too elongated for the static tile list");
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
@@ -185,10 +159,9 @@ extern "C" int fs_step_noalloc(double *d_h, int width, int height, const fs_para
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
   fs::Ctl *ctl = reinterpret_cast<fs::Ctl *>(d.base + kOffCtl);
-  fs::RealCtl *rctl = reinterpret_cast<fs::RealCtl *>(d.base + kOffRctl);
   fs::RealDesc *desc = reinterpret_cast<fs::RealDesc *>(d.base + kOffDesc);
   fs::Tile *d_rt = reinterpret_cast<fs::Tile *>(d.base + kOffRtiles);
-  fs::Tile *d_dt = reinterpret_cast<fs::Tile *>(d.base + kOffDtiles);
+  fs::Tile *d_wt = reinterpret_cast<fs::Tile *>(d.base + kOffWtiles);
   double *tab = reinterpret_cast<double *>(d.base + kOffTab);
 
   if (!d.tab_valid || !same_params(d.tab_params, p)) {
@@ -213,9 +186,7 @@ extern "C" int fs_step_noalloc(double *d_h, int width, int height, const fs_para
   rd.lvl_base = 0;
   rd.nring = fs::ring_cells(width, height);
   rd.u_dt = p.ueq * p.dt;
-  rd.tol = p.tol;
-  std::memcpy(&rd.tol_bits, &p.tol, sizeof(double));
-  rd.tol_lo_f = fs::tol_lower_float(p.tol);
+  fs::set_tolerance(&rd, p.tol);
   rd.g_orth = static_cast<float>(1.0 / p.dr_orth);
   rd.g_diag = static_cast<float>(1.0 / p.dr_diag);
   rd.gmax = rd.g_orth > rd.g_diag ? rd.g_orth : rd.g_diag;
@@ -229,40 +200,32 @@ extern "C" int fs_step_noalloc(double *d_h, int width, int height, const fs_para
   fs::StepArgs a{};
   a.h = d_h;
   a.rec = reinterpret_cast<int8_t *>(d.base + kOffRec);
-  a.mask = reinterpret_cast<uint8_t *>(d.base + kOffMask);
-  a.ent = reinterpret_cast<int32_t *>(d.base + kOffEnt);
-  a.pdir = reinterpret_cast<uint8_t *>(d.base + kOffPdir);
-  a.par = reinterpret_cast<int32_t *>(d.base + kOffPar);
-  a.acc = reinterpret_cast<uint32_t *>(d.base + kOffAcc);
   a.amb = reinterpret_cast<int32_t *>(d.base + kOffAmb);
   a.amb_r = reinterpret_cast<int32_t *>(d.base + kOffAmbR);
-  a.lvl_off = reinterpret_cast<int32_t *>(d.base + kOffLvl);
   a.desc = desc;
-  a.rctl = rctl;
   a.ctl = ctl;
   a.nreal = 1;
   a.rtiles = d_rt;
   a.nrtiles = nrt;
-  a.dtiles = d_dt;
-  a.ndtiles = ndt;
+  fs::tile_carve(&a.tb, d.base + kOffTiles, nwt);
+  a.tb.tiles = d_wt;
+  a.tb.n = nwt;
+  a.tb.desc = desc;
+  a.tb.count = reinterpret_cast<uint32_t *>(d.base + kOffCount);
   a.nmode = (p.neq == 1.0) ? fs::kNOne : (p.neq == 2.0) ? fs::kNTwo : fs::kNGeneral;
   a.neq = p.neq;
   a.do_erode = 1;
-  a.stamp = 0;
   a.timeout_ns = 2000000000ull;
 
   // Start state: descriptors and tiles of this grid, control words zeroed,
-  // rings without receivers, ring-0 donor masks zero, rings at the head of
-  // level 0.
+  // rings without receivers.
   e = cudaMemcpyAsync(desc, &rd, sizeof(rd), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && nrt > 0)
     e = cudaMemcpyAsync(d_rt, rt, nrt * sizeof(fs::Tile), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess && ndt > 0)
-    e = cudaMemcpyAsync(d_dt, dt, ndt * sizeof(fs::Tile), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(d_wt, wt, nwt * sizeof(fs::Tile), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(ctl, 0, sizeof(fs::Ctl), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(a.rec, 0xff, size, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(a.mask, 0, size, s);
-  if (e == cudaSuccess) e = fs::launch_place_rings(a.ent, width, height, s);
   // NaN/Inf in the caller's field is refused before any timestep, like
   // fs_set_elevation refuses it
   if (e == cudaSuccess) e = fs::launch_check_finite(d_h, size, ctl, s);
@@ -278,10 +241,11 @@ extern "C" int fs_step_noalloc(double *d_h, int width, int height, const fs_para
   for (int i = 0; i < nsteps; i++) {
     e = cudaMemsetAsync(reinterpret_cast<char *>(ctl) + fs::kCtlResetOffset, 0,
                         fs::kCtlResetBytes, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(rctl, 0, sizeof(fs::RealCtl), s);
     if (e == cudaSuccess) e = fs::launch_receivers_fast(a, s);
-    if (e == cudaSuccess) e = fs::launch_donors_level0(a, s);
-    if (e == cudaSuccess) e = fs::launch_walk(a, d.sms, d.order_bps, d.accum_bps, d.erode_bps[a.nmode], s);
+    if (e == cudaSuccess) e = fs::launch_tile_drain(a, s);
+    if (e == cudaSuccess) e = fs::launch_tile_links(a, s);
+    if (e == cudaSuccess) e = fs::launch_tile_erode(a, d.room[a.nmode], s);
+    if (e == cudaSuccess) e = fs::launch_tile_rest(a, d.room[a.nmode], s);
     if (e != cudaSuccess) return cuda_fail(e, "timestep launch");
   }
   fs::Ctl h_ctl;

@@ -58,21 +58,19 @@ METRIC = "cell-steps/s at 10000^2 FP64"
 UNIT = "cell-steps/s"
 SIDE = 10000
 RUN_NSTEP = 20            # run(20) executes 21 timesteps
-# Algorithmic bytes per cell for each kernel in this layout (h f64, rec i8,
-# mask u8, stack i32, cnt u32): each array the kernel must touch, once.
+# Algorithmic bytes per cell for each kernel of the tile walk (h f64, rec i8):
+# each array the kernel must touch, once.
 ALG_BYTES = {
     "receivers": 8 + 1,                     # h read, rec write
-    "donors_level0": 1 + 1,                 # rec read, mask write (+ pit list)
-    "order": 4 + 1 + 4 + 1 + 4 + 4,
-    # k_order: entry read, mask read, entry + direction + receiver-position
-    # write, unit count write
-    "accum": 4 + 4 + 4,
-    # k_accum: own count and receiver position read, reduction into the
-    # receiver's count
-    "erode": 4 + 1 + 4 + 8 + 8,
-    # k_erode: entry, direction, count, h read, h write
+    "drain": 1 + 1 + 0.5 + 2,
+    # k_tile_drain: rec read; cell codes, bit planes and counts inside the
+    # tile written
+    "links": 0.1 * 4,                       # k_tile_links: the tiles' edges
+    "erode": 2 + 1 + 0.5 + 8 + 8,
+    # k_tile_rooted / k_tile_resident: counts, codes, planes, h read, h write
+    "rest": 0.04 * (2 + 8 + 4 + 8 + 8),     # k_tile_pull: the cells left, 4%
 }
-# k_erode leans on the FP64 pipe: per eroded cell fact*dh and the
+# The erosion uses the FP64 pipe: per eroded cell fact*dh and the
 # division's one multiplication (its residual and rounding run in integer
 # arithmetic), plus h0 - hn and h0 - q unless those run in integer
 # arithmetic too (the autotuner's erode_int_sub); the uplift always runs in
@@ -84,6 +82,17 @@ def erode_fp64_per_cell(int_sub: bool) -> int:
 
 FP64_PEAK_TFLOPS = 1.59 * 152 * 2.07e9 / 1e12
 STEP_ALG_BYTES = 79        # compulsory streaming bytes per cell-step with int32 receivers
+
+
+def kernel_split(t, nsteps: int) -> dict:
+    """Milliseconds per timestep and kernel from fs_get_phase_times."""
+    return {"receivers": t[0] / nsteps, "drain": t[1] / nsteps, "links": t[7] / nsteps,
+            "erode": t[8] / nsteps, "rest": t[9] / nsteps}
+
+
+# launches a timestep: receivers, fix-up, drain, links, then one kernel where
+# the tiles fit the GPU at once, else rooted, pull, mark, queue
+LAUNCHES_LARGE, LAUNCHES_RESIDENT = 8, 5
 
 
 def grid_config(side: int) -> dict:
@@ -418,9 +427,8 @@ def ensemble_result(pkg, n, side, nsteps, seed, rank, ws, dist, local, walk="aut
     shape = "equal-size" if side > 0 else "ragged"
     side_desc = f"{side}" if side > 0 else "log-U[256,2048]"
     peak, peak_kind = load_peaks()
-    kern = {"receivers": t[0], "donors_level0": t[1], "order": t[7], "accum": t[9],
-            "erode": t[8]}
-    dom = max(("order", "accum", "erode"), key=kern.get)
+    kern = kernel_split(t, 1)
+    dom = max(("receivers", "drain", "erode"), key=kern.get)
     achieved = ALG_BYTES[dom] * cells / (kern[dom] * 1e-3) / 1e9
     return {
         "metric": f"ensemble realizations/s ({nsteps}-timestep runs)",
@@ -442,7 +450,7 @@ def ensemble_result(pkg, n, side, nsteps, seed, rank, ws, dist, local, walk="aut
                      "unit": "GB/s", "frac": achieved / peak, "traffic": None,
                      "alg_bytes_per_cell": ALG_BYTES[dom],
                      "peak_source": f"{peak_kind} hbm_gbs", "kernel_ms": kern},
-        "gpu_launches": 6 * nsteps,
+        "gpu_launches": (LAUNCHES_RESIDENT if tune.get("cta_walk") else LAUNCHES_LARGE) * nsteps,
         "clocks": clk.summary(),
     }
 
@@ -752,9 +760,7 @@ def run_sweep(args, dist, rank, ws, local):
                "cell_steps_per_s": ws * side * side * nstep / dev_s,
                "run_wall_s": wall,
                "run_cell_steps_per_s": ws * side * side * nstep / wall,
-               "kernel_ms": {"receivers": t[0] / nstep, "donors_level0": t[1] / nstep,
-                             "order": t[7] / nstep, "accum": t[9] / nstep,
-                             "erode": t[8] / nstep}}
+               "kernel_ms": kernel_split(t, nstep)}
         if rank == 0 and ws == 1 and not args.no_cpu_baseline and side <= 10000:
             nst = int(max(1, min(nstep, 4e7 / (side * side))))
             v, kind, thr, _ = cpu_sample(side, nst, prefer_reference=False)
@@ -826,7 +832,7 @@ def run_refconst(args, dist, rank, ws, local):
             "kernel_ms": {"receivers": t[0] / args.steps, "donors_level0": t[1] / args.steps,
                           "order": t[7] / args.steps, "accum": t[9] / args.steps,
                           "erode": t[8] / args.steps},
-            "gpu_launches": 6 * args.steps,
+            "gpu_launches": LAUNCHES_LARGE * args.steps,
             "cpu_baseline": cpu,
             "clocks": clk.summary(),
         }), flush=True)
@@ -890,13 +896,9 @@ def run_deep(args, dist, rank, ws, local):
             "config": {"workload": f"{side}x{side} FP64, Philox initial field, K 1e-5 m 0.6 "
                                    f"n 1 U 5e-3 dt 1000 dx 100, after {DEEP_SPINUP} "
                                    "untimed timesteps", "levels": levels, "launch": tune},
-            "kernel_ms": {"receivers": t[0] / nsteps, "donors_level0": t[1] / nsteps,
-                          "order": t[7] / nsteps, "accum": t[9] / nsteps,
-                          "erode": t[8] / nsteps},
-            "per_level_us": {"order": 1e3 * t[7] / nsteps / levels,
-                             "accum": 1e3 * t[9] / nsteps / levels,
-                             "erode": 1e3 * t[8] / nsteps / levels},
-            "gpu_launches": 6 * nsteps,
+            "kernel_ms": kernel_split(t, nsteps),
+            "per_level_us": {"erode": 1e3 * t[8] / nsteps / levels},
+            "gpu_launches": LAUNCHES_RESIDENT * nsteps,
             "cpu_baseline": cpu,
             "clocks": clk.summary(),
         }), flush=True)
@@ -1019,14 +1021,11 @@ def main():
     split_total_ms = float(t[3])
     cells = side * side
     value = ws * cells * args.steps / (total_ms * 1e-3)
-    # receivers filter + fix-up, donors/level 0, ordering, accumulation,
-    # erosion: six launches a timestep
-    launches = 6 * args.steps
+    launches = LAUNCHES_LARGE * args.steps
 
     # ---- roofline of the dominant kernel ----------------------------------
     peak, peak_kind = load_peaks()
-    kern = {"receivers": t[0], "donors_level0": t[1], "order": t[7], "accum": t[9],
-            "erode": t[8]}
+    kern = kernel_split(t, 1)
     dom = max(kern, key=kern.get)
     per_launch_ms = kern[dom] / args.steps
     achieved = ALG_BYTES[dom] * cells / (per_launch_ms * 1e-3) / 1e9
@@ -1034,9 +1033,7 @@ def main():
                 "unit": "GB/s", "frac": achieved / peak, "traffic": None,
                 "alg_bytes_per_cell": ALG_BYTES[dom], "peak_source": f"{peak_kind} hbm_gbs",
                 "kernel_ms": {k: v / args.steps for k, v in kern.items()},
-                "walk_split_ms": {"ordering": t[4] / args.steps,
-                                  "accumulation": t[5] / args.steps,
-                                  "erosion": t[6] / args.steps}}
+                "walk_ms": t[2] / args.steps}
     # the erosion kernel against the FP64 pipe (eroded cells: all but level 0)
     lid, _ = m.levels()
     eroded = int(np.count_nonzero(lid >= 1))

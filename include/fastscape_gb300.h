@@ -157,11 +157,15 @@ int64_t fs_steps_executed(const fs_model *m);
  * since the last reset, measured with CUDA events on the model's stream
  * (enabled by fs_set_timing(m, FS_TIMING_KERNELS)). ms[] holds FS_NUM_TIMERS
  * values:
- *   0 receiver kernels, 1 donor/level-0 kernel, 2 level walk (both of
- *   its kernels), 3 whole timed calls (first event to last),
- *   4..6 split of the level walk measured inside it by the GPU clock
- *        (ordering, accumulation, uplift+erosion),
- *   7 ordering kernel, 8 erosion kernel, 9 accumulation kernel (events). */
+ *   0 receiver kernels, 1 drainage inside the tiles, 2 everything after it,
+ *   3 whole timed calls (first event to last),
+ *   4..6 timer 2's parts: drainage between the tiles; erosion of the trees that
+ *        leave their tile, for grids of more tiles than the GPU holds at once;
+ *        the other trees' (of smaller grids: all) erosion,
+ *   7, 9, 8 the same, under the numbers of the ordering, accumulation and
+ *        erosion kernels that they replace.
+ * A batch on the per-realization walk has donor masks in 1, ordering and
+ * accumulation in 4 and 7, erosion in 6 and 8. */
 #define FS_NUM_TIMERS 10
 /* Timing modes: FS_TIMING_KERNELS launches each timestep's kernels directly
  * with events between them (fills every timer); FS_TIMING_CALL keeps the
@@ -180,7 +184,8 @@ int fs_use_int_sub(fs_model *m, int enable);
 int fs_launch_config(const fs_model *m, int *order_bps, int *erode_bps, int *graph,
                      int *erode_int_sub);
 
-/* Limit (milliseconds) on every grid-wide barrier wait; default 2000. */
+/* Limit (milliseconds) on every wait of one block for another's progress;
+ * default 2000. */
 int fs_set_barrier_timeout(fs_model *m, double ms);
 
 /* Waits for the model's stream. */
@@ -196,9 +201,7 @@ const char *fs_version(void);
 /* ---- Ragged batches ------------------------------------------------------
  * Many independent realizations, each with its own grid size and constants
  * (all sharing the slope exponent n), advanced together: one launch sequence
- * per timestep for the whole batch, all realizations walking their levels in
- * lock step so one grid barrier per level serves every realization. The
- * reference has no batch; each realization behaves exactly like a model of
+ * per timestep for the whole batch. The reference has no batch; each realization behaves exactly like a model of
  * its own (same results bit for bit). */
 typedef struct fs_batch fs_batch;
 
@@ -232,29 +235,29 @@ int fs_batch_use_graph(fs_batch *b, int enable);
  * (1) or on the FP64 pipe (0, default); identical results, different speed
  * (fs_batch_autotune picks). Ignored for other n. */
 int fs_batch_use_int_sub(fs_batch *b, int enable);
-/* Times every launch configuration (blocks per SM of the ordering and
- * erosion kernels, graph or direct; for n = 1 or 2 then the best of these with
- * the erosion's elevation subtractions in integer arithmetic) over
+/* Times every launch configuration (graph or direct; for n = 1 or 2 then the
+ * better of these with the erosion's elevation subtractions in integer
+ * arithmetic) over
  * probe_steps timesteps of the batch's own state, restores the state and
- * keeps the fastest; chosen[0] = erosion kernel blocks per SM, chosen[1] =
- * graph (fs_batch_launch_config reports every choice). The level walk is set
- * by size: per realization (fs_batch_use_cta_walk) when the batch has more
- * than one realization and none has more than 2^19 cells, grid-wide
- * otherwise. Results do not depend on the configuration. */
+ * keeps the fastest; chosen[0] = 2 (the erosion's blocks per SM of earlier
+ * versions), chosen[1] = graph (fs_batch_launch_config reports every choice).
+ * The per-realization walk is chosen (fs_batch_use_cta_walk) when the batch
+ * has more than one realization and none has more than 2^19 cells. Results do
+ * not depend on the configuration. */
 int fs_batch_autotune(fs_batch *b, int probe_steps, int *chosen);
-/* The launch configuration in use: blocks per SM of the ordering kernel and
- * of the erosion kernel, graph replay (0/1), integer subtractions in the
+/* The launch configuration in use: blocks per SM of the ordering kernel
+ * (fs_get_levels) and 2, graph replay (0/1), integer subtractions in the
  * erosion (0/1). Any pointer may be NULL. */
 int fs_batch_launch_config(const fs_batch *b, int *order_bps, int *erode_bps,
                            int *graph, int *erode_int_sub);
 int fs_batch_synchronize(const fs_batch *b);
 
-/* Level walk of a batch: 0 = grid-wide (every realization walks its levels
- * in lock step, one grid barrier per level for the batch), 1 = one CTA per
- * realization (block barriers only; for batches of many small realizations
- * whose hundreds of levels each hold a few thousand cells). Identical
- * results; fs_batch_autotune picks by realization size. A launch that covers a single
- * realization always walks grid-wide. No reference counterpart. */
+/* Walk of a batch: 0 = tile by tile, as of a single grid; 1 = one CTA per
+ * realization (for batches of many small realizations whose hundreds of
+ * levels each hold a few thousand cells), where the batch's tiles do not all
+ * fit the GPU at once. Identical results; fs_batch_autotune picks by
+ * realization size. A launch that covers a single realization always walks
+ * tile by tile. No reference counterpart. */
 int fs_batch_use_cta_walk(fs_batch *b, int enable);
 int fs_batch_walk_mode(const fs_batch *b, int *cta);
 
@@ -315,7 +318,7 @@ int fs_batch_get_shape(const fs_batch *b, int r, int *width, int *height);
  * may not allocate device memory while running (a host application that
  * owns all device memory through its own pool, a latency-critical loop where
  * cudaMalloc/cudaFree would synchronize the device, a plugin with a fixed
- * footprint). All scratch (~24 MB) is one static device array in the
+ * footprint). All scratch (~50 MB) is one static device array in the
  * library, held on every GPU that loads it until the process exits, shared
  * by all calls and keeping the last call's contents: calls that overlap on
  * the GPU race. The library itself serializes its calls (a lock, and each
