@@ -24,9 +24,9 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long *p) {
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
   unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
 
@@ -238,7 +238,7 @@ __device__ __forceinline__ uint64_t sub_sterbenz(uint64_t x, uint64_t y) {
 
 // -RN(num/D) on bit patterns, given Rn = -R, R = RN(1/D), in one FP64
 // operation: q0n = RN(num*Rn) = -RN(num*R) (RN is symmetric), then
-// quotient_tabled_bits (fs_bits.h). tests/native/division_check.cpp replays it
+// quotient_tabled_bits (fs_bits.h). tests/native/tile_arith_check.cpp replays it
 // on the host against the IEEE division, near rounding midpoints included. It
 // replaces Markstein's correction q1 = RN(q0 + r0*R) with r0 = num - q0*D by a
 // fused multiply-add (P. Markstein, IBM J. Res. Dev. 34(1), 1990), which cost
@@ -317,15 +317,20 @@ __device__ __forceinline__ TabN1 load_tab_n1(const unsigned long long *Tb) {
 // an FP32 test on truncated magnitudes (each within 2^-23 relative, flushed
 // below 2^-126) with 2^-21 of slack proves it for almost every cell without
 // the subtraction.
-// Most cells' magnitudes are settled by their upper words alone: with |q| <
-// tol (1 - 2^-8) and |y| 2^-48 < tol 2^-9 the same bound holds.
-__device__ __forceinline__ bool step_below_tol(uint64_t qn, uint64_t y, const RealDesc &d) {
-  if (((uint32_t)(qn >> 32) & 0x7FFFFFFFu) < d.tol_q_hi &&
-      ((uint32_t)(y >> 32) & 0x7FFFFFFFu) < d.tol_y_hi)
-    return true;
+__device__ __forceinline__ bool step_below_tol(uint64_t qn, uint64_t y, const Tolerance &tl) {
   const float qf = fabsf(trunc_bits_to_float(qn));
   const float yf = fabsf(trunc_bits_to_float(y));
-  return qf * (1.f + 0x1p-21f) + yf * 0x1p-48f <= d.tol_lo_f;
+  return qf * (1.f + 0x1p-21f) + yf * 0x1p-48f <= tl.lo_f;
+}
+
+// Most steps are settled by the upper words alone, with |y| 2^-48 < tol 2^-9:
+// 1: |RN(x - y)| <= tol, as |q| < tol (1 - 2^-8) (the bound above); -1: it is
+// above, as |q| > tol (1 + 2^-7) and |RN(x - y)| >= (|q| - 2^-52 (|y| + |q|))
+// (1 - 2^-53); 0: not settled.
+__device__ __forceinline__ int step_against_tol(uint64_t q, uint64_t y, const Tolerance &tl) {
+  const uint32_t qh = (uint32_t)(q >> 32) & 0x7FFFFFFFu;
+  if (((uint32_t)(y >> 32) & 0x7FFFFFFFu) >= tl.y_hi) return 0;
+  return qh < tl.q_hi ? 1 : qh > tl.above_hi && qh < 0x7FF00000u ? -1 : 0;
 }
 
 // RN(x + y), y = -q with |q| far below x > 0 (a Newton correction): in
@@ -370,7 +375,10 @@ __device__ __forceinline__ uint64_t ffma_bits(uint64_t a, uint64_t b, uint64_t c
 __device__ __forceinline__ uint64_t fdiv_rn_bits(uint64_t nb, uint64_t db) {
   const uint64_t an = nb & ~kSignBit, ad = db & ~kSignBit;
   if ((unsigned)((int)(an >> 52) - 924) <= 200u && (unsigned)((int)(ad >> 52) - 924) <= 200u) {
-    const uint32_t rb = __float_as_uint(__frcp_rn(trunc_bits_to_float(ad)));
+    // |den| truncated to FP32: its exponent is in range
+    const uint32_t hi = (uint32_t)(ad >> 32);
+    const uint32_t rb = __float_as_uint(__frcp_rn(__uint_as_float(
+        (((hi >> 20) - 896u) << 23) | __funnelshift_l((uint32_t)ad, hi & 0xFFFFFu, 3))));
     // widen the positive normal FP32 reciprocal to FP64 bits
     const uint64_t r0 = ((uint64_t)((rb >> 23) + 896) << 52) | ((uint64_t)(rb & 0x7FFFFFu) << 29);
     const uint64_t e = ffma_bits(ad ^ kSignBit, r0, 0x3FF0000000000000ull);  // 1 - |den| r0
@@ -411,7 +419,7 @@ __device__ __forceinline__ uint64_t sub_gen(uint64_t x, uint64_t y) {
 // iterates without the subtraction. With ISUB the subtractions run in
 // integer arithmetic.
 template <bool ISUB>
-__device__ __forceinline__ uint64_t erode_cell_n2(const RealDesc &d, double neq, Ctl *ctl,
+__device__ __forceinline__ uint64_t erode_cell_n2(const Tolerance &tl, double neq, Ctl *ctl,
                                                   uint64_t factb, uint64_t h0, uint64_t hn) {
   auto sub = [](uint64_t x, uint64_t y) { return ISUB ? sub_gen(x, y) : fadd_bits(x, y ^ kSignBit); };
   constexpr uint64_t kOne = 0x3FF0000000000000ull;
@@ -430,12 +438,19 @@ __device__ __forceinline__ uint64_t erode_cell_n2(const RealDesc &d, double neq,
     const uint64_t den = fadd_bits(kOne, fmul_bits(fact2, dx));
     const uint64_t q = fdiv_rn_bits(num, den);
     const uint64_t xn = sub(x, q);
-    if (step_below_tol(q ^ kSignBit, x, d)) return xn;
+    const int step = step_against_tol(q, x, tl);
+    if (step > 0 || (step == 0 && step_below_tol(q ^ kSignBit, x, tl))) return xn;
+    if (step < 0) {  // surely not the last
+      x = xn;
+      if (it < kNewtonMaxIt) continue;
+      raise_err(ctl, FS_ERR_NEWTON, kPhaseErode);
+      return x;
+    }
     const uint64_t df = sub(xn, x);
     x = xn;
     // fabs(diff) > tol as an integer compare (a NaN diff stops the loop)
     const long long m = (long long)(df & ~kSignBit);
-    if (!(m > d.tol_bits && m <= 0x7FF0000000000000ll)) return x;
+    if (!(m > tl.bits && m <= 0x7FF0000000000000ll)) return x;
     if (it >= kNewtonMaxIt) {
       raise_err(ctl, FS_ERR_NEWTON, kPhaseErode);
       return x;
@@ -460,7 +475,7 @@ __device__ __forceinline__ uint64_t erode_cell_n2(const RealDesc &d, double neq,
 // arrives, which pays where the pipe, not latency, limits the erosion (the
 // autotuner decides per workload).
 template <bool ISUB>
-__device__ __forceinline__ uint64_t erode_cell_n1(const RealDesc &d, Ctl *ctl,
+__device__ __forceinline__ uint64_t erode_cell_n1(const Tolerance &tl, Ctl *ctl,
                                                   const unsigned long long *Tb, TabN1 t,
                                                   uint64_t h0, uint64_t hn) {
   const uint64_t factb = t.fact;
@@ -469,13 +484,14 @@ __device__ __forceinline__ uint64_t erode_cell_n1(const RealDesc &d, Ctl *ctl,
   const uint64_t num = fmul_bits(factb, dh);
   const uint64_t qn = neg_div_rn_bits(num, D, Rn);  // -q
   const uint64_t x1 = ISUB ? sub_far(h0, qn ^ kSignBit) : fadd_bits(h0, qn);
-  if (step_below_tol(qn, h0, d)) return x1;
+  const int step = step_against_tol(qn, h0, tl);
+  if (step > 0 || (step == 0 && step_below_tol(qn, h0, tl))) return x1;
   // diff = RN(x1 - h0); |diff| > tol as an integer compare of the
   // magnitudes' bits (a NaN diff stops the loop, as fabs(NaN) > tol is false)
   const uint64_t a = ISUB ? sub_sterbenz(x1, h0) : fadd_bits(x1, h0 ^ kSignBit);
   auto more = [&](uint64_t df) {
     const long long m = (long long)(df & ~kSignBit);
-    return m > d.tol_bits && m <= 0x7FF0000000000000ll;
+    return m > tl.bits && m <= 0x7FF0000000000000ll;
   };
   if (!more(a)) return x1;
   // second iterate: num2 = RN(a + RN(fact * RN(x1 - hn)))
@@ -488,14 +504,14 @@ __device__ __forceinline__ uint64_t erode_cell_n1(const RealDesc &d, Ctl *ctl,
   // and a step of at most one spacing <= tol ends the loop.
   if (add_pos_operand(x1)) {
     const float qe = __fdividef(fabsf(trunc_bits_to_float(num2)), trunc_bits_to_float(t.D));
-    int step;
+    int places;
     float ulp;
-    if (newton_step_in_spacing(num2, t.D, x1, qe, &step, &ulp) && ulp <= d.tol_lo_f)
-      return x1 + (uint64_t)(int64_t)step;
+    if (newton_step_in_spacing(num2, t.D, x1, qe, &places, &ulp) && ulp <= tl.lo_f)
+      return x1 + (uint64_t)(int64_t)places;
   }
   const uint64_t q2n = neg_div_rn_bits(num2, D, Rn);
   const uint64_t x2 = ISUB ? add_correction(x1, q2n) : fadd_bits(x1, q2n);
-  if (step_below_tol(q2n, x1, d)) return x2;
+  if (step_below_tol(q2n, x1, tl)) return x2;
   // third and later iterates: the reference's loop in FP64
   const double R = __longlong_as_double(__ldg(Tb + 2));
   const double fact = __longlong_as_double(factb), h0d = __longlong_as_double(h0),
@@ -520,16 +536,16 @@ __device__ __forceinline__ uint64_t erode_cell_n1(const RealDesc &d, Ctl *ctl,
 // uplifted elevation, hn the receiver's final elevation and T the table
 // record of the cell's drainage count and direction class (T[0] = fact).
 template <int NMODE>
-__device__ __forceinline__ double erode_cell(const RealDesc &d, double neq, Ctl *ctl,
+__device__ __forceinline__ double erode_cell(const Tolerance &tl, double neq, Ctl *ctl,
                                              const double *T, double h0, double hn) {
   const double fact = T[0];
   double hnew, hp, diff;
   int it;
   hnew = h0;
   hp = h0;
-  diff = 2 * d.tol;
+  diff = 2 * tl.tol;
   it = 0;
-  while (fabs(diff) > d.tol) {
+  while (fabs(diff) > tl.tol) {
     double pn, pn1;
     powers<NMODE>(hnew - hn, neq, pn, pn1);
     hnew -= (hnew - h0 + fact * pn) / (1. + fact * neq * pn1);

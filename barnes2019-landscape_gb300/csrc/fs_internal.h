@@ -51,6 +51,16 @@ struct RealCtl {
 };
 constexpr size_t kRealCtlResetBytes = 4 * sizeof(int);  // top, lvlcnt
 
+// The Newton tolerance in the forms the erosion compares with.
+struct Tolerance {
+  double tol;
+  long long bits;          // of tol (magnitude compares as integers)
+  float lo_f;              // an FP32 value <= tol*(1-2^-20)
+  uint32_t q_hi, y_hi;     // upper words at most tol*(1-2^-8)'s and
+                           // tol*2^39's (steps surely below tol)
+  uint32_t above_hi;       // and tol*(1+2^-7)'s (steps surely above)
+};
+
 // Read-only description of one realization.
 struct RealDesc {
   int W, H, size;
@@ -58,11 +68,7 @@ struct RealDesc {
   int lvl_base;            // first entry of its level table
   int nring;               // ring cells, pre-placed at ent[off, off+nring)
   double u_dt;             // ueq*dt
-  double tol;
-  long long tol_bits;      // bits of tol (magnitude compares as integers)
-  float tol_lo_f;          // an FP32 value <= tol*(1-2^-20)
-  uint32_t tol_q_hi, tol_y_hi;  // upper words at most tol*(1-2^-8)'s and
-                                // tol*2^39's (steps surely below tol)
+  Tolerance tol;
   float g_orth, g_diag, gmax;  // FP32 1/dr for the receiver filter
   double dr_orth, dr_diag;
   double rdr_orth_n, rdr_diag_n;  // -RN(1/dr) for the tabled receiver
@@ -277,7 +283,7 @@ cudaError_t launch_dfs_order(const DfsArgs &d, const int32_t *lvl_host, int nlev
                              int32_t *scratch, int32_t *out, cudaStream_t s);
 
 // Host helpers shared by the entry points.
-void set_tolerance(RealDesc *d, double tol);  // every field that tol fills
+Tolerance make_tolerance(double tol);
 // -RN(1/dr) when the tabled division covers dr (1 <= dr <= 2^60), else 0.
 double neg_recip_dr(double dr);
 int ring_cells(int W, int H);

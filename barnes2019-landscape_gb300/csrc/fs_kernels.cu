@@ -1157,14 +1157,14 @@ __global__ void __launch_bounds__(T, T == 128 ? 7 : 1024 / T) k_cta_erode(StepAr
         uint64_t hnew;
         if (NMODE == kNOne && !GENERIC) {
           const unsigned long long *Tb = reinterpret_cast<const unsigned long long *>(d.tab) + rec_at;
-          hnew = erode_cell_n1<ISUB>(d, ctl, Tb, load_tab_n1(Tb), h0, hn);
+          hnew = erode_cell_n1<ISUB>(d.tol, ctl, Tb, load_tab_n1(Tb), h0, hn);
         } else if (NMODE == kNTwo && !GENERIC) {
-          hnew = erode_cell_n2<ISUB>(d, a.neq, ctl,
+          hnew = erode_cell_n2<ISUB>(d.tol, a.neq, ctl,
                                      __ldg(reinterpret_cast<const unsigned long long *>(d.tab) + rec_at),
                                      h0, hn);
         } else {
           hnew = (uint64_t)__double_as_longlong(erode_cell<NMODE>(
-              d, a.neq, ctl, d.tab + rec_at, __longlong_as_double(h0), __longlong_as_double(hn)));
+              d.tol, a.neq, ctl, d.tab + rec_at, __longlong_as_double(h0), __longlong_as_double(hn)));
         }
         if (((hnew >> 52) & 0x7FF) == 0x7FF)  // Inf or NaN
           raise_err(ctl, FS_ERR_NONFINITE, kPhaseErode);
@@ -1420,20 +1420,23 @@ double neg_recip_dr(double dr) {
   return dr >= 1.0 && dr <= 0x1p60 ? -(1.0 / dr) : 0.0;
 }
 
-void set_tolerance(RealDesc *d, double tol) {
-  d->tol = tol;
-  std::memcpy(&d->tol_bits, &tol, sizeof(double));
+Tolerance make_tolerance(double tol) {
+  Tolerance r{};
+  r.tol = tol;
+  std::memcpy(&r.bits, &tol, sizeof(double));
   const double t = tol * (1.0 - 0x1p-20);
   float f = (float)t;
   while ((double)f > t) f = nextafterf(f, 0.f);
-  d->tol_lo_f = f;
+  r.lo_f = f;
   auto upper = [](double x) {  // x >= 0: a double whose upper word is below x's is below x
     uint64_t b;
     std::memcpy(&b, &x, sizeof(b));
     return (uint32_t)(b >> 32);
   };
-  d->tol_q_hi = upper(tol * (1.0 - 0x1p-8));
-  d->tol_y_hi = upper(tol * 0x1p39);
+  r.q_hi = upper(tol * (1.0 - 0x1p-8));
+  r.y_hi = upper(tol * 0x1p39);
+  r.above_hi = upper(tol * (1.0 + 0x1p-7));
+  return r;
 }
 
 int ring_cells(int W, int H) {

@@ -845,7 +845,7 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
     d.tile0 = b->tile0[r];
     d.id = r;
     d.u_dt = p.ueq * p.dt;
-    fs::set_tolerance(&d, p.tol);
+    d.tol = fs::make_tolerance(p.tol);
     d.g_orth = static_cast<float>(1.0 / p.dr_orth);
     d.g_diag = static_cast<float>(1.0 / p.dr_diag);
     d.gmax = std::max(d.g_orth, d.g_diag);

@@ -186,7 +186,7 @@ extern "C" int fs_step_noalloc(double *d_h, int width, int height, const fs_para
   rd.lvl_base = 0;
   rd.nring = fs::ring_cells(width, height);
   rd.u_dt = p.ueq * p.dt;
-  fs::set_tolerance(&rd, p.tol);
+  rd.tol = fs::make_tolerance(p.tol);
   rd.g_orth = static_cast<float>(1.0 / p.dr_orth);
   rd.g_diag = static_cast<float>(1.0 / p.dr_diag);
   rd.gmax = rd.g_orth > rd.g_diag ? rd.g_orth : rd.g_diag;

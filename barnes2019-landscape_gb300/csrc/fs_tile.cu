@@ -512,12 +512,13 @@ __device__ __forceinline__ int front_emit(unsigned long long m, int lane, uint16
 }
 
 // The exits whose receivers are final: donors of the final cells just outside
-// the tile.
+// the tile. Relaxed loads, all in flight at once (each acquire would wait for
+// its own, 700 clocks); a caller that goes on to read elevations fences first.
 __device__ __forceinline__ unsigned long long ready_exits(const StepArgs &a, int t, const Tile &tl,
                                                           int W, int H, const Front &f, int lane) {
   const unsigned long long *done = a.tb.done;
   auto row = [&](bool there, int tile, int y) -> unsigned long long {
-    return there ? ld_acquire_u64(done + (size_t)tile * kWalkH + y) : 0ull;
+    return there ? ld_relaxed_u64(done + (size_t)tile * kWalkH + y) : 0ull;
   };
   const bool w = tl.x0 > 0, e = tl.x0 + kWalkW < W, n = tl.y0 > 0, so = tl.y0 + kWalkH < H;
   const bool top = lane == 0, bottom = lane == 31;
@@ -623,7 +624,9 @@ __device__ __forceinline__ int find_levels(const StepArgs &a, int t, const Tile 
     if (!some || prod - dn >= 2) {
       const unsigned long long R = ready_exits(a, t, tl, W, H, f, lane) & ~(claimed | F);
       F |= R;
-      if (!some && dn == prod && !__any_sync(kFull, R != 0)) {
+      const bool found = __any_sync(kFull, R != 0);
+      if (found) __threadfence();  // the bits before the elevations
+      if (!some && dn == prod && !found) {
         if (MODE == kQueued || !__any_sync(kFull, (f.flow & ~claimed) != 0)) break;
         // waiting for the neighbours: bounded, while no tile gets further
         if ((++idle & 15u) == 0) {
@@ -656,32 +659,38 @@ __device__ __forceinline__ int find_levels(const StepArgs &a, int t, const Tile 
 // One cell on its way to being eroded.
 struct Cell {
   int c, rc;    // the cell, and its receiver's inside the tile (-1: outside)
+  bool out;     // cells of other tiles drain into it: its elevation goes there
   uint64_t h0;  // uplifted elevation
   uint64_t hx;  // the receiver's, outside
   const unsigned long long *Tb;
-  TabN1 tab;
+  ulonglong2 fd;  // F, D
+  uint64_t rn;    // -1/D
 };
 
 // The table record of drainage count k and direction dir.
 template <int NMODE, int VAR>
 __device__ __forceinline__ void cell_table(Cell &e, const RealDesc &d, uint32_t k, int dir) {
   e.Tb = reinterpret_cast<const unsigned long long *>(d.tab) + (size_t)k * kTabStride + 4 * (dir & 1);
-  if (NMODE == kNOne && VAR != 2) e.tab = load_tab_n1(e.Tb);
-  else e.tab.fact = __ldg(e.Tb);
+  if (NMODE == kNOne && VAR != 2) {
+    e.fd = __ldg(reinterpret_cast<const ulonglong2 *>(e.Tb));
+    e.rn = __ldg(e.Tb + 3);
+  } else {
+    e.fd.x = __ldg(e.Tb);
+  }
 }
 
 // The cell's final elevation from its receiver's (fastscape_RB.cpp:315-326).
 template <int NMODE, int VAR>
-__device__ __forceinline__ uint64_t cell_erode(const Cell &e, const RealDesc &d, double neq,
+__device__ __forceinline__ uint64_t cell_erode(const Cell &e, const Tolerance &tol, double neq,
                                                Ctl *ctl, uint64_t hn) {
   uint64_t h;
   if (NMODE == kNOne && VAR != 2) {
-    h = erode_cell_n1<VAR == 1>(d, ctl, e.Tb, e.tab, e.h0, hn);
+    h = erode_cell_n1<VAR == 1>(tol, ctl, e.Tb, TabN1{e.fd.x, e.fd.y, e.rn}, e.h0, hn);
   } else if (NMODE == kNTwo && VAR != 2) {
-    h = erode_cell_n2<VAR == 1>(d, neq, ctl, e.tab.fact, e.h0, hn);
+    h = erode_cell_n2<VAR == 1>(tol, neq, ctl, e.fd.x, e.h0, hn);
   } else {
     h = (uint64_t)__double_as_longlong(
-        erode_cell<NMODE>(d, neq, ctl, reinterpret_cast<const double *>(e.Tb),
+        erode_cell<NMODE>(tol, neq, ctl, reinterpret_cast<const double *>(e.Tb),
                           __longlong_as_double(e.h0), __longlong_as_double(hn)));
   }
   if (((h >> 52) & 0x7FF) == 0x7FF) raise_err(ctl, FS_ERR_NONFINITE, kPhaseErode);  // Inf or NaN
@@ -696,6 +705,7 @@ __device__ __forceinline__ void erode_levels(const StepArgs &a, int t, const Til
   const int wt = (int)threadIdx.x - 32;
   const int W = d.W;
   const uint64_t udt = (uint64_t)__double_as_longlong(d.u_dt);
+  const Tolerance tol = d.tol;
   unsigned long long *gh = reinterpret_cast<unsigned long long *>(a.h + d.off);
   const int org = tl.y0 * W + tl.x0;
   auto grid_cell = [&](int c) { return org + (c >> 6) * W + (c & 63); };
@@ -703,9 +713,11 @@ __device__ __forceinline__ void erode_levels(const StepArgs &a, int t, const Til
     Cell e;
     e.c = -1;
     e.rc = -1;
-    e.hx = 0;
+    e.h0 = e.hx = 0;
+    e.out = MODE == kQueued;
     if (i < hi) {
       e.c = s.list[i];
+      if (MODE == kResident) e.out = s.entry[e.c >> 6] >> (e.c & 63) & 1ull;
       int code;
       uint32_t k;
       uint64_t h;
@@ -723,19 +735,35 @@ __device__ __forceinline__ void erode_levels(const StepArgs &a, int t, const Til
       if (code >= kCodeExit) e.hx = __ldcg(gh + grid_cell(e.c) + nbr_off(dir, W));
       else e.rc = e.c + tile_off(dir);
       cell_table<NMODE, VAR>(e, d, k, dir);
-      e.h0 = uplift_bits(h, udt);
+      e.h0 = h;  // to be uplifted
     }
     return e;
   };
-  bool ahead = false;
+  auto turn = [&](int L) -> int {  // place among the level's workers
+    const int k = (wt >> 5) - L % (kWorkers / 32);
+    return 32 * (k < 0 ? k + kWorkers / 32 : k) + (wt & 31);
+  };
+  // nx: this thread's first cell of the level, loaded during the level before
+  // (first == L). The warps take turns: level L's first 32 cells, on deep
+  // ground often all of them, are warp L % 3's, which has loaded and uplifted
+  // them while another warp eroded the level before.
+  int first = -1;
   Cell nx;
   for (int L = MODE == kQueued ? 1 : 0;; ++L) {
     int ready;
     for (unsigned n = 0; (ready = ld_volatile_i32(&s.ready)) <= L; ++n)
       if (n > 2) __nanosleep(50);
-    if ((ready & ~kFinished) <= L) return;
+    if ((ready &= ~kFinished) <= L) return;
     __threadfence_block();
     const int lo = L ? s.end[(L - 1) % kRing] : 0, hi = s.end[L % kRing];
+    const int at = lo + turn(L);
+    Cell e = nx;
+    if (first != L && L) {
+      e = load(at, hi);
+      if (e.c >= 0) e.h0 = uplift_bits(e.h0, udt);
+    }
+    const bool more = ready > L + 1;
+    if (more) nx = load(hi + turn(L + 1), s.end[(L + 1) % kRing]);
     if (MODE != kQueued && L == 0) {
       // level 0, of which the pits rise with the land (fastscape_RB.cpp:291-295)
       for (int i = wt; i < hi; i += kWorkers) {
@@ -745,21 +773,20 @@ __device__ __forceinline__ void erode_levels(const StepArgs &a, int t, const Til
         if (MODE == kResident && (s.entry[c >> 6] >> (c & 63) & 1ull)) gh[grid_cell(c)] = h;
       }
     } else {
-      if (!ahead) nx = load(lo + wt, hi);
-      for (int i = lo + wt; i < hi; i += kWorkers) {
-        const Cell e = nx;
-        nx = load(i + kWorkers, hi);
+      for (int i = at; i < hi; i += kWorkers) {
+        if (i > at) {  // a wide level's further cells
+          e = load(i, hi);
+          e.h0 = uplift_bits(e.h0, udt);
+        }
         const uint64_t hn = e.rc >= 0 ? s.h[e.rc] : e.hx;
-        const uint64_t h = cell_erode<NMODE, VAR>(e, d, a.neq, a.ctl, hn);
+        const uint64_t h = cell_erode<NMODE, VAR>(e, tol, a.neq, a.ctl, hn);
         s.h[e.c] = h;
-        if (MODE == kQueued || (MODE == kResident && (s.entry[e.c >> 6] >> (e.c & 63) & 1ull)))
-          gh[grid_cell(e.c)] = h;
+        if (e.out) gh[grid_cell(e.c)] = h;
       }
     }
-    ahead = (ld_volatile_i32(&s.ready) & ~kFinished) > L + 1;
-    if (ahead) {
-      __threadfence_block();
-      nx = load(hi + wt, s.end[(L + 1) % kRing]);
+    if (more) {
+      first = L + 1;
+      if (nx.c >= 0) nx.h0 = uplift_bits(nx.h0, udt);
     }
     group_sync(kWorkers);
     if (wt == 0) {
@@ -863,7 +890,7 @@ __device__ __forceinline__ unsigned long long root_row(const Tile &tl, int W, in
 }
 
 template <int NMODE, int VAR>
-__global__ void __launch_bounds__(kWalkThreads, 7) k_tile_resident(StepArgs a) {
+__global__ void __launch_bounds__(kWalkThreads, 6) k_tile_resident(StepArgs a) {
   if (stopped(a.ctl)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TileSmem &s = *reinterpret_cast<TileSmem *>(smem_raw);
@@ -948,6 +975,7 @@ __global__ void __launch_bounds__(kRootedThreads, 6) k_tile_rooted(StepArgs a) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wt = (int)threadIdx.x - 32;
   constexpr int kWarps = kRootedThreads / 32, kErode = kRootedThreads - 32;
   const uint64_t udt = (uint64_t)__double_as_longlong(d.u_dt);
+  const Tolerance tol = d.tol;
   tile_stage<kRootedThreads>(a, tl, d, s.h);
   Front f;
   unsigned long long F = 0, final = 0;
@@ -1017,7 +1045,7 @@ __global__ void __launch_bounds__(kRootedThreads, 6) k_tile_rooted(StepArgs a) {
       for (int i = lo + wt; i < hi; i += kErode) {
         const Cell e = nx;
         nx = load(i + kErode, hi);
-        s.h[e.c] = cell_erode<NMODE, VAR>(e, d, a.neq, a.ctl, s.h[e.rc]);
+        s.h[e.c] = cell_erode<NMODE, VAR>(e, tol, a.neq, a.ctl, s.h[e.rc]);
       }
       nx = load(hi + wt, hi2);
     }
@@ -1078,6 +1106,7 @@ __global__ void __launch_bounds__(kPullThreads) k_tile_pull(StepArgs a) {
   const Tile tl = a.tb.tiles[t];
   const RealDesc &d = a.tb.desc[tl.r];
   const int W = d.W;
+  const Tolerance tol = d.tol;
   unsigned long long *gh = reinterpret_cast<unsigned long long *>(a.h + d.off);
   if (threadIdx.x == 0) s_fail = 0;
   __syncthreads();
@@ -1114,7 +1143,7 @@ __global__ void __launch_bounds__(kPullThreads) k_tile_pull(StepArgs a) {
           Cell e;
           e.h0 = rest.h0[q];
           cell_table<NMODE, VAR>(e, d, rest.count[q], rest.cell[q] >> 11);
-          h = cell_erode<NMODE, VAR>(e, d, a.neq, a.ctl, h);
+          h = cell_erode<NMODE, VAR>(e, tol, a.neq, a.ctl, h);
         }
         gh[g0] = h;
       }
@@ -1218,8 +1247,9 @@ __global__ void __launch_bounds__(kWalkThreads, 7) k_tile_queue(StepArgs a) {
       s.entry[lane] = 0;
       __syncwarp();
       front_load(f, a.tb.planes + (size_t)t * 256, lane);
-      own = ld_acquire_u64(a.tb.done + (size_t)t * kWalkH + lane);
+      own = ld_relaxed_u64(a.tb.done + (size_t)t * kWalkH + lane);
       F = ready_exits(a, t, tl, W, H, f, lane) & ~own;
+      __threadfence();  // the bits before the elevations
       // k_tile_pull may have finished a tree's lower part: go on above it
       const unsigned long long above = front_next(f, own, lane) & ~own;
       F |= above;
