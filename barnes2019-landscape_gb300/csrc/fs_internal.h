@@ -29,8 +29,7 @@ struct Ctl {
   int pad0[3];
   // --- reset before every timestep (from `amb` on) ---
   int amb;                 // cells queued by the receiver filter
-  unsigned int bar;        // grid-barrier arrival counter (k_order)
-  unsigned int bar3;       // grid-barrier arrival counter (k_accum)
+  unsigned int bar;        // k_test_wait's arrivals
   int left;                // cells still to erode in trees that leave their
                            // tile (k_tile_queue), or tiles finished (resident)
   unsigned int qtail, qhead;  // pushes to and pops from the tile queue
@@ -40,16 +39,11 @@ constexpr size_t kCtlResetOffset = offsetof(Ctl, amb);
 constexpr size_t kCtlResetBytes = sizeof(Ctl) - kCtlResetOffset;
 constexpr size_t kCtlCallResetBytes = 5 * sizeof(int);  // err .. abort_r
 
-// Per-realization counters of the level order; `top` and `lvlcnt` are reset
-// before every ordering.
+// Per-realization counters, reset before every ordering.
 struct RealCtl {
   int top;                 // pits appended to level 0 (after the rings)
-  int lvlcnt[3];           // rotating per-level append counters
-  int nlevels;             // levels found by the last walk
-  int total;               // cells placed in the ordering by the last walk
-  int pad[2];
+  int nlevels;             // levels found (k_cta_order_accum, k_net_follow)
 };
-constexpr size_t kRealCtlResetBytes = 4 * sizeof(int);  // top, lvlcnt
 
 // The Newton tolerance in the forms the erosion compares with.
 struct Tolerance {
@@ -219,9 +213,6 @@ struct StepArgs {
 
 // Largest batch one walk launch handles.
 constexpr int kMaxReal = 4096;
-// Shared memory the walk kernel needs for `nreal` realizations.
-size_t walk_smem_bytes(int nreal);
-
 // Kernel launchers (fs_kernels.cu). All are asynchronous on `s`.
 cudaError_t launch_receivers_exact(const StepArgs &a, cudaStream_t s);
 // hmap: a single grid's elevation as a {W, H} map of 64-bit elements with
@@ -230,15 +221,6 @@ cudaError_t launch_receivers_fast(const StepArgs &a, cudaStream_t s,
                                   const CUtensorMap *hmap = nullptr);
 bool make_receiver_map(CUtensorMap *m, const double *h, int W, int H);
 cudaError_t launch_donors_level0(const StepArgs &a, cudaStream_t s);
-// The level order: k_order and k_accum with bps blocks per SM, cooperative
-// launches over `sms` SMs.
-cudaError_t launch_order(const StepArgs &a, int sms, int bps, cudaStream_t s);
-cudaError_t launch_accum(const StepArgs &a, int sms, int bps, cudaStream_t s);
-int walk_threads();
-const void *order_kernel_ptr(bool single);
-const void *accum_kernel_ptr(bool single);
-constexpr int kAccumMaxBps = 4;      // k_accum's register budget
-cudaError_t prepare_walk_kernels();  // dynamic shared memory limit
 // The tile walk (fs_tile.cu): drainage inside the tiles, drainage between
 // them, and the counts alone or the erosion. `resident` and `queued` are the
 // blocks that k_tile_resident and k_tile_queue can keep on the GPU at once.
@@ -266,21 +248,25 @@ cudaError_t launch_no_receivers(int8_t *rec, int W, int H, cudaStream_t s);
 cudaError_t launch_test_wait(Ctl *ctl, int blocks, unsigned long long timeout_ns,
                              cudaStream_t s);
 
-// One realization's level-walk arrays, for the Braun-Willett order.
-struct DfsArgs {
+// The drainage network of one realization (fs_network.cu), for read-backs.
+struct NetArgs {
   const int8_t *rec;
-  const int32_t *ent;
-  const int32_t *par;
-  const uint8_t *pdir;
-  const uint32_t *acc;
-  int W, size;
+  const uint32_t *count;      // drainage counts (not for the levels)
+  int n, W;                   // cells, row length
+  unsigned long long *words;  // [n] scratch
 };
-// Scratch ints launch_dfs_order needs for a realization of `size` cells.
-size_t dfs_scratch_ints(int size);
-// The Braun-Willett (depth-first) order into out[size], given the level
-// offsets on the host.
-cudaError_t launch_dfs_order(const DfsArgs &d, const int32_t *lvl_host, int nlev,
-                             int32_t *scratch, int32_t *out, cudaStream_t s);
+// Levels into out[n]; rctl->nlevels becomes the number of levels.
+cudaError_t launch_net_levels(const NetArgs &a, RealCtl *rctl, Ctl *ctl, int32_t *out,
+                              cudaStream_t s);
+// First position of each tree of the depth-first order into starts, the
+// number of trees into sums[net_sums(n)].y, and the words that
+// launch_net_order turns into the order (which may take starts' place).
+int net_sums(int n);
+cudaError_t launch_net_trees(const NetArgs &a, int2 *sums, int32_t *starts, cudaStream_t s);
+cudaError_t launch_net_order(const NetArgs &a, Ctl *ctl, int32_t *out, cudaStream_t s);
+cudaError_t launch_net_receivers(const NetArgs &a, int32_t *out, cudaStream_t s);
+cudaError_t launch_net_receiver_index(const NetArgs &a, long long *out, cudaStream_t s);
+cudaError_t launch_net_area(const NetArgs &a, double cell_area, double *out, cudaStream_t s);
 
 // Host helpers shared by the entry points.
 Tolerance make_tolerance(double tol);

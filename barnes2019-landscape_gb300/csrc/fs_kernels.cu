@@ -7,17 +7,11 @@
 // settle. Its other kernels, from the receivers on, are the tile walk
 // (fs_tile.cu).
 //
-// For callers that ask for the drainage network -- levels, donor masks, the
-// depth-first order -- the reference's level order is built from a timestep's
-// receivers:
-//   k_donors_level0  donor masks (pull form of fastscape_RB.cpp:188-203) and
-//                    the level-0 frontier (fastscape_RB.cpp:221-227)
-//   k_order          persistent cooperative kernel: level-by-level ordering
-//                    (:229-251)
-//   k_accum          persistent cooperative kernel: flow accumulation back
-//                    down the levels (:262-279), by position in the order
-//   All realizations walk their levels in lock step, so one grid barrier per
-//   level serves the whole batch.
+// k_donors_level0 writes donor masks (pull form of fastscape_RB.cpp:188-203)
+// and the level-0 frontier (fastscape_RB.cpp:221-227), for the
+// per-realization walk of large batches (k_cta_order_accum, k_cta_erode) and
+// for callers that read the masks. Levels and the depth-first order are read
+// back by fs_network.cu.
 //
 // Floating point follows the reference's operation order exactly; the whole
 // file is compiled with -fmad=false so no multiply-add is contracted, every
@@ -40,42 +34,7 @@ namespace fs {
 
 namespace {
 
-constexpr int kWalkThreads = 512;
-constexpr int kWalkWarps = kWalkThreads / 32;
-constexpr int kPer = 8;   // entries per thread per expansion chunk (measured best of 4..16)
-constexpr int kLevelCache = 2048;  // level offsets a single grid's walk keeps in shared memory
-constexpr int kChunk = kPer * kWalkThreads;
-
-// Exclusive prefix over realizations of count(r) into s_pre[0..n]; the walk
-// kernel's block-wide view of how a level's work splits across the batch.
-template <class F>
-__device__ __forceinline__ int block_prefix(int n, F count, int *s_pre) {
-  const int per = (n + kWalkThreads - 1) / kWalkThreads;
-  const int r0 = threadIdx.x * per;
-  int sum = 0;
-  for (int r = r0; r < r0 + per && r < n; r++) sum += count(r);
-  int total;
-  int run = block_excl_scan(sum, total, threadIdx.x, kWalkThreads);
-  for (int r = r0; r < r0 + per && r < n; r++) {
-    s_pre[r] = run;
-    run += count(r);
-  }
-  if (threadIdx.x == 0) s_pre[n] = total;
-  __syncthreads();
-  return total;
-}
-
-// Realization of global work item g: the r with s_pre[r] <= g < s_pre[r+1]
-// (g < s_pre[n]); empty realizations are skipped because the largest such
-// r is taken.
-__device__ __forceinline__ int find_real(const int *s_pre, int n, int g) {
-  int lo = 0, hi = n;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (s_pre[mid] <= g) lo = mid; else hi = mid;
-  }
-  return lo;
-}
+constexpr int kLevelCache = 2048;  // level offsets a realization's walk keeps in shared memory
 
 // ---------------------------------------------------------------------------
 // 1. Receivers: fastscape_RB.cpp:160-182. slope = (h[c]-h[n])/dr[n], strict
@@ -578,408 +537,6 @@ __global__ void __launch_bounds__(256) k_donors_level0(StepArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// 4. Persistent level walker (cooperative launch).
-//
-// The ordering is kept as arrays indexed by position in the level order
-// (fs_internal.h): accumulation and erosion read them by position --
-// coalesced -- instead of gathering receivers, masks and counts by cell.
-// Per level, every block keeps each realization's range [lo, hi) in shared
-// memory and maps global work items (expansion chunks, 32-entry groups) to
-// realizations through a prefix over the batch.
-// ---------------------------------------------------------------------------
-template <bool SINGLE, int MINB>
-__global__ void __launch_bounds__(kWalkThreads, MINB) k_order(StepArgs a) {
-  extern __shared__ int smem[];
-  const int nreal = a.nreal;
-  int *s_lo = smem;               // per realization: current range start
-  int *s_hi = s_lo + nreal;       // and end (local positions)
-  int *s_nlev = s_hi + nreal;     // levels found so far
-  int *s_pre = s_nlev + nreal;    // prefix over the batch, nreal+1
-  __shared__ int s_cw[2][kWalkWarps];  // warp totals / prefixes of a chunk
-  __shared__ int s_cbase[2];           // the chunk's first position
-  int cbuf = 0;
-  __shared__ uint8_t s_own[kWalkWarps][32 * 8];  // (lane, direction) per donor slot of a pass
-  unsigned epoch = 0;
-  Ctl *ctl = a.ctl;
-  if (stopped(ctl)) return;
-  // A batch of one keeps its descriptor in registers and skips the
-  // realization lookups.
-  RealDesc d0;
-  if (SINGLE) d0 = a.desc[0];
-  auto desc = [&](int r) -> const RealDesc & { return SINGLE ? d0 : a.desc[r]; };
-  auto real_of = [&](int g) -> int { return SINGLE ? 0 : find_real(s_pre, nreal, g); };
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-
-  // ---- ordering: fastscape_RB.cpp:229-251 -------------------------------
-  // Level k+1 = the donors of level k. A block expands a chunk of kChunk
-  // consecutive entries of one realization; warp w covers 32*kPer of them
-  // in kPer coalesced passes (entry wbase+32q+lane). Warp scans give each
-  // entry's first-donor offset in entry order, one block scan over the
-  // warps and one atomic place the chunk, and the donors are written
-  // cooperatively (lane r writes the r-th donor of the pass), so the next
-  // level keeps this level's order. Each realization's append counter
-  // rotates over three words so a block that reads the size of level k after
-  // the barrier never races with the reset for level k+2.
-  // s_tot[L & 1]: entries of level L over the batch (double-buffered: the
-  // next level's count is summed while this one's may still be read)
-  __shared__ int s_tot[2];
-  if (threadIdx.x == 0) s_tot[0] = s_tot[1] = 0;
-  __syncthreads();
-  for (int r = threadIdx.x; r < nreal; r += kWalkThreads) {
-    const RealDesc &d = desc(r);
-    s_lo[r] = 0;
-    s_hi[r] = d.nring + ld_volatile_i32(&a.rctl[r].top);
-    s_nlev[r] = 1;
-    atomicAdd(&s_tot[0], s_hi[r]);
-    if (blockIdx.x == 0) {
-      a.lvl_off[d.lvl_base + 0] = 0;
-      a.lvl_off[d.lvl_base + 1] = s_hi[r];
-    }
-  }
-  __syncthreads();
-  int L = 0;  // level being expanded
-  for (;;) {
-    const int j = L % 3;
-    if (blockIdx.x == 0)
-      for (int r = threadIdx.x; r < nreal; r += kWalkThreads) a.rctl[r].lvlcnt[(L + 1) % 3] = 0;
-    // Passes per warp in this level's chunks: kPer, or one for a level that
-    // fits one round of one-pass chunks over the grid, so that its chunks
-    // spread over more blocks (two compiled forms: a run-time pass count
-    // slows the big levels' expansion).
-    const bool one_pass = s_tot[L & 1] <= (int)gridDim.x * kWalkThreads;
-    if (threadIdx.x == 0) s_tot[(L + 1) & 1] = 0;  // summed after this level's barrier
-    const int chunk = (one_pass ? 1 : kPer) * kWalkThreads;
-    const int nchunks = block_prefix(
-        nreal, [&](int r) { return (s_hi[r] - s_lo[r] + chunk - 1) / chunk; }, s_pre);
-    auto expand = [&](auto passes, int g) {
-      constexpr int NP = decltype(passes)::value;
-      const int r = real_of(g);
-      const RealDesc &d = desc(r);
-      const int hi = s_hi[r];
-      const int base = s_lo[r] + (g - s_pre[r]) * (NP * kWalkThreads);
-      const int wbase = base + wid * (32 * NP);
-      int32_t *ent = a.ent + d.off;
-      const uint8_t *mask = a.mask + d.off;
-      const int offk = nbr_off(lane & 7, d.W);  // lane k < 8: offset of direction k
-      // Per pass q: the entry's cell, and its donor mask with the warp's
-      // inclusive donor prefix (relative to the warp's first donor, below
-      // 32 * 8 * kPer) packed as (prefix << 8) | mask, to keep the chunk's
-      // state in registers across its barriers.
-      int cs[NP];
-      unsigned mi[NP];
-#pragma unroll
-      for (int q = 0; q < NP; q++) {
-        const int i = wbase + 32 * q + lane;
-        cs[q] = 0;
-        mi[q] = 0;
-        if (i < hi) {
-          cs[q] = __ldcg(&ent[i]);
-          mi[q] = mask[cs[q]];
-        }
-      }
-      int wtot = 0;
-#pragma unroll
-      for (int q = 0; q < NP; q++) {
-        int v = __popc(mi[q]);
-#pragma unroll
-        for (int dd = 1; dd < 32; dd <<= 1) {
-          const int x = __shfl_up_sync(kFull, v, dd);
-          if (lane >= dd) v += x;
-        }
-        mi[q] |= (unsigned)(wtot + v) << 8;  // inclusive prefix
-        wtot += __shfl_sync(kFull, v, 31);
-      }
-      // Place the chunk: prefix of the warp totals and one atomic, with two
-      // barriers; the shared words alternate between two buffers so the next
-      // chunk can fill one while this chunk's readers finish with the other.
-      if (lane == 0) s_cw[cbuf][wid] = wtot;
-      __syncthreads();
-      if (wid == 0) {
-        int w = lane < kWalkWarps ? s_cw[cbuf][lane] : 0;
-#pragma unroll
-        for (int dd = 1; dd < 32; dd <<= 1) {
-          const int x = __shfl_up_sync(kFull, w, dd);
-          if (lane >= dd) w += x;
-        }
-        if (lane < kWalkWarps) s_cw[cbuf][lane] = w;  // inclusive prefix over warps
-        const int total = __shfl_sync(kFull, w, kWalkWarps - 1);
-        if (lane == 0) s_cbase[cbuf] = total ? atomicAdd(&a.rctl[r].lvlcnt[j], total) : 0;
-      }
-      __syncthreads();
-      // position of the warp's first donor
-      const int cbase = hi + s_cbase[cbuf] + (wid ? s_cw[cbuf][wid - 1] : 0);
-      cbuf ^= 1;
-#pragma unroll
-      for (int q = 0; q < NP; q++) {
-        const int i = wbase + 32 * q + lane;
-        const unsigned msk = mi[q] & 0xFFu;
-        const int incl = (int)(mi[q] >> 8);
-        const int n_d = __popc(msk);
-        if (i < hi) {
-          a.acc[d.off + i] = 1u;  // the cell itself; donors add theirs below
-        }
-        // The pass's donors go to positions cbase + [q_lo, q_lo + q_n) in
-        // entry order. Each lane records (its lane, direction) for the slots
-        // of its donors in the warp's shared bytes; then lane t writes slot t
-        // of every 32, coalesced.
-        const int q_lo = __shfl_sync(kFull, incl - n_d, 0);
-        const int q_n = __shfl_sync(kFull, incl, 31) - q_lo;  // <= 32 * 8
-        {
-          int slot = incl - n_d - q_lo;
-          // every direction, predicated: no divergence across the warp (a
-          // loop over the set bits runs as long as the lane with most donors)
-#pragma unroll
-          for (int k = 0; k < 8; k++) {
-            if (msk >> k & 1u) s_own[wid][slot++] = (uint8_t)((lane << 3) | k);
-          }
-        }
-        __syncwarp();
-        for (int r0 = 0; r0 < q_n; r0 += 32) {
-          const int rr = r0 + lane;
-          const unsigned pk = rr < q_n ? s_own[wid][rr] : 0u;
-          const int k = pk & 7;
-          const int oc = __shfl_sync(kFull, cs[q], pk >> 3);
-          const int ok = __shfl_sync(kFull, offk, k);
-          if (rr < q_n) {
-            const int pos = cbase + q_lo + rr;
-            if (pos < d.size) {
-              ent[pos] = oc + ok;
-              a.pdir[d.off + pos] = (uint8_t)((k + 4) & 7);
-              a.par[d.off + pos] = wbase + 32 * q + (int)(pk >> 3);  // receiver's position
-            } else {
-              raise_err(ctl, FS_ERR_LEVEL_OVERFLOW, kPhaseOrder);
-            }
-          }
-        }
-        __syncwarp();  // s_own is refilled by the next pass
-      }
-        };
-    for (int g = blockIdx.x; g < nchunks; g += gridDim.x) {
-      if (one_pass) expand(std::integral_constant<int, 1>{}, g);
-      else expand(std::integral_constant<int, kPer>{}, g);
-    }
-    if (!grid_barrier(ctl, &ctl->bar, epoch, a.timeout_ns)) return;
-    // Thread r alone reads realization r's size (one load per block, not a
-    // load of one word by every thread). Every block sees the same sizes:
-    // an overflow ends the walk in all of them; other errors reach them at
-    // the next barrier's spin.
-    int any = 0, ovf = 0;
-    for (int r = threadIdx.x; r < nreal; r += kWalkThreads) {
-      const int added = ld_volatile_i32(&a.rctl[r].lvlcnt[j]);
-      s_lo[r] = s_hi[r];
-      if (added) {
-        atomicAdd(&s_tot[(L + 1) & 1], added);
-        s_hi[r] += added;
-        s_nlev[r] = L + 2;
-        any = 1;
-        if (s_hi[r] > desc(r).size) {
-          if (blockIdx.x == 0) raise_err(ctl, FS_ERR_LEVEL_OVERFLOW, kPhaseOrder);
-          ovf = 1;
-        } else if (blockIdx.x == 0) {
-          a.lvl_off[desc(r).lvl_base + L + 2] = s_hi[r];
-        }
-      }
-    }
-    if (__syncthreads_or(ovf)) return;
-    if (!__syncthreads_or(any)) break;
-    ++L;
-  }
-  // s_hi[r] is the realization's total; anything short of its size means
-  // cells that never reached base level: the receivers contain a cycle.
-  {
-    int bad = 0;
-    for (int r = threadIdx.x; r < nreal; r += kWalkThreads) {
-      if (blockIdx.x == 0) {
-        a.rctl[r].nlevels = s_nlev[r];
-        a.rctl[r].total = s_hi[r];
-      }
-      bad |= s_hi[r] != desc(r).size;
-    }
-    if (__syncthreads_or(bad)) {
-      if (tid == 0) raise_err(ctl, FS_ERR_ORDER, kPhaseOrder);
-      return;
-    }
-  }
-}
-
-// Accumulation (fastscape_RB.cpp:262-279) level by level back down to base
-// level, then the pits' uplift, after k_order has placed the levels. A
-// kernel of its own: its little per-thread state lets it run 4 blocks of
-// 512 threads per SM, hiding more of the latency of its loads.
-template <bool SINGLE>
-__global__ void __launch_bounds__(kWalkThreads, 4) k_accum(StepArgs a) {
-  extern __shared__ int smem[];
-  const int nreal = a.nreal;
-  int *s_lo = smem;
-  int *s_hi = s_lo + nreal;
-  int *s_nlev = s_hi + nreal;
-  int *s_pre = s_nlev + nreal;
-  __shared__ int s_maxlev;
-  unsigned epoch = 0;
-  Ctl *ctl = a.ctl;
-  if (stopped(ctl)) return;
-  RealDesc d0;
-  if (SINGLE) d0 = a.desc[0];
-  auto desc = [&](int r) -> const RealDesc & { return SINGLE ? d0 : a.desc[r]; };
-  auto real_of = [&](int g) -> int { return SINGLE ? 0 : find_real(s_pre, nreal, g); };
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nthreads = gridDim.x * blockDim.x;
-  const int lane = threadIdx.x & 31;
-  const int warp_global = tid >> 5, nwarps = nthreads >> 5;
-  if (threadIdx.x == 0) s_maxlev = 0;
-  __syncthreads();
-  for (int r = threadIdx.x; r < nreal; r += kWalkThreads) {
-    s_nlev[r] = __ldcg(&a.rctl[r].nlevels);
-    atomicMax(&s_maxlev, s_nlev[r]);
-  }
-  __syncthreads();
-  const int maxlev = s_maxlev;
-
-  // Level Lv of every realization as [lo_of(r), hi_of(r)) (empty past its
-  // depth), and the prefix of its 32-entry groups over the batch. A batch
-  // of one copies its level table into shared memory once (one load per
-  // entry and block) and takes each level's range from there into
-  // registers: no block barrier, scan or global load per level.
-  __shared__ int s_off[kLevelCache + 1];
-  if (SINGLE) {
-    const int n = min(maxlev, kLevelCache) + 1;
-    for (int k = threadIdx.x; k < n; k += kWalkThreads) s_off[k] = __ldcg(&a.lvl_off[d0.lvl_base + k]);
-    __syncthreads();
-  }
-  int lv_lo = 0, lv_hi = 0;
-  auto lo_of = [&](int r) -> int { return SINGLE ? lv_lo : s_lo[r]; };
-  auto hi_of = [&](int r) -> int { return SINGLE ? lv_hi : s_hi[r]; };
-  auto pre_of = [&](int r) -> int { return SINGLE ? 0 : s_pre[r]; };
-  auto level_groups = [&](int Lv) -> int {
-    if (SINGLE) {
-      if (Lv < kLevelCache) {
-        lv_lo = s_off[Lv];
-        lv_hi = s_off[Lv + 1];
-      } else {  // deeper than the cache: one load per block
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          s_lo[0] = __ldcg(&a.lvl_off[d0.lvl_base + Lv]);
-          s_hi[0] = __ldcg(&a.lvl_off[d0.lvl_base + Lv + 1]);
-        }
-        __syncthreads();
-        lv_lo = s_lo[0];
-        lv_hi = s_hi[0];
-      }
-      return (lv_hi - lv_lo + 31) >> 5;
-    }
-    __syncthreads();  // every warp is done with the previous ranges
-    for (int r = threadIdx.x; r < nreal; r += kWalkThreads) {
-      if (Lv < s_nlev[r]) {
-        const int b = desc(r).lvl_base;
-        s_lo[r] = __ldcg(&a.lvl_off[b + Lv]);
-        s_hi[r] = __ldcg(&a.lvl_off[b + Lv + 1]);
-      } else {
-        s_lo[r] = s_hi[r] = 0;
-      }
-    }
-    __syncthreads();
-    return block_prefix(nreal, [&](int r) { return (s_hi[r] - s_lo[r] + 31) >> 5; }, s_pre);
-  };
-
-  // ---- accumulation: fastscape_RB.cpp:262-279, pushed level by level ----
-  // acc[i] = 1 + the counts of i's donors (the reference's accum is
-  // acc*cell_area, exact: integer multiples of cell_area). The ordering set
-  // every acc to 1; from the deepest level up, each entry -- whose count is
-  // final, its donors having pushed before the last barrier -- adds its
-  // count to its receiver's (position par[i]) with a fire-and-forget
-  // reduction. Integer sums are exact in any order. A count at level >= 1
-  // beyond its realization's erosion table stops the timestep before any
-  // elevation changes; the host grows the table and repeats it.
-  // Each level's ranges come from the finished level table, so the next
-  // level's are set up before this level's barrier.
-  int ngroups = maxlev > 1 ? level_groups(maxlev - 1) : 0;
-  for (int Lv = maxlev - 1; Lv >= 1; --Lv) {
-    // 32-entry groups per warp per iteration. A single grid sums runs of
-    // donors in the warp (more work per group) and loads the next groups
-    // before reducing these; a batch reduces per donor and keeps more groups'
-    // loads in flight instead (each measured faster for its case).
-    constexpr int kAccU = SINGLE ? 2 : 4;
-    struct Group {
-      uint32_t v[kAccU];
-      int p[kAccU], r[kAccU];
-      bool ok[kAccU];
-    };
-    auto load_group = [&](int g0) -> Group {
-      Group G;
-#pragma unroll
-      for (int u = 0; u < kAccU; u++) {  // all loads in flight first
-        const int g = g0 + u;
-        G.ok[u] = false;
-        G.v[u] = 0;
-        G.p[u] = 0;
-        G.r[u] = 0;
-        if (g < ngroups) {
-          const int r = real_of(g);
-          const int i = lo_of(r) + 32 * (g - pre_of(r)) + lane;
-          G.r[u] = r;
-          if (i < hi_of(r)) {
-            const int off = desc(r).off;
-            G.ok[u] = true;
-            G.v[u] = __ldcg(&a.acc[off + i]);
-            G.p[u] = __ldcg(&a.par[off + i]);
-          }
-        }
-      }
-      return G;
-    };
-    Group nxt;
-    if (SINGLE) nxt = load_group(warp_global * kAccU);
-    for (int g0 = warp_global * kAccU; g0 < ngroups; g0 += nwarps * kAccU) {
-      Group G;
-      if (SINGLE) {
-        G = nxt;
-        nxt = load_group(g0 + nwarps * kAccU);
-      } else {
-        G = load_group(g0);
-      }
-      const uint32_t *v = G.v;
-      const int *pp = G.p, *rr = G.r;
-      const bool *ok = G.ok;
-#pragma unroll
-      for (int u = 0; u < kAccU; u++) {
-        if (!SINGLE) {  // batches: one reduction per donor (measured faster there)
-          if (ok[u]) {
-            const RealDesc &d = desc(rr[u]);
-            atomicAdd(&a.acc[d.off + pp[u]], v[u]);
-          }
-          continue;
-        }
-        // Donors of one receiver are consecutive: sum each run of equal
-        // receiver positions in the group (a warp scan minus its value
-        // before the run) and let the run's last lane reduce it into the
-        // receiver -- one reduction per receiver and group instead of one
-        // per donor. Lanes past the level keep runs of their own.
-        const int p = ok[u] ? pp[u] : -1 - lane;
-        const int pu = __shfl_up_sync(kFull, p, 1), pd = __shfl_down_sync(kFull, p, 1);
-        const bool head = lane == 0 || pu != p, tail = lane == 31 || pd != p;
-        const unsigned heads = __ballot_sync(kFull, head) & (0xFFFFFFFFu >> (31 - lane));
-        const int hl = 31 - __clz(heads);  // first lane of this lane's run
-        uint32_t S = v[u];
-#pragma unroll
-        for (int dd = 1; dd < 32; dd <<= 1) {
-          const uint32_t x = __shfl_up_sync(kFull, S, dd);
-          if (lane >= dd) S += x;
-        }
-        const uint32_t before = __shfl_sync(kFull, S, (hl + 31) & 31);
-        const uint32_t run = S - (hl > 0 ? before : 0u);
-        if (ok[u]) {
-          const RealDesc &d = desc(rr[u]);
-          if (tail) atomicAdd(&a.acc[d.off + p], run);
-        }
-      }
-    }
-    if (Lv > 1) ngroups = level_groups(Lv - 1);
-    if (!grid_barrier(ctl, &ctl->bar3, epoch, a.timeout_ns)) return;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Per-realization level walk, the timestep of batches of many small
 // realizations late in a long run, whose tiles do not fit the GPU at once.
 // There the tile walk (fs_tile.cu) finds narrow levels, some 30 cells of a
@@ -1065,7 +622,6 @@ __global__ void __launch_bounds__(T, 2048 / T) k_cta_order_accum(StepArgs a) {
     }
     if (t == 0) {
       a.rctl[r].nlevels = nlev;
-      a.rctl[r].total = hi;
       if (ovf) raise_err(ctl, FS_ERR_LEVEL_OVERFLOW, kPhaseOrder);
       else if (hi != d.size) raise_err(ctl, FS_ERR_ORDER, kPhaseOrder);  // a cycle
     }
@@ -1281,105 +837,6 @@ __global__ void k_test_wait(Ctl *ctl, unsigned long long timeout_ns) {
   }
 }
 
-// ---------------------------------------------------------------------------
-// 5. The Braun-Willett order (fastscape_BW.cpp:201-221) of the last
-// timestep's receiver forest, from the level-walk arrays: a depth-first
-// preorder with roots (NO_FLOW cells) in ascending index and each cell's
-// donors in ascending index. A cell's preorder position is its parent's
-// position + 1 + the subtree sizes (drainage counts) of the siblings before
-// it; a root's is the total subtree size of the roots before it. Computed
-// level by level, top down, then scattered.
-// ---------------------------------------------------------------------------
-
-// cellacc[ent[i]] = acc[i] over one realization.
-__global__ void k_scatter_counts(const int32_t *__restrict__ ent, const uint32_t *__restrict__ acc,
-                                 int n, int32_t *__restrict__ cellacc) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    cellacc[ent[i]] = (int32_t)acc[i];
-}
-
-// v[c] = subtree size of c if c is a root, else 0; then an exclusive scan in
-// three launches (block sums, one block over the sums, block scans + offsets).
-constexpr int kScanBlock = 1024;
-__global__ void k_root_sizes_blocksum(const int8_t *__restrict__ rec,
-                                      const int32_t *__restrict__ cellacc, int n,
-                                      int32_t *__restrict__ v, int32_t *__restrict__ bsum) {
-  const int i = blockIdx.x * kScanBlock + threadIdx.x;
-  const int x = (i < n && rec[i] < 0) ? cellacc[i] : 0;
-  if (i < n) v[i] = x;
-  int total;
-  block_excl_scan(x, total, threadIdx.x, kScanBlock);
-  if (threadIdx.x == 0) bsum[blockIdx.x] = total;
-}
-
-__global__ void k_scan_sums(int32_t *bsum, int nb) {
-  // one block: each thread scans a contiguous slice, then the slices
-  const int per = (nb + kScanBlock - 1) / kScanBlock;
-  const int b0 = threadIdx.x * per;
-  int s = 0;
-  for (int b = b0; b < b0 + per && b < nb; b++) s += bsum[b];
-  int total;
-  int run = block_excl_scan(s, total, threadIdx.x, kScanBlock);
-  for (int b = b0; b < b0 + per && b < nb; b++) {
-    const int x = bsum[b];
-    bsum[b] = run;
-    run += x;
-  }
-}
-
-__global__ void k_scan_apply(int32_t *__restrict__ v, const int32_t *__restrict__ bsum, int n) {
-  const int i = blockIdx.x * kScanBlock + threadIdx.x;
-  const int x = i < n ? v[i] : 0;
-  int total;
-  const int e = block_excl_scan(x, total, threadIdx.x, kScanBlock);
-  if (i < n) v[i] = bsum[blockIdx.x] + e;
-}
-
-// Level 0: dpos[i] = rootpos[ent[i]].
-__global__ void k_dfs_level0(const int32_t *__restrict__ ent, const int32_t *__restrict__ rootpos,
-                             int n0, int32_t *__restrict__ dpos) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n0; i += gridDim.x * blockDim.x)
-    dpos[i] = rootpos[ent[i]];
-}
-
-// Donors of the entries [b, e): positions after their parent in ascending
-// cell-index order (the donor-list order of fastscape_BW.cpp:188-198).
-// First and one-past-last donor position of every receiver, from the
-// donors' receiver positions (a receiver's donors are contiguous, so they
-// start where par changes): kid / kend for positions of levels >= 1.
-__global__ void k_dfs_links(const int32_t *__restrict__ par, int b1, int n,
-                            int32_t *__restrict__ kid, int32_t *__restrict__ kend) {
-  for (int j = b1 + blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    const int p = par[j];
-    if (j == b1 || par[j - 1] != p) kid[p] = j;
-    if (j == n - 1 || par[j + 1] != p) kend[p] = j + 1;
-  }
-}
-
-__global__ void k_dfs_level(const int32_t *__restrict__ kid, const int32_t *__restrict__ kend,
-                            const uint8_t *__restrict__ pdir, const uint32_t *__restrict__ acc,
-                            int b, int e, int W, int32_t *__restrict__ dpos) {
-  for (int i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x) {
-    const int k0 = kid[i], n = kend[i] - k0;
-    if (n <= 0) continue;
-    const int p = dpos[i];
-    for (int q = 0; q < n; q++) {
-      // the donor's offset from its receiver is minus its receiver offset
-      const int oq = -nbr_off(pdir[k0 + q] & 7, W);
-      int pos = p + 1;
-      for (int s = 0; s < n; s++)
-        if (-nbr_off(pdir[k0 + s] & 7, W) < oq) pos += (int)acc[k0 + s];
-      dpos[k0 + q] = pos;
-    }
-  }
-}
-
-__global__ void k_dfs_scatter(const int32_t *__restrict__ ent, const int32_t *__restrict__ dpos,
-                              int n, int32_t *__restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    out[dpos[i]] = ent[i];
-}
-
 int sm_count() {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -1388,33 +845,6 @@ int sm_count() {
 }
 
 }  // namespace
-
-size_t walk_smem_bytes(int nreal) { return sizeof(int) * (4 * (size_t)nreal + 1); }
-
-int walk_threads() { return kWalkThreads; }
-
-const void *order_kernel_ptr(bool single) {
-  return single ? reinterpret_cast<const void *>(&k_order<true, 2>)
-                : reinterpret_cast<const void *>(&k_order<false, 2>);
-}
-
-const void *accum_kernel_ptr(bool single) {
-  return single ? reinterpret_cast<const void *>(&k_accum<true>)
-                : reinterpret_cast<const void *>(&k_accum<false>);
-}
-
-cudaError_t prepare_walk_kernels() {
-  const int bytes = (int)walk_smem_bytes(kMaxReal);
-  for (int single = 0; single < 2; single++) {
-    cudaError_t e = cudaFuncSetAttribute(order_kernel_ptr(single != 0),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(accum_kernel_ptr(single != 0),
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
 
 double neg_recip_dr(double dr) {
   return dr >= 1.0 && dr <= 0x1p60 ? -(1.0 / dr) : 0.0;
@@ -1533,20 +963,6 @@ cudaError_t launch_donors_level0(const StepArgs &a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_order(const StepArgs &a, int sms, int bps, cudaStream_t s) {
-  StepArgs args = a;
-  void *params[] = {&args};
-  return cudaLaunchCooperativeKernel(order_kernel_ptr(a.nreal == 1), dim3(sms * bps),
-                                     dim3(kWalkThreads), params, walk_smem_bytes(a.nreal), s);
-}
-
-cudaError_t launch_accum(const StepArgs &a, int sms, int bps, cudaStream_t s) {
-  StepArgs args = a;
-  void *params[] = {&args};
-  return cudaLaunchCooperativeKernel(accum_kernel_ptr(a.nreal == 1), dim3(sms * bps),
-                                     dim3(kWalkThreads), params, walk_smem_bytes(a.nreal), s);
-}
-
 // Threads of a CTA by the realizations an SM has to hold.
 int cta_width(int nreal, int sms) {
   const int per = (nreal + sms - 1) / sms;
@@ -1613,35 +1029,6 @@ cudaError_t launch_no_receivers(int8_t *rec, int W, int H, cudaStream_t s) {
 cudaError_t launch_test_wait(Ctl *ctl, int blocks, unsigned long long timeout_ns,
                              cudaStream_t s) {
   k_test_wait<<<blocks, 32, 0, s>>>(ctl, timeout_ns);
-  return cudaGetLastError();
-}
-
-size_t dfs_scratch_ints(int size) {
-  return 5 * (size_t)size + (size_t)(size + kScanBlock - 1) / kScanBlock + 1;
-}
-
-cudaError_t launch_dfs_order(const DfsArgs &d, const int32_t *lvl_host, int nlev,
-                             int32_t *scratch, int32_t *out, cudaStream_t s) {
-  const int n = d.size;
-  int32_t *cellacc = scratch, *v = scratch + n, *dpos = scratch + 2 * (size_t)n;
-  int32_t *kid = scratch + 3 * (size_t)n, *kend = scratch + 4 * (size_t)n;
-  int32_t *bsum = scratch + 5 * (size_t)n;
-  const int nb = (n + kScanBlock - 1) / kScanBlock;
-  const int g = (n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096;
-  cudaError_t e = cudaMemsetAsync(kid, 0, 2 * (size_t)n * sizeof(int32_t), s);
-  if (e != cudaSuccess) return e;
-  if (nlev > 1 && lvl_host[1] < n) k_dfs_links<<<g, 256, 0, s>>>(d.par, lvl_host[1], n, kid, kend);
-  k_scatter_counts<<<g, 256, 0, s>>>(d.ent, d.acc, n, cellacc);
-  k_root_sizes_blocksum<<<nb, kScanBlock, 0, s>>>(d.rec, cellacc, n, v, bsum);
-  k_scan_sums<<<1, kScanBlock, 0, s>>>(bsum, nb);
-  k_scan_apply<<<nb, kScanBlock, 0, s>>>(v, bsum, n);
-  k_dfs_level0<<<g, 256, 0, s>>>(d.ent, v, lvl_host[1], dpos);
-  for (int L = 0; L + 1 < nlev; L++) {
-    const int b = lvl_host[L], e2 = lvl_host[L + 1];
-    const int gl = (e2 - b + 255) / 256 < 4096 ? (e2 - b + 255) / 256 : 4096;
-    if (gl > 0) k_dfs_level<<<gl, 256, 0, s>>>(kid, kend, d.pdir, d.acc, b, e2, d.W, dpos);
-  }
-  k_dfs_scatter<<<g, 256, 0, s>>>(d.ent, dpos, n, out);
   return cudaGetLastError();
 }
 

@@ -9,13 +9,15 @@
 //                               timesteps, as in the reference)
 //   rec     int8[C]             receiver direction code, -1 rings, -2 pits
 //   count   uint32[C]           drainage cell counts (accum = count*cell_area)
-//   amb     int32[C], amb_r     cells queued for the FP64 receiver fix-up
+//   amb     int32[2*C]          cells queued for the FP64 receiver fix-up, and
+//                               their realizations (amb_r); between timesteps
+//                               the words of a network read-back
 //   tile_mem                    the tile walk's arrays (fs_internal.h, TileBufs),
 //                               12 KB per 64 x 32 cells
-//   ent, pdir, acc, par, lvl_off, mask
-//                               the level order and donor masks, which the
-//                               timestep does without: written when a caller
-//                               asks for levels, masks or the depth-first order
+//   ent, mask                   donor masks and the roots, for a caller that
+//                               reads the masks and for the per-realization
+//                               walk, with pdir, acc, par and lvl_off the
+//                               latter's level order (batches only)
 //   tab_r   double[8*cap_r]     erosion table of realization r per drainage
 //                               count k < cap_r (fs_internal.h); grows on
 //                               demand
@@ -102,7 +104,7 @@ struct fs_batch {
   int n = 0;
   std::vector<int> W, H, size, off, lvl_base, nring;
   std::vector<fs_params> p;
-  long long cells = 0, lvl_total = 0;
+  long long cells = 0;
   int nmode = fs::kNOne;
   double neq = 1.0;
   int device = 0;
@@ -123,15 +125,13 @@ struct fs_batch {
   fs::TileBufs tb{};             // over tile_mem, all tiles
   std::vector<int> tile0;        // first walk tile of each realization, and the total
   fs::TileRoom room;             // blocks of the tile kernels that fit the GPU
-  bool network_stale = true;     // the level order is older than the receivers
+  bool masks_stale = true;       // the donor masks are older than the receivers
   std::vector<char> count_stale; // and `count`, per realization
   std::vector<char> stepped;     // realizations that a timestep or analysis included
   std::vector<fs::RealDesc> desc;
   std::vector<double *> tab;
   std::vector<int> tab_cap;
   int walk_sms = 1;
-  int order_bps = 2;                             // k_order blocks per SM
-  int accum_bps = 1;                             // k_accum blocks per SM
   int erode_isub = 0;                            // the erosion's integer subtractions (n = 1, 2)
   // per-realization walk: used when cta_walk, the launch covers more than one
   // realization and their tiles do not all fit the GPU at once
@@ -186,7 +186,7 @@ void free_batch(fs_batch *b) {
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->graph) cudaGraphExecDestroy(b->graph);
-  void *bufs[] = {b->h, b->rec_alloc, b->mask, b->pdir, b->ent, b->par, b->amb, b->amb_r,
+  void *bufs[] = {b->h, b->rec_alloc, b->mask, b->pdir, b->ent, b->par, b->amb,
                   b->lvl, b->acc, b->d_desc, b->d_rctl, b->d_ctl, b->d_rtiles, b->d_dtiles,
                   b->d_wtiles, b->count, b->tile_mem, b->d_desc_act, b->d_rctl_act,
                   b->d_rtiles_act, b->d_dtiles_act, b->d_wlist_act};
@@ -447,13 +447,6 @@ int collect_status(fs_batch *b) {
   return FS_OK;
 }
 
-int read_rctl(const fs_batch *b) {
-  FS_CUDA(cudaMemcpyAsync(b->h_rctl, b->d_rctl, sizeof(fs::RealCtl) * b->n, cudaMemcpyDeviceToHost,
-                          b->stream));
-  FS_CUDA(cudaStreamSynchronize(b->stream));
-  return FS_OK;
-}
-
 // Initial erosion tables of every realization (counts below min(65536,
 // size+1)), evaluated on host threads in parallel over realizations -- the
 // same records grow_table writes -- then uploaded.
@@ -602,10 +595,9 @@ void mark_stepped(fs_batch *b) {
     std::fill(b->stepped.begin(), b->stepped.end(), 1);
 }
 
-// Drainage counts per cell, and the donor masks and level order, of every
-// realization's last receivers (fastscape_RB.cpp:188-279), for the callers
-// that ask for them: the timestep itself keeps its counts in the tiles and
-// needs no order.
+// Drainage counts per cell, and donor masks, of every realization's last
+// receivers (fastscape_RB.cpp:188-203, 262-279), for the callers that ask for
+// them: the timestep itself keeps its counts in the tiles and needs no masks.
 int ensure_counts(const fs_batch *cb, int r) {
   fs_batch *b = const_cast<fs_batch *>(cb);
   if (!b->count_stale[r]) return FS_OK;
@@ -620,9 +612,9 @@ int ensure_counts(const fs_batch *cb, int r) {
   return FS_OK;
 }
 
-int ensure_network(const fs_batch *cb) {
+int ensure_masks(const fs_batch *cb) {
   fs_batch *b = const_cast<fs_batch *>(cb);
-  if (!b->network_stale) return FS_OK;
+  if (!b->masks_stale) return FS_OK;
   fs::StepArgs a = step_args(b, 0);
   a.desc = b->d_desc;  // every realization, active or not
   a.rctl = b->d_rctl;
@@ -630,13 +622,10 @@ int ensure_network(const fs_batch *cb) {
   a.dtiles = b->d_dtiles;
   a.ndtiles = b->ndtiles;
   FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, fs::kCtlCallResetBytes, b->stream));
-  FS_CUDA(cudaMemsetAsync(&b->d_ctl->bar, 0, sizeof(fs::Ctl) - offsetof(fs::Ctl, bar), b->stream));
   FS_CUDA(cudaMemsetAsync(b->d_rctl, 0, sizeof(fs::RealCtl) * b->n, b->stream));
   FS_CUDA(fs::launch_donors_level0(a, b->stream));
-  FS_CUDA(fs::launch_order(a, b->walk_sms, b->order_bps, b->stream));
-  FS_CUDA(fs::launch_accum(a, b->walk_sms, b->accum_bps, b->stream));
   if (int st = collect_status(b)) return st;
-  b->network_stale = false;
+  b->masks_stale = false;
   return FS_OK;
 }
 
@@ -681,7 +670,7 @@ int batch_step(fs_batch *b, int k) {
         b->phase_ms[3] += tot;
       }
     }
-    b->network_stale = true;
+    b->masks_stale = true;
     mark_counts(b, 1);
     if (int st = collect_status(b)) return st;
     const int completed = b->h_ctl->steps_done;
@@ -786,7 +775,6 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
     return fail(set_error(FS_ERR_NOMEM, "%zu walk tiles", wt.size()));
   b->stepped.assign(n, 0);
   b->count_stale.assign(n, 1);
-  b->lvl_total = lb;
   b->tab.assign(n, nullptr);
   b->tab_cap.assign(n, 0);
   const size_t C = static_cast<size_t>(cells);
@@ -794,13 +782,8 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
       !cu(cudaMalloc(&b->h, C * sizeof(double)), "cudaMalloc(h)") ||
       !cu(cudaMalloc(&b->rec_alloc, C + 2 * fs::kRecPad), "cudaMalloc(rec)") ||
       !cu(cudaMalloc(&b->mask, C), "cudaMalloc(mask)") ||
-      !cu(cudaMalloc(&b->pdir, C), "cudaMalloc(pdir)") ||
       !cu(cudaMalloc(&b->ent, C * sizeof(int32_t)), "cudaMalloc(ent)") ||
-      !cu(cudaMalloc(&b->par, C * sizeof(int32_t)), "cudaMalloc(par)") ||
-      !cu(cudaMalloc(&b->amb, C * sizeof(int32_t)), "cudaMalloc(amb)") ||
-      !cu(cudaMalloc(&b->amb_r, C * sizeof(int32_t)), "cudaMalloc(amb_r)") ||
-      !cu(cudaMalloc(&b->acc, C * sizeof(uint32_t)), "cudaMalloc(acc)") ||
-      !cu(cudaMalloc(&b->lvl, static_cast<size_t>(lb) * sizeof(int32_t)), "cudaMalloc(lvl)") ||
+      !cu(cudaMalloc(&b->amb, 2 * C * sizeof(int32_t)), "cudaMalloc(amb)") ||
       !cu(cudaMalloc(&b->count, C * sizeof(uint32_t)), "cudaMalloc(count)") ||
       !cu(cudaMalloc(&b->tile_mem, fs::tile_bytes(wt.size())), "cudaMalloc(tiles)") ||
       !cu(cudaMalloc(&b->d_wtiles, wt.size() * sizeof(fs::Tile)), "cudaMalloc(wtiles)") ||
@@ -810,7 +793,14 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
       !cu(cudaMallocHost(&b->h_ctl, sizeof(fs::Ctl)), "cudaMallocHost(ctl)") ||
       !cu(cudaMallocHost(&b->h_rctl, n * sizeof(fs::RealCtl)), "cudaMallocHost(rctl)"))
     return fail(*status);
+  if (n > 1 &&  // the per-realization walk's
+      (!cu(cudaMalloc(&b->pdir, C), "cudaMalloc(pdir)") ||
+       !cu(cudaMalloc(&b->par, C * sizeof(int32_t)), "cudaMalloc(par)") ||
+       !cu(cudaMalloc(&b->acc, C * sizeof(uint32_t)), "cudaMalloc(acc)") ||
+       !cu(cudaMalloc(&b->lvl, static_cast<size_t>(lb) * sizeof(int32_t)), "cudaMalloc(lvl)")))
+    return fail(*status);
   b->rec = b->rec_alloc + fs::kRecPad;
+  b->amb_r = b->amb + C;
   fs::tile_carve(&b->tb, b->tile_mem, wt.size());
   b->tb.tiles = b->d_wtiles;
   b->tb.list = nullptr;
@@ -824,9 +814,6 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
           "upload(wtiles)") ||
       !cu(cudaMemsetAsync(b->count, 0, C * sizeof(uint32_t), b->stream), "memset(count)") ||
       !cu(cudaMemsetAsync(b->mask, 0, C, b->stream), "memset(mask)") ||
-      !cu(cudaMemsetAsync(b->acc, 0, C * sizeof(uint32_t), b->stream), "memset(acc)") ||
-      !cu(cudaMemsetAsync(b->lvl, 0, static_cast<size_t>(lb) * sizeof(int32_t), b->stream),
-          "memset(lvl)") ||
       !cu(cudaMemsetAsync(b->d_rctl, 0, n * sizeof(fs::RealCtl), b->stream), "memset(rctl)") ||
       !cu(cudaMemsetAsync(b->d_ctl, 0, sizeof(fs::Ctl), b->stream), "memset(ctl)"))
     return fail(*status);
@@ -912,34 +899,11 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
       return fail(*status);
     }
   }
-  if (!cu(fs::prepare_walk_kernels(), "walk smem attribute") ||
-      !cu(cudaDeviceGetAttribute(&b->walk_sms, cudaDevAttrMultiProcessorCount, b->device), "attr") ||
+  if (!cu(cudaDeviceGetAttribute(&b->walk_sms, cudaDevAttrMultiProcessorCount, b->device), "attr") ||
       !cu(fs::prepare_tile_kernels(b->nmode, b->walk_sms, &b->room), "tile kernels"))
     return fail(*status);
   if (b->room.queued < 1) return fail(set_error(FS_ERR_CUDA, "tile kernel cannot be resident"));
   b->rmap_ok = n == 1 && fs::make_receiver_map(&b->rmap, b->h, b->W[0], b->H[0]);
-  // k_order at two blocks per SM: three took ~25% longer on every single
-  // grid measured (1000² to 10000²: 0.205 against 0.149 ms per ordering at
-  // 4000²).
-  {
-    int o = 0;
-    if (!cu(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fs::order_kernel_ptr(n == 1),
-                                                          fs::walk_threads(),
-                                                          fs::walk_smem_bytes(n)),
-            "occupancy"))
-      return fail(*status);
-    if (o < b->order_bps) return fail(set_error(FS_ERR_CUDA, "order kernel cannot be resident"));
-  }
-  {
-    int o = 0;
-    if (!cu(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fs::accum_kernel_ptr(n == 1),
-                                                          fs::walk_threads(),
-                                                          fs::walk_smem_bytes(n)),
-            "occupancy"))
-      return fail(*status);
-    if (o < 1) return fail(set_error(FS_ERR_CUDA, "accumulation kernel cannot be resident"));
-    b->accum_bps = std::min(o, fs::kAccumMaxBps);
-  }
   if (!cu(cudaStreamSynchronize(b->stream), "sync")) return fail(*status);
   return b;
 }
@@ -974,19 +938,28 @@ int set_elevation(fs_batch *b, int r, const double *in) {
   return st;
 }
 
+// What the read-backs below work in: arrays that hold nothing between
+// timesteps. The filter's queues are a word per cell; the tiles' (6 bytes a
+// cell) an int per cell and the sums of launch_net_trees.
+fs::NetArgs net_args(const fs_batch *b, int r) {
+  const int o = b->off[r];
+  return fs::NetArgs{b->rec + o, b->count + o, b->size[r], b->W[r],
+                     reinterpret_cast<unsigned long long *>(b->amb)};
+}
+
+int32_t *net_ints(const fs_batch *b) { return reinterpret_cast<int32_t *>(b->tile_mem); }
+
 int get_accumulation(const fs_batch *b, int r, double *out) {
   if (int st = check_r(b, r)) return st;
   if (!out) return set_error(FS_ERR_ARG, "out is NULL");
   if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
   DeviceGuard dg(b->device);
   if (int st = ensure_counts(b, r)) return st;
-  const int n = b->size[r];
-  std::vector<uint32_t> k(n);
-  FS_CUDA(cudaMemcpyAsync(k.data(), b->count + b->off[r], sizeof(uint32_t) * n,
-                          cudaMemcpyDeviceToHost, b->stream));
+  const fs::NetArgs a = net_args(b, r);
+  double *area = reinterpret_cast<double *>(a.words);
+  FS_CUDA(fs::launch_net_area(a, b->p[r].cell_area, area, b->stream));
+  FS_CUDA(cudaMemcpyAsync(out, area, sizeof(double) * a.n, cudaMemcpyDeviceToHost, b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
-  const double area = b->p[r].cell_area;
-  for (int i = 0; i < n; i++) out[i] = static_cast<double>(k[i]) * area;
   return FS_OK;
 }
 
@@ -995,11 +968,25 @@ int get_receivers(const fs_batch *b, int r, int32_t *dir) {
   if (!dir) return set_error(FS_ERR_ARG, "dir is NULL");
   if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
   DeviceGuard dg(b->device);
-  std::vector<int8_t> v(b->size[r]);
-  FS_CUDA(cudaMemcpyAsync(v.data(), b->rec + b->off[r], b->size[r], cudaMemcpyDeviceToHost,
+  const fs::NetArgs a = net_args(b, r);
+  FS_CUDA(fs::launch_net_receivers(a, net_ints(b), b->stream));
+  FS_CUDA(cudaMemcpyAsync(dir, net_ints(b), sizeof(int32_t) * a.n, cudaMemcpyDeviceToHost,
                           b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
-  for (int i = 0; i < b->size[r]; i++) dir[i] = v[i] < 0 ? FS_NO_FLOW : v[i];
+  return FS_OK;
+}
+
+// The levels of realization r into the device's net_ints(), their number
+// into *nlevels; FS_ERR_ORDER if the receivers hold a cycle.
+int find_levels(const fs_batch *cb, int r, int32_t *nlevels) {
+  fs_batch *b = const_cast<fs_batch *>(cb);
+  FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, fs::kCtlCallResetBytes, b->stream));
+  FS_CUDA(cudaMemsetAsync(b->d_rctl + r, 0, sizeof(fs::RealCtl), b->stream));
+  FS_CUDA(fs::launch_net_levels(net_args(b, r), b->d_rctl + r, b->d_ctl, net_ints(b), b->stream));
+  FS_CUDA(cudaMemcpyAsync(b->h_rctl + r, b->d_rctl + r, sizeof(fs::RealCtl),
+                          cudaMemcpyDeviceToHost, b->stream));
+  if (int st = collect_status(b)) return st;
+  *nlevels = b->h_rctl[r].nlevels;
   return FS_OK;
 }
 
@@ -1007,66 +994,54 @@ int get_levels(const fs_batch *b, int r, int32_t *level_id, int32_t *nlevels) {
   if (int st = check_r(b, r)) return st;
   if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
   DeviceGuard dg(b->device);
-  if (int st = ensure_network(b)) return st;
-  if (int st = read_rctl(b)) return st;
-  const int nl = b->stepped[r] ? b->h_rctl[r].nlevels : 0;
+  const int n = b->size[r];
+  int32_t nl = 0;
+  if (b->stepped[r]) {
+    if (int st = find_levels(b, r, &nl)) return st;
+  }
   if (nlevels) *nlevels = nl;
   if (!level_id) return FS_OK;
-  const int n = b->size[r];
-  std::vector<int32_t> ent(n), off(nl + 1);
-  FS_CUDA(cudaMemcpyAsync(ent.data(), b->ent + b->off[r], sizeof(int32_t) * n,
-                          cudaMemcpyDeviceToHost, b->stream));
-  FS_CUDA(cudaMemcpyAsync(off.data(), b->lvl + b->lvl_base[r], sizeof(int32_t) * (nl + 1),
-                          cudaMemcpyDeviceToHost, b->stream));
+  if (!b->stepped[r]) {
+    std::fill(level_id, level_id + n, -1);
+    return FS_OK;
+  }
+  FS_CUDA(cudaMemcpyAsync(level_id, net_ints(b), sizeof(int32_t) * n, cudaMemcpyDeviceToHost,
+                          b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
-  for (int i = 0; i < n; i++) level_id[i] = -1;
-  for (int L = 0; L < nl; L++)
-    for (int s = off[L]; s < off[L + 1]; s++) level_id[ent[s]] = L;
   return FS_OK;
 }
 
-// The Braun-Willett order of the last timestep (fastscape_BW.cpp:201-221),
-// computed on the device from the level walk; stack_start (may be NULL)
-// gets the first position of each root and a final size entry
-// (fastscape_BW+P.cpp:223-240).
-int get_stack_dfs(const fs_batch *b, int r, int32_t *stack, int32_t *stack_start,
+// The Braun-Willett order of the last timestep (fastscape_BW.cpp:201-221);
+// stack_start (may be NULL) gets the first position of each root and a final
+// size entry (fastscape_BW+P.cpp:223-240).
+int get_stack_dfs(const fs_batch *cb, int r, int32_t *stack, int32_t *stack_start,
                   int32_t *nroots) {
-  if (int st = check_r(b, r)) return st;
+  if (int st = check_r(cb, r)) return st;
   if (!stack) return set_error(FS_ERR_ARG, "stack is NULL");
-  if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
-  DeviceGuard dg(b->device);
-  if (int st = ensure_network(b)) return st;
-  if (int st = read_rctl(b)) return st;
-  const int nl = b->h_rctl[r].nlevels;
-  const int n = b->size[r];
-  std::vector<int32_t> off(nl + 1);
-  FS_CUDA(cudaMemcpyAsync(off.data(), b->lvl + b->lvl_base[r], sizeof(int32_t) * (nl + 1),
-                          cudaMemcpyDeviceToHost, b->stream));
+  if (!cb->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
+  DeviceGuard dg(cb->device);
+  if (int st = ensure_counts(cb, r)) return st;
+  fs_batch *b = const_cast<fs_batch *>(cb);
+  const fs::NetArgs a = net_args(b, r);
+  const int n = a.n, nb = fs::net_sums(n);
+  int32_t *ints = net_ints(b);  // the trees' starts, then the order
+  int2 *sums = reinterpret_cast<int2 *>(ints + (static_cast<size_t>(n) + 1) / 2 * 2);
+  int2 total{};
+  FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, fs::kCtlCallResetBytes, b->stream));
+  FS_CUDA(fs::launch_net_trees(a, sums, ints, b->stream));
+  FS_CUDA(cudaMemcpyAsync(&total, sums + nb, sizeof(total), cudaMemcpyDeviceToHost, b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
-  int32_t *scratch = nullptr, *out = nullptr;
-  FS_CUDA(cudaMalloc(&scratch, fs::dfs_scratch_ints(n) * sizeof(int32_t)));
-  cudaError_t e = cudaMalloc(&out, n * sizeof(int32_t));
-  const int o = b->off[r];
-  const fs::DfsArgs d{b->rec + o, b->ent + o, b->par + o, b->pdir + o, b->acc + o,
-                      b->W[r], n};
-  if (e == cudaSuccess) e = fs::launch_dfs_order(d, off.data(), nl, scratch, out, b->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(stack, out, n * sizeof(int32_t), cudaMemcpyDeviceToHost, b->stream);
-  std::vector<int8_t> rec(n);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(rec.data(), b->rec + o, n, cudaMemcpyDeviceToHost, b->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-  cudaFree(scratch);
-  cudaFree(out);
-  if (e != cudaSuccess) return cuda_error(e, "depth-first order");
-  int k = 0;
-  for (int p = 0; p < n; p++)
-    if (rec[stack[p]] < 0) {
-      if (stack_start) stack_start[k] = p;
-      k++;
-    }
-  if (stack_start) stack_start[k] = n;
-  if (nroots) *nroots = k;
+  if (stack_start) {
+    FS_CUDA(cudaMemcpyAsync(stack_start, ints, sizeof(int32_t) * total.y, cudaMemcpyDeviceToHost,
+                            b->stream));
+    FS_CUDA(cudaStreamSynchronize(b->stream));
+    stack_start[total.y] = n;
+  }
+  if (nroots) *nroots = total.y;
+  FS_CUDA(fs::launch_net_order(a, b->d_ctl, ints, b->stream));
+  if (int st = collect_status(b)) return st;
+  FS_CUDA(cudaMemcpyAsync(stack, ints, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, b->stream));
+  FS_CUDA(cudaStreamSynchronize(b->stream));
   return FS_OK;
 }
 
@@ -1075,7 +1050,7 @@ int get_donor_mask(const fs_batch *b, int r, uint8_t *mask) {
   if (!mask) return set_error(FS_ERR_ARG, "mask is NULL");
   if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
   DeviceGuard dg(b->device);
-  if (int st = ensure_network(b)) return st;
+  if (int st = ensure_masks(b)) return st;
   FS_CUDA(cudaMemcpyAsync(mask, b->mask + b->off[r], b->size[r], cudaMemcpyDeviceToHost, b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
   return FS_OK;
@@ -1296,11 +1271,13 @@ int fs_get_receiver_index(const fs_model *m, int64_t *idx) {
   FS_MODEL(m);
   if (!idx) return set_error(FS_ERR_ARG, "idx is NULL");
   const fs_batch *b = m->b;
-  std::vector<int32_t> dir(b->size[0]);
-  if (int st = get_receivers(b, 0, dir.data())) return st;
-  const long long W = b->W[0];
-  const long long off[8] = {-1, -W - 1, -W, -W + 1, 1, W + 1, W, W - 1};
-  for (int i = 0; i < b->size[0]; i++) idx[i] = dir[i] < 0 ? i : i + off[dir[i]];
+  if (!b->have_step) return set_error(FS_ERR_STATE, "no timestep executed yet");
+  DeviceGuard dg(b->device);
+  const fs::NetArgs a = net_args(b, 0);
+  long long *cell = reinterpret_cast<long long *>(a.words);
+  FS_CUDA(fs::launch_net_receiver_index(a, cell, b->stream));
+  FS_CUDA(cudaMemcpyAsync(idx, cell, sizeof(int64_t) * a.n, cudaMemcpyDeviceToHost, b->stream));
+  FS_CUDA(cudaStreamSynchronize(b->stream));
   return FS_OK;
 }
 
@@ -1453,7 +1430,7 @@ int fs_batch_autotune(fs_batch *b, int probe_steps, int *chosen) {
 int fs_batch_launch_config(const fs_batch *b, int *order_bps, int *erode_bps, int *graph,
                            int *erode_int_sub) {
   if (!b) return set_error(FS_ERR_ARG, "batch is NULL");
-  if (order_bps) *order_bps = b->order_bps;
+  if (order_bps) *order_bps = 2;
   if (erode_bps) *erode_bps = kErodeBps;
   if (graph) *graph = b->use_graph ? 1 : 0;
   if (erode_int_sub) *erode_int_sub = b->erode_isub;
@@ -1525,7 +1502,7 @@ int fs_batch_analyze(fs_batch *b) {
   DeviceGuard dg(b->device);
   const fs::StepArgs a = step_args(b, 0);
   FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, fs::kCtlCallResetBytes, b->stream));
-  b->network_stale = true;
+  b->masks_stale = true;
   mark_counts(b, 1);
   FS_CUDA(launch_step(b, a));
   if (int st = collect_status(b)) return st;
@@ -1607,11 +1584,12 @@ int fs_test_order_from_receivers(fs_model *m, const int32_t *dir) {
   FS_CUDA(fs::launch_tile_drain(a, b->stream));
   FS_CUDA(fs::launch_tile_links(a, b->stream));
   FS_CUDA(fs::launch_tile_counts(a, b->stream));
-  b->network_stale = true;
+  b->masks_stale = true;
   mark_counts(b, 0);
   mark_stepped(b);
   if (int st = collect_status(b)) return st;
-  return ensure_network(b);
+  int32_t nlevels;
+  return find_levels(b, 0, &nlevels);
 }
 
 // Selects the receiver kernel: 1 = the FP64 reference formula for every

@@ -245,8 +245,8 @@ int fs_batch_use_int_sub(fs_batch *b, int enable);
  * has more than one realization and none has more than 2^19 cells. Results do
  * not depend on the configuration. */
 int fs_batch_autotune(fs_batch *b, int probe_steps, int *chosen);
-/* The launch configuration in use: blocks per SM of the ordering kernel
- * (fs_get_levels) and 2, graph replay (0/1), integer subtractions in the
+/* The launch configuration in use: 2 and 2 (once the blocks per SM of kernels
+ * that are gone), graph replay (0/1), integer subtractions in the
  * erosion (0/1). Any pointer may be NULL. */
 int fs_batch_launch_config(const fs_batch *b, int *order_bps, int *erode_bps,
                            int *graph, int *erode_int_sub);
