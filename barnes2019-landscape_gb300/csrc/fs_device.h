@@ -39,9 +39,10 @@ __device__ __forceinline__ void cp_async8(void *dst, const void *src) {
                : "memory");
 }
 
-// Barrier of n threads of the block (a multiple of 32), beside __syncthreads.
-__device__ __forceinline__ void group_sync(int n) {
-  asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
+// Barrier number id (1 to 15) of n threads of the block (a multiple of 32),
+// beside __syncthreads.
+__device__ __forceinline__ void group_sync(int id, int n) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
 __device__ __forceinline__ void cp_async_wait() {

@@ -224,8 +224,9 @@ cudaError_t launch_donors_level0(const StepArgs &a, cudaStream_t s);
 // The tile walk (fs_tile.cu): drainage inside the tiles, drainage between
 // them, and the counts alone or the erosion. `resident` and `queued` are the
 // blocks that k_tile_resident and k_tile_queue can keep on the GPU at once.
+constexpr int kResidentWidths = 3;  // of k_tile_resident's blocks, narrowest first
 struct TileRoom {
-  int resident = 0, queued = 0;
+  int resident[kResidentWidths] = {}, queued = 0;
 };
 cudaError_t launch_tile_drain(const StepArgs &a, cudaStream_t s);
 cudaError_t launch_tile_links(const StepArgs &a, cudaStream_t s);

@@ -318,7 +318,7 @@ cudaError_t reset_ctl(fs_batch *b) {
 // whose tiles the GPU cannot hold at once (resident tiles are faster: 8
 // realizations of eroded 512^2 0.35 against 1.6 ms).
 bool use_cta(const fs_batch *b, const fs::StepArgs &a) {
-  return b->cta_walk && a.nreal > 1 && a.do_erode && a.tb.n > b->room.resident;
+  return b->cta_walk && a.nreal > 1 && a.do_erode && a.tb.n > b->room.resident[0];
 }
 
 // The launches of one timestep (no synchronization).

@@ -41,8 +41,14 @@ namespace {
 
 constexpr int kDrainThreads = 256;
 constexpr int kWalkThreads = 128;  // a warp that finds the levels, 3 that erode
-constexpr int kWorkers = kWalkThreads - 32;
-constexpr int kLead = 6;           // levels found ahead of the erosion, at most
+// Of k_tile_resident's blocks: 6, 4 and 2 share an SM (80 registers a thread).
+constexpr int kResidentThreads[kResidentWidths] = {128, 192, 384};
+constexpr int kCore = 96;          // threads that erode every level
+// Levels found ahead of the erosion, at most. What a neighbour makes ready is
+// eroded behind them: 501^2 with n = 2 takes 1130 us at 6, 1070 at 4, 1036 at
+// 3 and 1041 at 2, where eroded 512^2 begins to wait for the finder (617 us
+// against 607).
+constexpr int kLead = 3;
 constexpr int kRing = 8;           // level ends and rows kept
 constexpr int kStageFrom = 256;    // unfinished cells worth staging a tile for
 constexpr int kPullMost = 256;     // unfinished cells k_tile_pull takes from a tile, at most
@@ -423,7 +429,11 @@ __global__ void __launch_bounds__(256) k_tile_links(StepArgs a) {
 // that drain that way, so the donors of a set of cells are eight shifts and
 // masks; it writes their cell numbers to a list, rows in order. It runs up to
 // kLead levels ahead of the other warps, which erode the cells of a level and
-// meet at a barrier of their own. What takes time is the chain of one cell's
+// meet at a barrier of their own. On young ground one level holds half of a
+// tile: where the SMs have room for wider blocks, more warps sleep at another
+// barrier and help with the levels wider than two rounds of the first three
+// (100^2: 70 -> 57 us a timestep, 1000^2: 96 -> 87), which deep ground's narrow
+// levels do not wait for. What takes time is the chain of one cell's
 // arithmetic after its receiver's elevation is known (64 clocks for an FP64
 // operation, four to eight of them, and the quotient's integer steps), once a
 // level: everything else of a cell -- its elevation, count, table record, an
@@ -447,6 +457,7 @@ struct TileSmem {
   int ready;                            // levels found (| kFinished: all)
   int done;                             // levels eroded
   int task, flag;
+  int wide;                             // the level that all workers erode, or -1
 };
 
 __device__ __forceinline__ void st_volatile_i32(int *p, int v) {
@@ -699,9 +710,10 @@ __device__ __forceinline__ uint64_t cell_erode(const Cell &e, const Tolerance &t
 
 // The other warps. staged: the tile's elevations, counts and codes are in
 // shared memory (kResident: always).
-template <int NMODE, int VAR, int MODE>
+template <int NMODE, int VAR, int MODE, int WORKERS>
 __device__ __forceinline__ void erode_levels(const StepArgs &a, int t, const Tile &tl,
                                              const RealDesc &d, TileSmem &s, bool staged) {
+  constexpr bool kHelpers = WORKERS > kCore;
   const int wt = (int)threadIdx.x - 32;
   const int W = d.W;
   const uint64_t udt = (uint64_t)__double_as_longlong(d.u_dt);
@@ -740,9 +752,31 @@ __device__ __forceinline__ void erode_levels(const StepArgs &a, int t, const Til
     return e;
   };
   auto turn = [&](int L) -> int {  // place among the level's workers
-    const int k = (wt >> 5) - L % (kWorkers / 32);
-    return 32 * (k < 0 ? k + kWorkers / 32 : k) + (wt & 31);
+    const int k = (wt >> 5) - L % (kCore / 32);
+    return 32 * (k < 0 ? k + kCore / 32 : k) + (wt & 31);
   };
+  auto erode = [&](const Cell &e) {
+    const uint64_t hn = e.rc >= 0 ? s.h[e.rc] : e.hx;
+    const uint64_t h = cell_erode<NMODE, VAR>(e, tol, a.neq, a.ctl, hn);
+    s.h[e.c] = h;
+    if (e.out) gh[grid_cell(e.c)] = h;
+  };
+  auto erode_from = [&](int i, int hi, int step) {
+    for (; i < hi; i += step) {
+      Cell e = load(i, hi);
+      e.h0 = uplift_bits(e.h0, udt);
+      erode(e);
+    }
+  };
+  if (kHelpers && wt >= kCore) {  // wide levels only; asleep at the barrier between them
+    for (;;) {
+      group_sync(2, WORKERS);
+      const int L = s.wide;
+      if (L < 0) return;
+      erode_from(s.end[(L - 1) % kRing] + wt, s.end[L % kRing], WORKERS);
+      group_sync(2, WORKERS);
+    }
+  }
   // nx: this thread's first cell of the level, loaded during the level before
   // (first == L). The warps take turns: level L's first 32 cells, on deep
   // ground often all of them, are warp L % 3's, which has loaded and uplifted
@@ -753,7 +787,13 @@ __device__ __forceinline__ void erode_levels(const StepArgs &a, int t, const Til
     int ready;
     for (unsigned n = 0; (ready = ld_volatile_i32(&s.ready)) <= L; ++n)
       if (n > 2) __nanosleep(50);
-    if ((ready &= ~kFinished) <= L) return;
+    if ((ready &= ~kFinished) <= L) {
+      if (kHelpers) {
+        if (wt == 0) s.wide = -1;
+        group_sync(2, WORKERS);
+      }
+      return;
+    }
     __threadfence_block();
     const int lo = L ? s.end[(L - 1) % kRing] : 0, hi = s.end[L % kRing];
     const int at = lo + turn(L);
@@ -764,31 +804,30 @@ __device__ __forceinline__ void erode_levels(const StepArgs &a, int t, const Til
     }
     const bool more = ready > L + 1;
     if (more) nx = load(hi + turn(L + 1), s.end[(L + 1) % kRing]);
+    const bool wide = kHelpers && L && hi - lo > 2 * kCore;
+    if (wide) {
+      if (wt == 0) s.wide = L;
+      group_sync(2, WORKERS);
+    }
     if (MODE != kQueued && L == 0) {
       // level 0, of which the pits rise with the land (fastscape_RB.cpp:291-295)
-      for (int i = wt; i < hi; i += kWorkers) {
+      for (int i = wt; i < hi; i += kCore) {
         const int c = s.list[i];
         const uint64_t h = fadd_bits(s.h[c], udt);
         s.h[c] = h;
         if (MODE == kResident && (s.entry[c >> 6] >> (c & 63) & 1ull)) gh[grid_cell(c)] = h;
       }
-    } else {
-      for (int i = at; i < hi; i += kWorkers) {
-        if (i > at) {  // a wide level's further cells
-          e = load(i, hi);
-          e.h0 = uplift_bits(e.h0, udt);
-        }
-        const uint64_t hn = e.rc >= 0 ? s.h[e.rc] : e.hx;
-        const uint64_t h = cell_erode<NMODE, VAR>(e, tol, a.neq, a.ctl, hn);
-        s.h[e.c] = h;
-        if (e.out) gh[grid_cell(e.c)] = h;
-      }
+    } else if (e.c >= 0) {
+      erode(e);
+      const int step = wide ? WORKERS : kCore;
+      erode_from(at + step, hi, step);
     }
     if (more) {
       first = L + 1;
       if (nx.c >= 0) nx.h0 = uplift_bits(nx.h0, udt);
     }
-    group_sync(kWorkers);
+    if (wide) group_sync(2, WORKERS);
+    else group_sync(1, kCore);
     if (wt == 0) {
       __threadfence_block();
       st_volatile_i32(&s.done, L + 1);
@@ -889,8 +928,8 @@ __device__ __forceinline__ unsigned long long root_row(const Tile &tl, int W, in
   return roots;
 }
 
-template <int NMODE, int VAR>
-__global__ void __launch_bounds__(kWalkThreads, 6) k_tile_resident(StepArgs a) {
+template <int NMODE, int VAR, int T>
+__global__ void __launch_bounds__(T, 768 / T) k_tile_resident(StepArgs a) {
   if (stopped(a.ctl)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TileSmem &s = *reinterpret_cast<TileSmem *>(smem_raw);
@@ -898,7 +937,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_tile_resident(StepArgs a) {
   const Tile tl = a.tb.tiles[t];
   const RealDesc &d = a.tb.desc[tl.r];
   const int lane = threadIdx.x & 31;
-  tile_stage<kWalkThreads>(a, tl, d, s.h);
+  tile_stage<T>(a, tl, d, s.h);
   if (threadIdx.x == 0) s.ready = s.done = 0;
   tile_counts(a, t, s.acc, s.code, s.entry);
   if (threadIdx.x < 32) {
@@ -914,10 +953,10 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_tile_resident(StepArgs a) {
     if (lane == 0) st_volatile_i32(&s.ready, 1);
     find_levels<kResident>(a, t, tl, d.W, d.H, s, f, front_next(f, final, lane), final, pos, lane);
   } else {
-    erode_levels<NMODE, VAR, kResident>(a, t, tl, d, s, true);
+    erode_levels<NMODE, VAR, kResident, T - 32>(a, t, tl, d, s, true);
   }
   __syncthreads();
-  tile_store<kWalkThreads>(a, tl, d, s.h);
+  tile_store<T>(a, tl, d, s.h);
   if (threadIdx.x == 0 && atomicAdd(&a.ctl->left, 1) == (int)gridDim.x - 1)
     atomicAdd(&a.ctl->steps_done, 1);
 }
@@ -1285,7 +1324,7 @@ __global__ void __launch_bounds__(kWalkThreads, 7) k_tile_queue(StepArgs a) {
     int n = 0;
     if (flag) {
       if (wid == 0) n = find_levels<kQueued>(a, t, tl, W, H, s, f, F, own, 0, lane);
-      else erode_levels<NMODE, VAR, kQueued>(a, t, tl, d, s, flag == 2);
+      else erode_levels<NMODE, VAR, kQueued, kWalkThreads - 32>(a, t, tl, d, s, flag == 2);
     }
     __syncthreads();
     if (tid == 0) {
@@ -1299,15 +1338,20 @@ __global__ void __launch_bounds__(kWalkThreads, 7) k_tile_queue(StepArgs a) {
   }
 }
 
-enum Kernel { kKernelResident, kKernelRooted, kKernelPull, kKernelQueue, kKernels };
+enum Kernel { kKernelRooted, kKernelPull, kKernelQueue, kKernelResident };  // + width
 
 template <int NMODE, int VAR>
 const void *kernel_of_nv(int k) {
   switch (k) {
-    case kKernelResident: return reinterpret_cast<const void *>(&k_tile_resident<NMODE, VAR>);
     case kKernelRooted: return reinterpret_cast<const void *>(&k_tile_rooted<NMODE, VAR>);
     case kKernelPull: return reinterpret_cast<const void *>(&k_tile_pull<NMODE, VAR>);
-    default: return reinterpret_cast<const void *>(&k_tile_queue<NMODE, VAR>);
+    case kKernelQueue: return reinterpret_cast<const void *>(&k_tile_queue<NMODE, VAR>);
+    case kKernelResident:
+      return reinterpret_cast<const void *>(&k_tile_resident<NMODE, VAR, kResidentThreads[0]>);
+    case kKernelResident + 1:
+      return reinterpret_cast<const void *>(&k_tile_resident<NMODE, VAR, kResidentThreads[1]>);
+    default:
+      return reinterpret_cast<const void *>(&k_tile_resident<NMODE, VAR, kResidentThreads[2]>);
   }
 }
 
@@ -1387,16 +1431,19 @@ cudaError_t launch_tile_erode(const StepArgs &a, const TileRoom &room, cudaStrea
   StepArgs args = a;
   void *params[] = {&args};
   const int var = variant(a);
-  // resident tiles wait for one another: a cooperative launch
-  if (a.tb.n <= room.resident)
-    return cudaLaunchCooperativeKernel(kernel_of(kKernelResident, a.nmode, var), dim3(a.tb.n),
-                                       dim3(kWalkThreads), params, sizeof(TileSmem), s);
+  // Resident tiles wait for one another: a cooperative launch, of the widest
+  // blocks that all fit. 768 threads for one tile an SM measured the same as
+  // 384.
+  for (int w = kResidentWidths - 1; w >= 0; w--)
+    if (a.tb.n <= room.resident[w])
+      return cudaLaunchCooperativeKernel(kernel_of(kKernelResident + w, a.nmode, var), dim3(a.tb.n),
+                                         dim3(kResidentThreads[w]), params, sizeof(TileSmem), s);
   return cudaLaunchKernel(kernel_of(kKernelRooted, a.nmode, var), dim3(a.tb.n), dim3(kRootedThreads),
                           params, sizeof(RootedSmem), s);
 }
 
 cudaError_t launch_tile_rest(const StepArgs &a, const TileRoom &room, cudaStream_t s) {
-  if (a.tb.n <= room.resident) return cudaSuccess;
+  if (a.tb.n <= room.resident[0]) return cudaSuccess;
   StepArgs args = a;
   void *params[] = {&args};
   const int var = variant(a);
@@ -1412,22 +1459,24 @@ cudaError_t launch_tile_rest(const StepArgs &a, const TileRoom &room, cudaStream
 }
 
 cudaError_t prepare_tile_kernels(int nmode, int sms, TileRoom *room) {
-  int least[kKernels] = {1 << 20, 1 << 20, 1 << 20, 1 << 20};
-  for (int var = 0; var < 3; var++)
-    for (int k : {kKernelResident, kKernelRooted, kKernelQueue}) {
+  for (int k = 0; k < kKernelResident + kResidentWidths; k++) {
+    if (k == kKernelPull) continue;
+    const int threads = k < kKernelResident ? kWalkThreads : kResidentThreads[k - kKernelResident];
+    const size_t bytes = k == kKernelRooted ? sizeof(RootedSmem) : sizeof(TileSmem);
+    int least = 1 << 20;
+    for (int var = 0; var < 3; var++) {
       const void *f = kernel_of(k, nmode, var);
-      cudaError_t e = cudaFuncSetAttribute(
-          f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-          (int)(k == kKernelRooted ? sizeof(RootedSmem) : sizeof(TileSmem)));
+      cudaError_t e =
+          cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
       if (e != cudaSuccess) return e;
-      if (k == kKernelRooted) continue;
       int occ = 0;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, kWalkThreads, sizeof(TileSmem));
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, threads, bytes);
       if (e != cudaSuccess) return e;
-      least[k] = occ < least[k] ? occ : least[k];
+      least = occ < least ? occ : least;
     }
-  room->resident = least[kKernelResident] * sms;
-  room->queued = least[kKernelQueue] * sms;
+    if (k == kKernelQueue) room->queued = least * sms;
+    if (k >= kKernelResident) room->resident[k - kKernelResident] = least * sms;
+  }
   return cudaSuccess;
 }
 

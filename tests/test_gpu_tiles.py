@@ -49,6 +49,24 @@ def test_timesteps_equal_the_oracle(pkg, oracle, W, H, n, kind):
             h = ref["h"]
 
 
+@pytest.mark.parametrize("W,H", [(1024, 608), (320, 1952), (1216, 1024), (1344, 928),
+                                 (1536, 1216), (704, 2656)])
+def test_block_widths(pkg, oracle, W, H):
+    """The most tiles that blocks of each width hold on 152 SMs (two, four and
+    six to an SM), and one more: wide levels and narrow ones in one grid."""
+    p = pkg.workload_params()
+    op = Params(*p.as_tuple())
+    h = field(W, H, "young")
+    h.reshape(H, W)[:, W // 2:] += field(W, H, "deep").reshape(H, W)[:, W // 2:]
+    with pkg.FastScape_RBP(W, H, params=p, init=pkg.INIT_ZERO) as m:
+        m.setH(h)
+        m.step(1)
+        ref = oracle.phases(h, W, H, op)
+        assert np.array_equal(m.receivers(), ref["rec"])
+        assert np.array_equal(m.accumulation(), ref["accum"])
+        assert np.array_equal(m.getH(), ref["h"])
+
+
 def test_subset_of_large_grids(pkg):
     """A subset of a batch, its tiles in a list: the others keep their fields."""
     sides = [(900, 800), (1000, 700), (1100, 900), (70, 90)]
