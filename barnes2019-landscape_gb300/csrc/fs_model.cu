@@ -309,9 +309,13 @@ const CUtensorMap *receiver_map(const fs_batch *b) {
   return b->rtma && b->rmap_ok && b->n == 1 ? &b->rmap : nullptr;
 }
 
-cudaError_t reset_ctl(fs_batch *b) {
-  return cudaMemsetAsync(reinterpret_cast<char *>(b->d_ctl) + fs::kCtlResetOffset, 0,
-                         fs::kCtlResetBytes, b->stream);
+// What k_tile_drain resets in the tile walk: the per-realization walk does
+// without that kernel.
+cudaError_t reset_walk(fs_batch *b, const fs::StepArgs &a) {
+  const cudaError_t e = cudaMemsetAsync(reinterpret_cast<char *>(b->d_ctl) + fs::kCtlResetOffset, 0,
+                                        fs::kCtlResetBytes, b->stream);
+  if (e != cudaSuccess) return e;
+  return cudaMemsetAsync(a.rctl, 0, sizeof(fs::RealCtl) * a.nreal, b->stream);
 }
 
 // The per-realization walk runs when chosen, for more than one realization
@@ -323,10 +327,8 @@ bool use_cta(const fs_batch *b, const fs::StepArgs &a) {
 
 // The launches of one timestep (no synchronization).
 cudaError_t launch_step(fs_batch *b, const fs::StepArgs &a) {
-  cudaError_t e = reset_ctl(b);
   const bool cta = use_cta(b, a);
-  if (cta && e == cudaSuccess)
-    e = cudaMemsetAsync(a.rctl, 0, sizeof(fs::RealCtl) * a.nreal, b->stream);
+  cudaError_t e = cta ? reset_walk(b, a) : cudaSuccess;
   if (e == cudaSuccess)
     e = b->exact_receivers ? fs::launch_receivers_exact(a, b->stream)
                            : fs::launch_receivers_fast(a, b->stream, receiver_map(b));
@@ -363,9 +365,8 @@ constexpr int kEvPerStep = 5;
 int timed_step(fs_batch *b, const fs::StepArgs &a, int i) {
   cudaEvent_t *ev = &b->ev[kEvPerStep * i];
   FS_CUDA(cudaEventRecord(ev[0], b->stream));
-  FS_CUDA(reset_ctl(b));
   const bool cta = use_cta(b, a);
-  if (cta) FS_CUDA(cudaMemsetAsync(a.rctl, 0, sizeof(fs::RealCtl) * a.nreal, b->stream));
+  if (cta) FS_CUDA(reset_walk(b, a));
   FS_CUDA(b->exact_receivers ? fs::launch_receivers_exact(a, b->stream)
                              : fs::launch_receivers_fast(a, b->stream, receiver_map(b)));
   FS_CUDA(cudaEventRecord(ev[1], b->stream));
@@ -1578,7 +1579,7 @@ int fs_test_order_from_receivers(fs_model *m, const int32_t *dir) {
   }
   DeviceGuard dg(b->device);
   FS_CUDA(cudaMemcpyAsync(b->rec, v.data(), n, cudaMemcpyHostToDevice, b->stream));
-  FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, sizeof(fs::Ctl), b->stream));
+  FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, fs::kCtlCallResetBytes, b->stream));
   FS_CUDA(cudaMemsetAsync(b->d_rctl, 0, sizeof(fs::RealCtl) * b->n, b->stream));
   const fs::StepArgs a = step_args(b, 0);
   FS_CUDA(fs::launch_tile_drain(a, b->stream));
@@ -1618,7 +1619,7 @@ int fs_test_receiver_fixups(const fs_model *m, int32_t *count) {
   DeviceGuard dg(b->device);
   FS_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(fs::Ctl), cudaMemcpyDeviceToHost, b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
-  *count = b->h_ctl->amb;
+  *count = b->h_ctl->queued;
   return FS_OK;
 }
 
@@ -1638,7 +1639,7 @@ int fs_test_barrier_timeout(fs_model *m, double ms) {
   if (!(ms > 0) || ms > 10000) return set_error(FS_ERR_ARG, "ms must be in (0, 10000]");
   fs_batch *b = m->b;
   DeviceGuard dg(b->device);
-  FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, sizeof(fs::Ctl), b->stream));
+  FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, fs::kCtlCallResetBytes, b->stream));
   FS_CUDA(fs::launch_test_wait(b->d_ctl, 4, static_cast<unsigned long long>(ms * 1e6), b->stream));
   return collect_status(b);
 }

@@ -239,9 +239,7 @@ extern "C" int fs_step_noalloc(double *d_h, int width, int height, const fs_para
   if (in_err != 0) return fail(in_err, "input check failed on the device");
 
   for (int i = 0; i < nsteps; i++) {
-    e = cudaMemsetAsync(reinterpret_cast<char *>(ctl) + fs::kCtlResetOffset, 0,
-                        fs::kCtlResetBytes, s);
-    if (e == cudaSuccess) e = fs::launch_receivers_fast(a, s);
+    e = fs::launch_receivers_fast(a, s);
     if (e == cudaSuccess) e = fs::launch_tile_drain(a, s);
     if (e == cudaSuccess) e = fs::launch_tile_links(a, s);
     if (e == cudaSuccess) e = fs::launch_tile_erode(a, d.room[a.nmode], s);

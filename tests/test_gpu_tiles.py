@@ -91,3 +91,32 @@ def test_subset_of_large_grids(pkg):
                 assert np.array_equal(b.accumulation(r), singles[r].accumulation()), (subset, r)
         for m in singles:
             m.close()
+
+
+@pytest.mark.parametrize("W,H", [(5, 5), (8, 7), (100, 100), (156, 260), (157, 260), (400, 300)])
+@pytest.mark.parametrize("ground", ["flat", "terraces", "tiny"])
+def test_queued_receivers(pkg, oracle, W, H, ground):
+    """Ground that the FP32 filter leaves open, cell by cell: eight threads a
+    cell up to 38912 of them (156 x 260 flat), one above; several timesteps, so
+    that a queue left over from the one before would show."""
+    rng = np.random.default_rng(W * H)
+    h = {"flat": np.zeros(W * H), "terraces": rng.integers(0, 3, W * H).astype(float),
+         "tiny": 1 + rng.integers(0, 4, W * H) * 2.0**-52}[ground]
+    hh = h.reshape(H, W)
+    hh[:2] = hh[-2:] = 0
+    hh[:, :2] = hh[:, -2:] = 0
+    p = pkg.workload_params()
+    op = Params(*p.as_tuple())
+    with pkg.FastScape_RBP(W, H, params=p, init=pkg.INIT_ZERO) as m:
+        m.setH(h)
+        for s in range(3):
+            m.step(1)
+            ref = oracle.phases(h, W, H, op)
+            assert np.array_equal(m.receivers(), ref["rec"]), s
+            assert np.array_equal(m.getH(), ref["h"]), s
+            h = ref["h"]
+        m.setH(h)
+        m.step(3)
+        for s in range(3):
+            h = oracle.phases(h, W, H, op)["h"]
+        assert np.array_equal(m.getH(), h)
