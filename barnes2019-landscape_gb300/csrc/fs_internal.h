@@ -102,7 +102,7 @@ constexpr int kTabStride = 8;
 // donors) spread each block's fixed costs -- staging halo, tile-wide bound,
 // queue scan and atomic -- over more cells; measured fastest from 1000^2 up
 // and within microseconds below.
-constexpr int kRxTile = 32, kRyTile = 96;
+constexpr int kRxTile = 32, kRyTile = 96, kRySmall = 32;
 constexpr int kDxTile = 128, kDyTile = 64;
 
 // The donor kernel reads rec as aligned 32-bit words around each tile row,
@@ -198,7 +198,7 @@ struct StepArgs {
   Ctl *ctl;
   int nreal;
   const Tile *rtiles;
-  int nrtiles;
+  int nrtiles, rrows;      // receiver tiles, and their rows (receiver_rows)
   const Tile *dtiles;
   int ndtiles;
   int nmode;
@@ -218,10 +218,10 @@ constexpr int kMaxReal = 4096;
 // Kernel launchers (fs_kernels.cu). All are asynchronous on `s`.
 cudaError_t launch_receivers_exact(const StepArgs &a, cudaStream_t s);
 // hmap: a single grid's elevation as a {W, H} map of 64-bit elements with
-// {36, 98} boxes (make_receiver_map): the filter stages its tiles by TMA.
+// {36, rows + 2} boxes (make_receiver_map): the filter stages its tiles by TMA.
 cudaError_t launch_receivers_fast(const StepArgs &a, cudaStream_t s,
                                   const CUtensorMap *hmap = nullptr);
-bool make_receiver_map(CUtensorMap *m, const double *h, int W, int H);
+bool make_receiver_map(CUtensorMap *m, const double *h, int W, int H, int rows);
 cudaError_t launch_donors_level0(const StepArgs &a, cudaStream_t s);
 // The tile walk (fs_tile.cu): drainage inside the tiles, drainage between
 // them, and the counts alone or the erosion. `resident` and `queued` are the
@@ -276,9 +276,14 @@ Tolerance make_tolerance(double tol);
 // -RN(1/dr) when the tabled division covers dr (1 <= dr <= 2^60), else 0.
 double neg_recip_dr(double dr);
 int ring_cells(int W, int H);
-// Appends the receiver (kind 0) or donor (kind 1) tiles of realization r to
+// Rows of the receiver tiles of n realizations: 96, or 32 where 96 would give
+// the 152 SMs less than a block each (receivers of 100^2 21.6 -> 18.7 us, of
+// 512^2 22.6 -> 20.5; 1000^2, of 352 tiles, 25.9 at 96 rows and 27.6 at 32,
+// whose halo costs 6% instead of 2%).
+int receiver_rows(int n, const int *W, const int *H);
+// Appends the receiver (rows > 0) or donor (rows = 0) tiles of realization r to
 // out (capacity cap); returns the number appended, or -1 if out is full.
-int append_tiles(int kind, int r, int W, int H, Tile *out, int cap);
+int append_tiles(int rows, int r, int W, int H, Tile *out, int cap);
 // Erosion-table records for counts [k0, k1) into rec (kTabStride doubles
 // each), single-threaded.
 void fill_table_range(double keq, double neq, double meq, double dt, double dr_orth,

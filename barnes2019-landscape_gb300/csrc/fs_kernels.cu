@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) k_receivers_exact(StepArgs a) {
   int8_t *rec = a.rec + d.off;
   const int x = t.x0 + threadIdx.x;
 #pragma unroll 1
-  for (int y = t.y0 + threadIdx.y; y < t.y0 + kRyTile; y += 8) {
+  for (int y = t.y0 + threadIdx.y; y < t.y0 + a.rrows; y += 8) {
     if (x < d.W - 2 && y < d.H - 2) {
       const int c = y * d.W + x;
       rec[c] = (int8_t)receiver_fp64(h, c, d.W, d.dr_orth, d.dr_diag);
@@ -156,21 +156,22 @@ constexpr int kRelEmax = 1123;  // |h| < 2^101
 
 // TMA staging of a single grid's tile (TMA variant): one box of FP64 values,
 // columns x0-2 .. x0+33 (the box's x must be even: 16-byte aligned) and rows
-// y0-1 .. y0+96, into shared memory; the staging then reads the values from
+// y0-1 .. y0+96 (y0+32), into shared memory; the staging then reads the values from
 // there (column offset 1) instead of loading them from global memory.
-constexpr int kRtW = kRxTile + 4, kRtH = kRyTile + 2;
+constexpr int kRtW = kRxTile + 4;
 
 __device__ __forceinline__ uint32_t rf_smem(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// Loads the box into dst with the transaction counted on bar (thread 0).
-__device__ __forceinline__ void rf_tma_tile(void *dst, const CUtensorMap *map, uint64_t *bar,
+// Loads the box of `rows` rows into dst with the transaction counted on bar
+// (thread 0).
+__device__ __forceinline__ void rf_tma_tile(int rows, void *dst, const CUtensorMap *map, uint64_t *bar,
                                             int x, int y) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(rf_smem(bar)) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(rf_smem(bar)),
-               "r"(static_cast<uint32_t>(kRtW * kRtH * 8))
+               "r"(static_cast<uint32_t>(kRtW * rows * 8))
                : "memory");
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
@@ -195,12 +196,12 @@ __device__ __forceinline__ bool rf_wait(uint64_t *bar, unsigned long long limit_
   }
 }
 
-template <bool TMA>
+template <bool TMA, int ROWS>
 __global__ void __launch_bounds__(256)
     k_receivers_filter(const __grid_constant__ CUtensorMap hmap, StepArgs a) {
   if (stopped(a.ctl)) return;
-  __shared__ float s[kRyTile + 2][kRxTile + 3];
-  __shared__ alignas(128) unsigned long long s64[TMA ? kRtH : 1][TMA ? kRtW : 1];
+  __shared__ float s[ROWS + 2][kRxTile + 3];
+  __shared__ alignas(128) unsigned long long s64[TMA ? ROWS + 2 : 1][TMA ? kRtW : 1];
   __shared__ uint64_t s_bar;
   __shared__ unsigned s_wmax[8];
   const Tile t = a.rtiles[blockIdx.x];
@@ -213,12 +214,12 @@ __global__ void __launch_bounds__(256)
   // (|h| >= 2^128, Inf, NaN) are taken over the whole tile.
   float m = 0.f;
   bool bad = false;
-  constexpr int kSw = kRxTile + 2, kSn = (kRyTile + 2) * kSw;
+  constexpr int kSw = kRxTile + 2, kSn = (ROWS + 2) * kSw;
   constexpr int kSPer = (kSn + 255) / 256;  // staged values per thread
   // all of a thread's loads in flight before the first is used
   const int t0 = threadIdx.y * 32 + threadIdx.x;
   if (TMA) {
-    if (t0 == 0) rf_tma_tile(&s64[0][0], &hmap, &s_bar, x0 - 1, y0);
+    if (t0 == 0) rf_tma_tile(ROWS + 2, &s64[0][0], &hmap, &s_bar, x0 - 1, y0);
     __syncthreads();  // the barrier is initialised
     if (!rf_wait(&s_bar, a.timeout_ns)) {
       raise_err(a.ctl, FS_ERR_TIMEOUT, kPhaseNone);
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(256)
   // the largest |f| of each cell's own window instead of the tile's, so a
   // jump inside the tile (base level next to high ground) widens the bound
   // only where it is.
-  constexpr int kRows = kRyTile / 8;
+  constexpr int kRows = ROWS / 8;
   const int lyb = kRows * threadIdx.y + 1;
   auto rows = [&](auto local) {
     constexpr bool LOCAL = decltype(local)::value;
@@ -385,7 +386,7 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   int q = s_qbase + excl;
 #pragma unroll 1
-  for (int r = 0; r < kRyTile / 8; r++) {
+  for (int r = 0; r < kRows; r++) {
     if (qbits >> r & 1u) {
       const int gy = y0 + kRows * threadIdx.y + r + 1;
       a.amb[q] = d.off + gy * W + gx;
@@ -427,8 +428,8 @@ __device__ __forceinline__ int receiver_fp64_eight(const double *h, int c, const
 // The queued cells of k_receivers_filter, with the reference formula in FP64.
 // A thread per cell divides up to eight times in a row (500 clocks each); a
 // queue that leaves seven of eight threads idle gets eight threads per cell
-// (1000^2: 82 us a timestep instead of 86), a longer one is bound by the issue slots, where the skipped
-// neighbours count.
+// (1000^2: 82 us a timestep instead of 86), a longer one is bound by the issue
+// slots, where the skipped neighbours count.
 __global__ void __launch_bounds__(256) k_receivers_fixup(StepArgs a) {
   if (stopped(a.ctl)) return;
   const int n_amb = ld_volatile_i32(&a.ctl->amb);
@@ -917,14 +918,23 @@ int ring_cells(int W, int H) {
   return W * H - (W > 4 ? W - 4 : 0) * (H > 4 ? H - 4 : 0);
 }
 
-int append_tiles(int kind, int r, int W, int H, Tile *out, int cap) {
+int receiver_rows(int n, const int *W, const int *H) {
+  long long tiles = 0;
+  for (int r = 0; r < n; r++)
+    if (W[r] > 4 && H[r] > 4)
+      tiles += (long long)((W[r] - 4 + kRxTile - 1) / kRxTile) * ((H[r] - 4 + kRyTile - 1) / kRyTile);
+  return tiles < 152 ? kRySmall : kRyTile;
+}
+
+int append_tiles(int rows, int r, int W, int H, Tile *out, int cap) {
+  const int kind = rows ? 0 : 1;
   // receivers: interior x, y in [2, W-3]; donors: x, y in [1, W-2]
   // (donor tiles start at x = 0 and cover x in [0, W-2]; x = 0 is skipped)
   const int lo = kind == 0 ? 2 : 1;
   const int xlo = kind == 0 ? 2 : 0;
   const int iw = W - 2 * lo, ih = H - 2 * lo;
   if (iw <= 0 || ih <= 0) return 0;
-  const int tx = kind == 0 ? kRxTile : kDxTile, ty = kind == 0 ? kRyTile : kDyTile;
+  const int tx = kind == 0 ? kRxTile : kDxTile, ty = kind == 0 ? rows : kDyTile;
   const int xw = W - lo - xlo;  // columns [xlo, W-1-lo]
   const int nx = (xw + tx - 1) / tx, ny = (ih + ty - 1) / ty;
   if ((long long)nx * ny > cap) return -1;
@@ -962,20 +972,21 @@ cudaError_t launch_receivers_exact(const StepArgs &a, cudaStream_t s) {
 
 cudaError_t launch_receivers_fast(const StepArgs &a, cudaStream_t s, const CUtensorMap *hmap) {
   if (a.nrtiles == 0) return cudaSuccess;
-  if (hmap) {
-    k_receivers_filter<true><<<a.nrtiles, dim3(32, 8), 0, s>>>(*hmap, a);
-  } else {
-    CUtensorMap none;
-    std::memset(&none, 0, sizeof(none));
-    k_receivers_filter<false><<<a.nrtiles, dim3(32, 8), 0, s>>>(none, a);
-  }
+  CUtensorMap map;
+  if (hmap) map = *hmap;
+  else std::memset(&map, 0, sizeof(map));
+  const auto kernel = a.rrows == kRySmall ? (hmap ? &k_receivers_filter<true, kRySmall>
+                                                  : &k_receivers_filter<false, kRySmall>)
+                                          : (hmap ? &k_receivers_filter<true, kRyTile>
+                                                  : &k_receivers_filter<false, kRyTile>);
+  kernel<<<a.nrtiles, dim3(32, 8), 0, s>>>(map, a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_receivers_fixup<<<8 * sm_count(), 256, 0, s>>>(a);
   return cudaGetLastError();
 }
 
-bool make_receiver_map(CUtensorMap *m, const double *h, int W, int H) {
+bool make_receiver_map(CUtensorMap *m, const double *h, int W, int H, int rows) {
   typedef CUresult (*Encode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
                              const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                              const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -994,7 +1005,7 @@ bool make_receiver_map(CUtensorMap *m, const double *h, int W, int H) {
   if (W % 2 || W < kRxTile + 4 || H < 5) return false;
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(W), static_cast<cuuint64_t>(H)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(W) * 8};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kRtW), static_cast<cuuint32_t>(kRtH)};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kRtW), static_cast<cuuint32_t>(rows + 2)};
   const cuuint32_t estr[2] = {1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<double *>(h), dims, strides, box,
              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,

@@ -132,6 +132,7 @@ struct fs_batch {
   std::vector<double *> tab;
   std::vector<int> tab_cap;
   int walk_sms = 1;
+  int rrows = 0;                                 // rows of a receiver tile
   int erode_isub = 0;                            // the erosion's integer subtractions (n = 1, 2)
   // per-realization walk: used when cta_walk, the launch covers more than one
   // realization and their tiles do not all fit the GPU at once
@@ -282,6 +283,7 @@ fs::StepArgs step_args(const fs_batch *b, int do_erode) {
   a.nreal = b->n;
   a.rtiles = b->d_rtiles;
   a.nrtiles = b->nrtiles;
+  a.rrows = b->rrows;
   a.dtiles = b->d_dtiles;
   a.ndtiles = b->ndtiles;
   a.tb = b->tb;
@@ -526,7 +528,7 @@ int set_active(fs_batch *b, int n, const int *idx) {
       std::vector<fs::Tile> &v = kind == 0 ? rt : dt;
       const size_t at = v.size();
       v.resize(at + static_cast<size_t>(b->W[r] / 32 + 2) * (b->H[r] / 32 + 2));
-      const int got = fs::append_tiles(kind, i, b->W[r], b->H[r], v.data() + at,
+      const int got = fs::append_tiles(kind == 0 ? b->rrows : 0, i, b->W[r], b->H[r], v.data() + at,
                                        static_cast<int>(v.size() - at));
       v.resize(at + std::max(got, 0));
     }
@@ -848,6 +850,7 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
     return fail(*status);
   if (int st = init_tables(b)) return fail(st);
   // Stencil tiles of every realization.
+  b->rrows = fs::receiver_rows(n, widths, heights);
   {
     std::vector<fs::Tile> rt, dt;
     for (int r = 0; r < n; r++) {
@@ -855,7 +858,7 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
         std::vector<fs::Tile> &v = kind == 0 ? rt : dt;
         const size_t at = v.size();
         v.resize(at + static_cast<size_t>(b->W[r] / 32 + 2) * (b->H[r] / 32 + 2));
-        const int got = fs::append_tiles(kind, r, b->W[r], b->H[r], v.data() + at,
+        const int got = fs::append_tiles(kind == 0 ? b->rrows : 0, r, b->W[r], b->H[r], v.data() + at,
                                          static_cast<int>(v.size() - at));
         v.resize(at + std::max(got, 0));
       }
@@ -904,7 +907,7 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
       !cu(fs::prepare_tile_kernels(b->nmode, b->walk_sms, &b->room), "tile kernels"))
     return fail(*status);
   if (b->room.queued < 1) return fail(set_error(FS_ERR_CUDA, "tile kernel cannot be resident"));
-  b->rmap_ok = n == 1 && fs::make_receiver_map(&b->rmap, b->h, b->W[0], b->H[0]);
+  b->rmap_ok = n == 1 && fs::make_receiver_map(&b->rmap, b->h, b->W[0], b->H[0], b->rrows);
   if (!cu(cudaStreamSynchronize(b->stream), "sync")) return fail(*status);
   return b;
 }

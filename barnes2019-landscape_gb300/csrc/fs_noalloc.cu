@@ -147,7 +147,7 @@ extern "C" int fs_step_noalloc(double *d_h, int width, int height, const fs_para
   fs::Tile *rt = g_host_tiles[0], *wt = g_host_tiles[1];
 
   std::lock_guard<std::mutex> lock(g_mutex);
-  const int nrt = fs::append_tiles(0, 0, width, height, rt, kMaxTiles);
+  const int nrt = fs::append_tiles(fs::receiver_rows(1, &width, &height), 0, width, height, rt, kMaxTiles);
   const int nwt = fs::append_walk_tiles(0, width, height, wt, kMaxWalkTiles);
   if (nrt < 0 || nwt < 0) return fail(FS_ERR_ARG, "grid too elongated for the static tile list");
   int dev = 0;
@@ -207,6 +207,7 @@ extern "C" int fs_step_noalloc(double *d_h, int width, int height, const fs_para
   a.nreal = 1;
   a.rtiles = d_rt;
   a.nrtiles = nrt;
+  a.rrows = fs::receiver_rows(1, &width, &height);
   fs::tile_carve(&a.tb, d.base + kOffTiles, nwt);
   a.tb.tiles = d_wt;
   a.tb.n = nwt;

@@ -120,3 +120,21 @@ def test_queued_receivers(pkg, oracle, W, H, ground):
         for s in range(3):
             h = oracle.phases(h, W, H, op)["h"]
         assert np.array_equal(m.getH(), h)
+
+
+@pytest.mark.parametrize("W,H", [(36, 36), (37, 37), (420, 1060), (420, 1064), (612, 772),
+                                 (612, 773)])
+def test_receiver_tile_rows(pkg, oracle, W, H):
+    """Receiver tiles of 32 rows up to 151 of 96 rows, and of 96 beyond: grids
+    at the edge of a tile and around the line between the two."""
+    p = pkg.workload_params()
+    op = Params(*p.as_tuple())
+    h = field(W, H, "young")
+    with pkg.FastScape_RBP(W, H, params=p, init=pkg.INIT_ZERO) as m:
+        for tma in (False, True) if W % 2 == 0 else (False,):  # rows of whole 16 bytes
+            m.setH(h)
+            pkg.check(pkg.library().fs_use_tma_staging(m.handle, int(tma)))
+            m.step(1)
+            ref = oracle.phases(h, W, H, op)
+            assert np.array_equal(m.receivers(), ref["rec"]), tma
+            assert np.array_equal(m.getH(), ref["h"]), tma
