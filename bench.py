@@ -829,9 +829,7 @@ def run_refconst(args, dist, rank, ws, local):
             "config": {"workload": f"FastScape timestep, {side}x{side} FP64, reference initial "
                                    "field, K 2e-6 n 2 m 0.8 U 2e-3 dt 1000 dr {1, sqrt 2}",
                        "levels": levels, "launch": tune},
-            "kernel_ms": {"receivers": t[0] / args.steps, "donors_level0": t[1] / args.steps,
-                          "order": t[7] / args.steps, "accum": t[9] / args.steps,
-                          "erode": t[8] / args.steps},
+            "kernel_ms": kernel_split(t, args.steps),
             "gpu_launches": LAUNCHES_LARGE * args.steps,
             "cpu_baseline": cpu,
             "clocks": clk.summary(),
