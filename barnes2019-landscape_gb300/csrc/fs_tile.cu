@@ -1137,9 +1137,11 @@ __global__ void __launch_bounds__(kRootedThreads, 6) k_tile_rooted(StepArgs a) {
 // is eroded as often (1.3 times on average), by the same operations on the
 // same operands; nothing waits, since the paths' uplifted elevations lie
 // aside and the grid's are read where they were final before. Longer paths
-// are k_tile_queue's.
+// are k_tile_queue's. Waiting for gathers bounds it, so 14 blocks share an SM
+// (48 registers, 40 bytes spilled; with the kernels after it 354 us of a
+// 10000^2 timestep at ten blocks, 317 at 12, 278 at 14, 330 at 16).
 template <int NMODE, int VAR>
-__global__ void __launch_bounds__(kPullThreads) k_tile_pull(StepArgs a) {
+__global__ void __launch_bounds__(kPullThreads, 14) k_tile_pull(StepArgs a) {
   if (stopped(a.ctl)) return;
   __shared__ unsigned s_path[kPullDepth][kPullThreads];  // tile * kPullMost + index
   __shared__ int s_fail;
