@@ -1233,7 +1233,7 @@ __global__ void __launch_bounds__(256) k_tile_mark(StepArgs a) {
 // fit the GPU. A tile is in the ring once at most; a block takes the next one,
 // erodes what has become ready and queues the neighbours that wait for cells
 // it finished. No block waits for a tile, only for the ring, so the order does
-// not matter. A tile with many unfinished cells is staged like k_tile_erode's;
+// not matter. A tile with many unfinished cells is staged like k_tile_resident's;
 // of one with few (young ground: 80 of 2048) only those are gathered.
 // ---------------------------------------------------------------------------
 
