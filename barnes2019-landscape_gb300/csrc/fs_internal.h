@@ -148,7 +148,6 @@ struct TileBufs {
   const Tile *tiles;       // every walk tile of the batch
   const int32_t *list;     // the tiles of this launch (null: all, in order)
   int n;                   // how many
-  int total;               // tiles of the batch (queue capacity)
   const RealDesc *desc;    // every realization (not only the active ones)
   uint8_t *code;           // [t][2048] cell codes
   uint32_t *planes;        // [t][4][64] bit planes of the directions' three
@@ -161,7 +160,7 @@ struct TileBufs {
   int32_t *nstart;         // [t] how many
   unsigned long long *done;  // [t][32] rows of cells whose elevation is final
   int32_t *state;          // [t] kTileQueued | kTileAgain
-  int32_t *queue;          // [total] ring of queued tiles + 1, 0 where empty
+  int32_t *queue;          // [n] ring of queued tiles + 1, 0 where empty
   uint32_t *count;         // drainage count per cell (grid layout)
 };
 // Bytes of one tile in the arrays above (12 KB), before rounding.

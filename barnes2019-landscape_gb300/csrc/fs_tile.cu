@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kDrainThreads) k_tile_drain(StepArgs a) {
   if (tid == 0) {
     a.tb.nstart[t] = s_nstart;
     a.tb.state[t] = 0;
-    a.tb.queue[t] = 0;
+    a.tb.queue[blockIdx.x] = 0;  // a ring of the launch's own n places, whatever tiles it lists
   }
 }
 
@@ -562,10 +562,20 @@ __device__ __forceinline__ unsigned long long ready_exits(const StepArgs &a, int
 __device__ __forceinline__ void queue_push(const StepArgs &a, int u) {
   if (atomicOr(a.tb.state + u, kTileQueued | kTileAgain) & kTileQueued) return;
   __threadfence();  // what the tile's last block wrote, before its next one
-  const unsigned at = atomicAdd(&a.ctl->qtail, 1u) % (unsigned)a.tb.total;
-  // a tile is in the ring once at most, so the place is free or about to be
-  while (atomicCAS(a.tb.queue + at, 0, u + 1) != 0)
+  const unsigned at = atomicAdd(&a.ctl->qtail, 1u) % (unsigned)a.tb.n;
+  // A tile is in the ring once at most, so the place is free, or its block
+  // about to take the tile from it: bounded all the same.
+  unsigned long long t0 = 0;
+  for (unsigned n = 0; atomicCAS(a.tb.queue + at, 0, u + 1) != 0; ++n) {
     if (ld_volatile_i32(&a.ctl->err) != 0) return;
+    if ((n & 63u) != 63u) continue;
+    const unsigned long long now = globaltimer_ns();
+    if (n == 63u) t0 = now;
+    if (now - t0 > a.timeout_ns) {
+      raise_err(a.ctl, FS_ERR_TIMEOUT, kPhaseBarrier);
+      return;
+    }
+  }
 }
 
 // Queues the neighbours that drain into the newly final cells e of the lanes'
@@ -1240,13 +1250,12 @@ __global__ void __launch_bounds__(256) k_tile_mark(StepArgs a) {
 // The next tile, or -1 when every cell is final (one thread).
 __device__ int queue_pop(const StepArgs &a) {
   Ctl *ctl = a.ctl;
-  int32_t *at = a.tb.queue + atomicAdd(&ctl->qhead, 1u) % (unsigned)a.tb.total;
+  int32_t *at = a.tb.queue + atomicAdd(&ctl->qhead, 1u) % (unsigned)a.tb.n;
   unsigned long long t0 = globaltimer_ns();
   int seen = 0;
   for (unsigned n = 0;; ++n) {
     const int v = ld_volatile_i32(at);
-    if (v > 0) {
-      atomicExch(at, 0);
+    if (v > 0 && atomicCAS(at, v, 0) == v) {
       __threadfence();
       return v - 1;
     }
@@ -1396,7 +1405,6 @@ void tile_carve(TileBufs *b, void *base, size_t total) {
     p += (bytes + 255) / 256 * 256;
     return at;
   };
-  b->total = static_cast<int>(total);
   b->code = reinterpret_cast<uint8_t *>(take(total * kWalkCells));
   b->planes = reinterpret_cast<uint32_t *>(take(total * 256 * sizeof(uint32_t)));
   b->local = reinterpret_cast<uint16_t *>(take(total * kWalkCells * sizeof(uint16_t)));

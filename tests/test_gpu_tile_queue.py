@@ -1,0 +1,71 @@
+"""Launches of more tiles than the GPU holds at once, whose trees are rooted in
+their tile, pulled, or eroded from the queue of tiles, in the forms that the
+smaller grids of the other files never take there."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def field(W, H, kind, seed):
+    """As test_gpu_tiles.py's: noise, or a cone with noise."""
+    rng = np.random.default_rng(seed)
+    yy, xx = np.divmod(np.arange(W * H), W)
+    h = rng.uniform(0, 1 if kind == "young" else 3, W * H)
+    if kind == "deep":
+        h += 5.0 * np.minimum.reduce([xx, yy, W - 1 - xx, H - 1 - yy])
+    h[(xx <= 1) | (yy <= 1) | (xx >= W - 2) | (yy >= H - 2)] = 0
+    return h
+
+
+def tiles(sides):
+    return sum((w + 63) // 64 * ((h + 31) // 32) for w, h in sides)
+
+
+def most_resident():
+    """Tiles that the GPU holds at once: six blocks on an SM."""
+    torch = pytest.importorskip("torch")
+    return 6 * torch.cuda.get_device_properties(0).multi_processor_count
+
+
+SIDES = [(300, 200), (1400, 1100), (1000, 700)]
+
+
+@pytest.mark.parametrize("before", ["nothing", "another batch", "a failed timestep"])
+@pytest.mark.parametrize("kinds", [("young", "deep", "young"), ("deep", "young", "young")])
+def test_strict_subset_from_the_queue(pkg, before, kinds):
+    """The first timesteps of a subset that leaves realization 0 out, in memory
+    just allocated, in memory that another batch's tiles and queue lay in, and
+    after a timestep that an error of realization 0 stopped while tiles of the
+    others were queued. The others must evolve as models of their own, and
+    realization 0 must not change."""
+    assert tiles(SIDES[1:]) > most_resident()
+    p = pkg.workload_params()
+    ps = [p, p, p]
+    if before == "a failed timestep":
+        ps[0] = pkg.workload_params(ueq=1e306)  # uplifted to infinity
+    if before == "another batch":
+        with pkg.FastScape_RBP(1700, 1500, params=p, init=pkg.INIT_ZERO) as m:
+            m.setH(field(1700, 1500, "deep", 9))
+            m.step(2)
+    fields = [field(w, h, k, 20 + r) for r, ((w, h), k) in enumerate(zip(SIDES, kinds))]
+    with pkg.FastScapeBatch([w for w, _ in SIDES], [h for _, h in SIDES], ps,
+                            init=pkg.INIT_ZERO) as b:
+        for r in range(3):
+            b.setH(r, fields[r])
+        if before == "a failed timestep":
+            with pytest.raises(pkg.FastScapeError) as e:
+                b.step(1)
+            assert e.value.status == -5
+            for r in range(3):
+                b.setH(r, fields[r])
+        b.set_active([1, 2])
+        b.step(2)
+        assert np.array_equal(b.getH(0), fields[0])
+        for r in (1, 2):
+            with pkg.FastScape_RBP(*SIDES[r], params=p, init=pkg.INIT_ZERO) as m:
+                m.setH(fields[r])
+                m.step(2)
+                assert np.array_equal(b.getH(r), m.getH()), r
+                assert np.array_equal(b.receivers(r), m.receivers()), r
+                assert np.array_equal(b.accumulation(r), m.accumulation()), r
