@@ -550,7 +550,7 @@ class FastScapeBatch:
 
     def use_cta_walk(self, on: bool = True) -> None:
         """One CTA per realization walks its levels (block barriers only)
-        instead of the grid-wide lock step; identical results."""
+        instead of tile by tile; identical results."""
         check(library().fs_batch_use_cta_walk(self._b, int(bool(on))))
 
     def synchronize(self) -> None:

@@ -134,9 +134,9 @@ struct fs_batch {
   int walk_sms = 1;
   int rrows = 0;                                 // rows of a receiver tile
   int erode_isub = 0;                            // the erosion's integer subtractions (n = 1, 2)
-  // per-realization walk: used when cta_walk, the launch covers more than one
-  // realization and their tiles do not all fit the GPU at once
-  bool cta_walk = false;
+  // per-realization walk (use_cta): asked for by the caller, or chosen by the
+  // autotuner (cta_auto)
+  bool cta_walk = false, cta_auto = false;
   // a single grid's receiver filter may stage its tiles by TMA (rmap_ok:
   // the map exists; rtma: in use; the autotuner decides)
   CUtensorMap rmap;
@@ -320,11 +320,17 @@ cudaError_t reset_walk(fs_batch *b, const fs::StepArgs &a) {
   return cudaMemsetAsync(a.rctl, 0, sizeof(fs::RealCtl) * a.nreal, b->stream);
 }
 
-// The per-realization walk runs when chosen, for more than one realization
-// whose tiles the GPU cannot hold at once (resident tiles are faster: 8
-// realizations of eroded 512^2 0.35 against 1.6 ms).
+// The per-realization walk is on: always where the caller asked for it; where
+// the autotuner chose it, for tiles that the GPU cannot hold at once (resident
+// ones are faster: 8 realizations of eroded 512^2 0.35 against 1.6 ms).
+bool cta_on(const fs_batch *b) {
+  const int tiles = b->act_n > 0 ? b->nwt_act : b->tb.n;
+  return b->cta_walk && (!b->cta_auto || tiles > b->room.resident[0]);
+}
+
+// It runs for the timesteps of more than one realization.
 bool use_cta(const fs_batch *b, const fs::StepArgs &a) {
-  return b->cta_walk && a.nreal > 1 && a.do_erode && a.tb.n > b->room.resident[0];
+  return cta_on(b) && a.nreal > 1 && a.do_erode;
 }
 
 // The launches of one timestep (no synchronization).
@@ -1142,9 +1148,11 @@ int autotune(fs_batch *b, int probe, int *chosen) {
     }
   }
   b->rtma = best_rtma;
-  if (st == FS_OK)
+  if (st == FS_OK) {
     b->cta_walk =
         b->n > 1 && *std::max_element(b->size.begin(), b->size.end()) <= kCtaWalkCells;
+    b->cta_auto = true;
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaStreamSynchronize(b->stream);
@@ -1460,13 +1468,14 @@ int fs_launch_config(const fs_model *m, int *order_bps, int *erode_bps, int *gra
 int fs_batch_use_cta_walk(fs_batch *b, int enable) {
   if (!b) return set_error(FS_ERR_ARG, "batch is NULL");
   b->cta_walk = enable != 0;
+  b->cta_auto = false;
   b->graph_dirty = true;
   return FS_OK;
 }
 
 int fs_batch_walk_mode(const fs_batch *b, int *cta) {
   if (!b) return set_error(FS_ERR_ARG, "batch is NULL");
-  if (cta) *cta = b->cta_walk ? 1 : 0;
+  if (cta) *cta = cta_on(b) ? 1 : 0;
   return FS_OK;
 }
 

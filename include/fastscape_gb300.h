@@ -241,9 +241,10 @@ int fs_batch_use_int_sub(fs_batch *b, int enable);
  * probe_steps timesteps of the batch's own state, restores the state and
  * keeps the fastest; chosen[0] = 2 (the erosion's blocks per SM of earlier
  * versions), chosen[1] = graph (fs_batch_launch_config reports every choice).
- * The per-realization walk is chosen (fs_batch_use_cta_walk) when the batch
- * has more than one realization and none has more than 2^19 cells. Results do
- * not depend on the configuration. */
+ * The per-realization walk (fs_batch_use_cta_walk) is chosen when the batch
+ * has more than one realization and none has more than 2^19 cells, for
+ * launches whose tiles do not all fit the GPU at once. Results do not depend
+ * on the configuration. */
 int fs_batch_autotune(fs_batch *b, int probe_steps, int *chosen);
 /* The launch configuration in use: 2 and 2 (once the blocks per SM of kernels
  * that are gone), graph replay (0/1), integer subtractions in the
@@ -254,10 +255,11 @@ int fs_batch_synchronize(const fs_batch *b);
 
 /* Walk of a batch: 0 = tile by tile, as of a single grid; 1 = one CTA per
  * realization (for batches of many small realizations whose hundreds of
- * levels each hold a few thousand cells), where the batch's tiles do not all
- * fit the GPU at once. Identical results; fs_batch_autotune picks by
- * realization size. A launch that covers a single realization always walks
- * tile by tile. No reference counterpart. */
+ * levels each hold a few thousand cells). Identical results; fs_batch_autotune
+ * picks. A launch that covers a single realization always walks tile by tile.
+ * fs_batch_walk_mode: the walk in use; a walk that the autotuner chose is not
+ * in use while the realizations of the next launch (fs_batch_set_active) fit
+ * the GPU tile by tile. No reference counterpart. */
 int fs_batch_use_cta_walk(fs_batch *b, int enable);
 int fs_batch_walk_mode(const fs_batch *b, int *cta);
 
