@@ -16,8 +16,10 @@
 //                               12 KB per 64 x 32 cells
 //   ent, mask                   donor masks and the roots, for a caller that
 //                               reads the masks and for the per-realization
-//                               walk, with pdir, acc, par and lvl_off the
-//                               latter's level order (batches only)
+//                               walk. The rest of that walk's level order lies
+//                               in arrays that its timestep does not need
+//                               otherwise (step_args): 32 bytes a cell in all
+//                               either way
 //   tab_r   double[8*cap_r]     erosion table of realization r per drainage
 //                               count k < cap_r (fs_internal.h); grows on
 //                               demand
@@ -112,9 +114,8 @@ struct fs_batch {
   double *h = nullptr;
   int8_t *rec = nullptr;
   int8_t *rec_alloc = nullptr;  // rec - kRecPad
-  uint8_t *mask = nullptr, *pdir = nullptr;
-  int32_t *ent = nullptr, *par = nullptr, *amb = nullptr, *amb_r = nullptr, *lvl = nullptr;
-  uint32_t *acc = nullptr;
+  uint8_t *mask = nullptr;
+  int32_t *ent = nullptr, *amb = nullptr, *amb_r = nullptr;
   fs::RealDesc *d_desc = nullptr;
   fs::RealCtl *d_rctl = nullptr, *h_rctl = nullptr;
   fs::Ctl *d_ctl = nullptr, *h_ctl = nullptr;
@@ -187,10 +188,9 @@ void free_batch(fs_batch *b) {
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->graph) cudaGraphExecDestroy(b->graph);
-  void *bufs[] = {b->h, b->rec_alloc, b->mask, b->pdir, b->ent, b->par, b->amb,
-                  b->lvl, b->acc, b->d_desc, b->d_rctl, b->d_ctl, b->d_rtiles, b->d_dtiles,
-                  b->d_wtiles, b->count, b->tile_mem, b->d_desc_act, b->d_rctl_act,
-                  b->d_rtiles_act, b->d_dtiles_act, b->d_wlist_act};
+  void *bufs[] = {b->h, b->rec_alloc, b->mask, b->ent, b->amb, b->d_desc, b->d_rctl, b->d_ctl,
+                  b->d_rtiles, b->d_dtiles, b->d_wtiles, b->count, b->tile_mem, b->d_desc_act,
+                  b->d_rctl_act, b->d_rtiles_act, b->d_dtiles_act, b->d_wlist_act};
   for (void *x : bufs) cudaFree(x);
   for (double *t : b->tab) cudaFree(t);
   if (b->h_ctl) cudaFreeHost(b->h_ctl);
@@ -271,12 +271,16 @@ fs::StepArgs step_args(const fs_batch *b, int do_erode) {
   a.rec = b->rec;
   a.mask = b->mask;
   a.ent = b->ent;
-  a.pdir = b->pdir;
-  a.par = b->par;
-  a.acc = b->acc;
   a.amb = b->amb;
   a.amb_r = b->amb_r;
-  a.lvl_off = b->lvl;
+  // The per-realization walk's level order: receivers' places (4 bytes a cell)
+  // and directions (1) in the tiles' memory (6), counts in `count`, which every
+  // timestep leaves stale, and the levels' ends (size + 2 a realization) over
+  // the filter's queues, which the fix-up has emptied by then.
+  a.par = static_cast<int32_t *>(b->tile_mem);
+  a.pdir = reinterpret_cast<uint8_t *>(a.par + b->cells);
+  a.acc = b->count;
+  a.lvl_off = b->amb;
   a.desc = b->d_desc;
   a.rctl = b->d_rctl;
   a.ctl = b->d_ctl;
@@ -649,6 +653,8 @@ int batch_step(fs_batch *b, int k) {
   while (done < k) {
     const int batch = k - done;
     const fs::StepArgs a = step_args(b, 1);
+    b->masks_stale = true;
+    mark_counts(b, 1);
     FS_CUDA(cudaMemsetAsync(b->d_ctl, 0, fs::kCtlCallResetBytes, b->stream));
     if (b->timing == 1) {
       if (int st = ensure_events(b, kEvPerStep * static_cast<size_t>(batch) + 1)) return st;
@@ -679,8 +685,6 @@ int batch_step(fs_batch *b, int k) {
         b->phase_ms[3] += tot;
       }
     }
-    b->masks_stale = true;
-    mark_counts(b, 1);
     if (int st = collect_status(b)) return st;
     const int completed = b->h_ctl->steps_done;
     if (completed > 0) mark_stepped(b);
@@ -801,12 +805,6 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
       !cu(cudaMalloc(&b->d_ctl, sizeof(fs::Ctl)), "cudaMalloc(ctl)") ||
       !cu(cudaMallocHost(&b->h_ctl, sizeof(fs::Ctl)), "cudaMallocHost(ctl)") ||
       !cu(cudaMallocHost(&b->h_rctl, n * sizeof(fs::RealCtl)), "cudaMallocHost(rctl)"))
-    return fail(*status);
-  if (n > 1 &&  // the per-realization walk's
-      (!cu(cudaMalloc(&b->pdir, C), "cudaMalloc(pdir)") ||
-       !cu(cudaMalloc(&b->par, C * sizeof(int32_t)), "cudaMalloc(par)") ||
-       !cu(cudaMalloc(&b->acc, C * sizeof(uint32_t)), "cudaMalloc(acc)") ||
-       !cu(cudaMalloc(&b->lvl, static_cast<size_t>(lb) * sizeof(int32_t)), "cudaMalloc(lvl)")))
     return fail(*status);
   b->rec = b->rec_alloc + fs::kRecPad;
   b->amb_r = b->amb + C;
