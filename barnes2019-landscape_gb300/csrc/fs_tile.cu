@@ -125,10 +125,13 @@ __device__ __forceinline__ int padded(int c) { return c + (c >> 3); }
 
 __global__ void __launch_bounds__(kDrainThreads) k_tile_drain(StepArgs a) {
   if (stopped(a.ctl)) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {  // for this timestep's walk and the next's filter
-    a.ctl->amb = 0;
-    a.ctl->left = a.ctl->progress = 0;
-    a.ctl->qtail = a.ctl->qhead = 0;
+  if (threadIdx.x == 0) {
+    a.tb.queue[blockIdx.x] = 0;  // a ring of the launch's own n places, whatever tiles it lists
+    if (blockIdx.x == 0) {       // for this timestep's walk and the next's filter
+      a.ctl->amb = 0;
+      a.ctl->left = a.ctl->progress = 0;
+      a.ctl->qtail = a.ctl->qhead = 0;
+    }
   }
   __shared__ __align__(16) uint32_t s_w[kPadded];
   __shared__ __align__(16) uint8_t s_code[kWalkCells];
@@ -376,7 +379,6 @@ __global__ void __launch_bounds__(kDrainThreads) k_tile_drain(StepArgs a) {
   if (tid == 0) {
     a.tb.nstart[t] = s_nstart;
     a.tb.state[t] = 0;
-    a.tb.queue[blockIdx.x] = 0;  // a ring of the launch's own n places, whatever tiles it lists
   }
 }
 
