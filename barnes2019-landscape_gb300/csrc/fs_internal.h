@@ -32,7 +32,7 @@ struct Ctl {
   int left;                // cells still to erode in trees that leave their
                            // tile (k_tile_queue), or tiles finished (resident)
   unsigned int qtail, qhead;  // pushes to and pops from the tile queue
-  int progress;            // moves now and then while resident tiles get further
+  int progress;            // moves, like left, while tiles get further (tiles_moved)
   unsigned int bar;        // k_test_wait's arrivals
   // --- kept ---
   int queued;              // cells that the last receiver filter queued

@@ -184,8 +184,9 @@ int fs_use_int_sub(fs_model *m, int enable);
 int fs_launch_config(const fs_model *m, int *order_bps, int *erode_bps, int *graph,
                      int *erode_int_sub);
 
-/* Limit (milliseconds) on every wait of one block for another's progress;
- * default 2000. */
+/* Limit (milliseconds) on every wait of one block for others, counted from
+ * the last progress of any of them (sixteen levels of a tile, or a level that
+ * another tile waits for), however long the timestep takes; default 2000. */
 int fs_set_barrier_timeout(fs_model *m, double ms);
 
 /* Waits for the model's stream. */
