@@ -171,7 +171,8 @@ constexpr size_t kWalkTileBytes = kWalkCells * (1 + 2) + 256 * 4 + kSlots * (4 +
 size_t tile_bytes(size_t total);
 void tile_carve(TileBufs *b, void *base, size_t total);
 // Walk tiles of realization r appended to out (capacity cap), as
-// append_tiles.
+// append_tiles: none where nothing flows, in grids without an interior (whose
+// tiles, three cells wide, would take 128 bytes a cell).
 int append_walk_tiles(int r, int W, int H, Tile *out, int cap);
 
 // Arrays indexed by position i in the level order (the reference's stack):
@@ -245,8 +246,9 @@ cudaError_t launch_cta_erode(const StepArgs &a, int sms, cudaStream_t s);
 cudaError_t launch_check_finite(const double *h, long long n, Ctl *ctl, cudaStream_t s);
 cudaError_t launch_philox_field(double *h, int W, int H, uint64_t seed, cudaStream_t s);
 cudaError_t launch_place_rings(int32_t *ent, int W, int H, cudaStream_t s);
-// Codes of a grid without receivers: -1 on the rings, kPit inside.
-cudaError_t launch_no_receivers(int8_t *rec, int W, int H, cudaStream_t s);
+// Codes and counts of a grid without receivers: -1 on the rings, kPit inside;
+// every cell drains itself.
+cudaError_t launch_no_receivers(int8_t *rec, uint32_t *count, int W, int H, cudaStream_t s);
 cudaError_t launch_test_wait(Ctl *ctl, int blocks, unsigned long long timeout_ns,
                              cudaStream_t s);
 

@@ -853,12 +853,13 @@ __global__ void k_place_rings(int32_t *ent, int W, int H) {
   }
 }
 
-// rec of a grid without receivers: -1 on the rings, kPit inside.
-__global__ void k_no_receivers(int8_t *rec, int W, int H) {
+// rec of a grid without receivers: -1 on the rings, kPit inside; and its counts.
+__global__ void k_no_receivers(int8_t *rec, uint32_t *count, int W, int H) {
   const int size = W * H;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < size; i += gridDim.x * blockDim.x) {
     const int y = i / W, x = i - y * W;
     rec[i] = (int8_t)(x >= 2 && y >= 2 && x < W - 2 && y < H - 2 ? kPit : FS_NO_FLOW);
+    count[i] = 1;
   }
 }
 
@@ -1075,9 +1076,9 @@ cudaError_t launch_place_rings(int32_t *ent, int W, int H, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_no_receivers(int8_t *rec, int W, int H, cudaStream_t s) {
+cudaError_t launch_no_receivers(int8_t *rec, uint32_t *count, int W, int H, cudaStream_t s) {
   const long long blocks = ((long long)W * H + 255) / 256;
-  k_no_receivers<<<(int)(blocks < 4096 ? blocks : 4096), 256, 0, s>>>(rec, W, H);
+  k_no_receivers<<<(int)(blocks < 4096 ? blocks : 4096), 256, 0, s>>>(rec, count, W, H);
   return cudaGetLastError();
 }
 

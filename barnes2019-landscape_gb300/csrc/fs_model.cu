@@ -580,8 +580,9 @@ int set_active(fs_batch *b, int n, const int *idx) {
   if (!dt.empty())
     FS_CUDA(cudaMemcpyAsync(b->d_dtiles_act, dt.data(), dt.size() * sizeof(fs::Tile),
                             cudaMemcpyHostToDevice, b->stream));
-  FS_CUDA(cudaMemcpyAsync(b->d_wlist_act, wl.data(), wl.size() * sizeof(int32_t),
-                          cudaMemcpyHostToDevice, b->stream));
+  if (!wl.empty())
+    FS_CUDA(cudaMemcpyAsync(b->d_wlist_act, wl.data(), wl.size() * sizeof(int32_t),
+                            cudaMemcpyHostToDevice, b->stream));
   FS_CUDA(cudaStreamSynchronize(b->stream));
   b->nrt_act = static_cast<int>(rt.size());
   b->ndt_act = static_cast<int>(dt.size());
@@ -649,6 +650,14 @@ int batch_step(fs_batch *b, int k) {
   if (k < 0) return set_error(FS_ERR_ARG, "step count must be >= 0 (got %d)", k);
   if (k == 0) return FS_OK;
   DeviceGuard dg(b->device);
+  {
+    const fs::StepArgs a = step_args(b, 1);
+    if (a.tb.n == 0 && !use_cta(b, a)) {  // no realization has an interior: nothing changes
+      mark_stepped(b);
+      b->steps += k;
+      return FS_OK;
+    }
+  }
   int done = 0;
   while (done < k) {
     const int batch = k - done;
@@ -779,7 +788,8 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
     lb += b->size.back() + 2;
     b->tile0.push_back(static_cast<int>(wt.size()));
     const size_t at = wt.size();
-    wt.resize(at + static_cast<size_t>(widths[r] / fs::kWalkW + 1) * (heights[r] / fs::kWalkH + 1));
+    if (std::min(widths[r], heights[r]) > 4)
+      wt.resize(at + static_cast<size_t>(widths[r] / fs::kWalkW + 1) * (heights[r] / fs::kWalkH + 1));
     wt.resize(at + fs::append_walk_tiles(r, widths[r], heights[r], wt.data() + at,
                                          static_cast<int>(wt.size() - at)));
   }
@@ -798,8 +808,12 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
       !cu(cudaMalloc(&b->ent, C * sizeof(int32_t)), "cudaMalloc(ent)") ||
       !cu(cudaMalloc(&b->amb, 2 * C * sizeof(int32_t)), "cudaMalloc(amb)") ||
       !cu(cudaMalloc(&b->count, C * sizeof(uint32_t)), "cudaMalloc(count)") ||
-      !cu(cudaMalloc(&b->tile_mem, fs::tile_bytes(wt.size())), "cudaMalloc(tiles)") ||
-      !cu(cudaMalloc(&b->d_wtiles, wt.size() * sizeof(fs::Tile)), "cudaMalloc(wtiles)") ||
+      // the tiles' arrays, and at least what borrows them: a level order
+      // (step_args) or a read-back (net_ints)
+      !cu(cudaMalloc(&b->tile_mem, std::max(fs::tile_bytes(wt.size()), 5 * C + 256)),
+          "cudaMalloc(tiles)") ||
+      !cu(cudaMalloc(&b->d_wtiles, std::max<size_t>(1, wt.size()) * sizeof(fs::Tile)),
+          "cudaMalloc(wtiles)") ||
       !cu(cudaMalloc(&b->d_desc, n * sizeof(fs::RealDesc)), "cudaMalloc(desc)") ||
       !cu(cudaMalloc(&b->d_rctl, n * sizeof(fs::RealCtl)), "cudaMalloc(rctl)") ||
       !cu(cudaMalloc(&b->d_ctl, sizeof(fs::Ctl)), "cudaMalloc(ctl)") ||
@@ -816,10 +830,9 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
   b->tb.count = b->count;
   // Rings keep NO_FLOW forever (fastscape_RB.cpp:361-362) and ring-0 cells
   // never have donors: receivers and masks are written for the interior only.
-  if (!cu(cudaMemcpyAsync(b->d_wtiles, wt.data(), wt.size() * sizeof(fs::Tile),
-                          cudaMemcpyHostToDevice, b->stream),
-          "upload(wtiles)") ||
-      !cu(cudaMemsetAsync(b->count, 0, C * sizeof(uint32_t), b->stream), "memset(count)") ||
+  if ((!wt.empty() && !cu(cudaMemcpyAsync(b->d_wtiles, wt.data(), wt.size() * sizeof(fs::Tile),
+                                          cudaMemcpyHostToDevice, b->stream),
+                          "upload(wtiles)")) ||
       !cu(cudaMemsetAsync(b->mask, 0, C, b->stream), "memset(mask)") ||
       !cu(cudaMemsetAsync(b->d_rctl, 0, n * sizeof(fs::RealCtl), b->stream), "memset(rctl)") ||
       !cu(cudaMemsetAsync(b->d_ctl, 0, sizeof(fs::Ctl), b->stream), "memset(ctl)"))
@@ -886,7 +899,9 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
   std::vector<double> host;
   for (int r = 0; r < n; r++) {
     if (!cu(fs::launch_place_rings(b->ent + b->off[r], b->W[r], b->H[r], b->stream), "rings") ||
-        !cu(fs::launch_no_receivers(b->rec + b->off[r], b->W[r], b->H[r], b->stream), "receivers"))
+        !cu(fs::launch_no_receivers(b->rec + b->off[r], b->count + b->off[r], b->W[r], b->H[r],
+                                    b->stream),
+            "receivers"))
       return fail(*status);
     const uint64_t seed = seeds ? seeds[r] : 0;
     double *hr = b->h + b->off[r];

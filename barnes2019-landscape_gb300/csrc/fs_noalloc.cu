@@ -14,9 +14,9 @@
 // Limits and sharing:
 //   * grids of at most FS_NOALLOC_MAX_CELLS cells (width*height); larger
 //     grids are rejected with FS_ERR_ARG;
-//   * the scratch array (~50 MB: receivers, drainage counts, the tile walk's
+//   * the scratch array (~41 MB: receivers, drainage counts, the tile walk's
 //     arrays for the most tiles a grid within the limit can have -- a
-//     3-cell-wide one, 2731 -- the erosion table for every possible count,
+//     5-cell-wide one, 1639 -- the erosion table for every possible count,
 //     stencil tiles, descriptors and the control block) lives in the library
 //     image, so every GPU that loads the library holds it until the process
 //     exits;
@@ -48,7 +48,7 @@ namespace {
 constexpr size_t kMaxCells = FS_NOALLOC_MAX_CELLS;
 constexpr size_t kTabRecords = kMaxCells + 1;  // counts 0..kMaxCells
 constexpr int kMaxTiles = 4096;                // receiver tiles
-constexpr size_t kMaxWalkTiles = kMaxCells / 3 / fs::kWalkH + 1;  // 3 cells wide
+constexpr size_t kMaxWalkTiles = kMaxCells / 5 / fs::kWalkH + 1;  // 5 cells wide
 constexpr int kMaxDevices = 64;
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
@@ -238,6 +238,7 @@ extern "C" int fs_step_noalloc(double *d_h, int width, int height, const fs_para
   if (e != cudaSuccess) return cuda_fail(e, "scratch reset");
   if (in_err == FS_ERR_NONFINITE) return fail(FS_ERR_NONFINITE, "input holds NaN or Inf");
   if (in_err != 0) return fail(in_err, "input check failed on the device");
+  if (nwt == 0) return FS_OK;  // no interior: a timestep changes nothing
 
   for (int i = 0; i < nsteps; i++) {
     e = fs::launch_receivers_fast(a, s);

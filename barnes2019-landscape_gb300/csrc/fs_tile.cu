@@ -1434,6 +1434,7 @@ void tile_carve(TileBufs *b, void *base, size_t total) {
 }
 
 int append_walk_tiles(int r, int W, int H, Tile *out, int cap) {
+  if (W <= 4 || H <= 4) return 0;  // no cell has a receiver or rises
   const int ntx = (W + kWalkW - 1) / kWalkW, nty = (H + kWalkH - 1) / kWalkH;
   if ((long long)ntx * nty > cap) return -1;
   int n = 0;
@@ -1443,16 +1444,19 @@ int append_walk_tiles(int r, int W, int H, Tile *out, int cap) {
 }
 
 cudaError_t launch_tile_drain(const StepArgs &a, cudaStream_t s) {
+  if (a.tb.n == 0) return cudaSuccess;
   k_tile_drain<<<a.tb.n, kDrainThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_tile_links(const StepArgs &a, cudaStream_t s) {
+  if (a.tb.n == 0) return cudaSuccess;
   k_tile_links<<<(a.tb.n + 7) / 8, 256, 0, s>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_tile_counts(const StepArgs &a, cudaStream_t s) {
+  if (a.tb.n == 0) return cudaSuccess;
   k_tile_counts<<<a.tb.n, kWalkThreads, 0, s>>>(a);
   return cudaGetLastError();
 }

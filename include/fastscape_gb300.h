@@ -321,7 +321,7 @@ int fs_batch_get_shape(const fs_batch *b, int r, int *width, int *height);
  * may not allocate device memory while running (a host application that
  * owns all device memory through its own pool, a latency-critical loop where
  * cudaMalloc/cudaFree would synchronize the device, a plugin with a fixed
- * footprint). All scratch (~50 MB) is one static device array in the
+ * footprint). All scratch (~41 MB) is one static device array in the
  * library, held on every GPU that loads it until the process exits, shared
  * by all calls and keeping the last call's contents: calls that overlap on
  * the GPU race. The library itself serializes its calls (a lock, and each
