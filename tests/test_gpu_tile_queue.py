@@ -69,3 +69,46 @@ def test_strict_subset_from_the_queue(pkg, before, kinds):
                 assert np.array_equal(b.getH(r), m.getH()), r
                 assert np.array_equal(b.receivers(r), m.receivers()), r
                 assert np.array_equal(b.accumulation(r), m.accumulation()), r
+
+
+@pytest.mark.parametrize("kind", ["young", "deep"])
+@pytest.mark.parametrize("n", [1.0, 2.0])
+def test_erosion_paths_agree(pkg, n, kind):
+    """Every arithmetic of the erosion on more tiles than fit the GPU: the
+    integer subtractions and the FP64 ones against the reference's Newton loop
+    taken literally, bit for bit."""
+    W, H = 1601, 1483
+    assert tiles([(W, H)]) > most_resident()
+    p = pkg.workload_params() if n == 1.0 else pkg.reference_params()
+    h = field(W, H, kind, 31)
+    out = []
+    for int_sub, literal in ((0, 0), (1, 0), (0, 1)):
+        with pkg.FastScape_RBP(W, H, params=p, init=pkg.INIT_ZERO) as m:
+            pkg.check(pkg.library().fs_use_int_sub(m.handle, int_sub))
+            pkg.check(pkg.library().fs_test_set_erosion_path(m.handle, literal))
+            m.setH(h)
+            m.step(3)
+            out.append((m.getH(), m.accumulation()))
+    for g, acc in out[:2]:
+        assert np.array_equal(g, out[2][0])
+        assert np.array_equal(acc, out[2][1])
+
+
+@pytest.mark.parametrize("kind", ["young", "deep"])
+@pytest.mark.parametrize("n", [2.0, 1.5])
+def test_steeper_exponents_against_the_oracle(pkg, oracle, n, kind):
+    """n = 2 and a general n there, each timestep from the oracle's ground,
+    within test_gpu_parity.py's 1e-12 for n != 1."""
+    from oracle.pyoracle import Params
+    W, H = 1601, 1483
+    p = pkg.reference_params() if n == 2.0 else pkg.workload_params(neq=n)
+    h = field(W, H, kind, 32)
+    with pkg.FastScape_RBP(W, H, params=p, init=pkg.INIT_ZERO) as m:
+        for s in range(2):
+            m.setH(h)
+            m.step(1)
+            ref = oracle.phases(h.copy(), W, H, Params(*p.as_tuple()))
+            assert np.array_equal(m.receivers(), ref["rec"]), s
+            assert np.array_equal(m.accumulation(), ref["accum"]), s
+            np.testing.assert_allclose(m.getH(), ref["h"], rtol=1e-12, atol=0)
+            h = ref["h"]
