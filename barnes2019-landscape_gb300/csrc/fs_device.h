@@ -63,6 +63,36 @@ __device__ __forceinline__ void raise_err(Ctl *ctl, int code, int phase) {
   if (atomicCAS(&ctl->err, 0, code) == 0) ctl->err_detail = phase;
 }
 
+// Barrier of all blocks of a cooperative launch, with a limit: false after an
+// error, whoever raised it. epoch counts the caller's barriers.
+__device__ __forceinline__ bool grid_barrier(Ctl *ctl, unsigned &epoch,
+                                             unsigned long long timeout_ns) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned target = ++epoch * gridDim.x;
+    __threadfence();  // the block's writes before its arrival
+    atomicAdd(&ctl->bar, 1u);
+    int ok = 1;
+    unsigned long long t0 = 0;
+    for (unsigned n = 1; ld_acquire_u32(&ctl->bar) < target; ++n) {
+      if ((n & 15u) == 0) {
+        const unsigned long long now = globaltimer_ns();
+        if (n == 16) t0 = now;
+        if (now - t0 > timeout_ns) raise_err(ctl, FS_ERR_TIMEOUT, kPhaseBarrier);
+        if (ld_volatile_i32(&ctl->err) != 0) {
+          ok = 0;
+          break;
+        }
+      }
+      __nanosleep(32);
+    }
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
 __device__ __forceinline__ bool stopped(const Ctl *ctl) {
   return (ld_volatile_i32(&ctl->err) | ld_volatile_i32(&ctl->abort_k)) != 0;
 }

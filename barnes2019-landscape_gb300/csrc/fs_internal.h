@@ -33,7 +33,8 @@ struct Ctl {
                            // tile (k_tile_queue), or tiles finished (resident)
   unsigned int qtail, qhead;  // pushes to and pops from the tile queue
   int progress;            // moves, like left, while tiles get further (tiles_moved)
-  unsigned int bar;        // k_test_wait's arrivals
+  unsigned int bar;        // blocks' arrivals (k_tile_front, k_test_wait)
+  unsigned int front[3];   // k_tile_front: cells of a round (rotating)
   // --- kept ---
   int queued;              // cells that the last receiver filter queued
 };
@@ -224,11 +225,12 @@ cudaError_t launch_receivers_fast(const StepArgs &a, cudaStream_t s,
 bool make_receiver_map(CUtensorMap *m, const double *h, int W, int H, int rows);
 cudaError_t launch_donors_level0(const StepArgs &a, cudaStream_t s);
 // The tile walk (fs_tile.cu): drainage inside the tiles, drainage between
-// them, and the counts alone or the erosion. `resident` and `queued` are the
-// blocks that k_tile_resident and k_tile_queue can keep on the GPU at once.
+// them, and the counts alone or the erosion. `resident`, `queued` and `front`
+// are the blocks that k_tile_resident, k_tile_queue and k_tile_front can
+// keep on the GPU at once.
 constexpr int kResidentWidths = 3;  // of k_tile_resident's blocks, narrowest first
 struct TileRoom {
-  int resident[kResidentWidths] = {}, queued = 0;
+  int resident[kResidentWidths] = {}, queued = 0, front = 0;
 };
 cudaError_t launch_tile_drain(const StepArgs &a, cudaStream_t s);
 cudaError_t launch_tile_links(const StepArgs &a, cudaStream_t s);

@@ -20,8 +20,10 @@
 //                       their receivers become final;
 //   4. otherwise
 //      k_tile_rooted    the same for the trees rooted in the tile,
-//      k_tile_pull      the cells of short paths into other tiles, each by
-//                       itself (k_tile_mark tells the queue),
+//      k_tile_pull      (n = 1) the cells of short paths into other tiles, each
+//                       by itself (k_tile_mark tells the queue),
+//      k_tile_front     (n != 1, or many cells left) cells in rounds of the
+//                       whole GPU,
 //      k_tile_queue     what is left, from a queue of tiles.
 // Counts are sums of integers, exact in any order, and a cell is eroded by
 // the same operations from the same operands as in the reference's order, so
@@ -55,6 +57,21 @@ constexpr int kPullMost = 256;     // unfinished cells k_tile_pull takes from a 
 constexpr int kPullDepth = 16;     // and how far up it follows their receivers
 constexpr int kPullThreads = 96;
 constexpr int kRootedThreads = 192;
+constexpr int kFrontThreads = 384;
+// n = 1: cells of trees that leave their tile from which k_tile_front takes
+// them. 256 realizations of eroded 512^2, 60e6 such cells, take 11.9 ms a
+// timestep with the queue alone and 7.6 so; eroded 2000^2, 3e6, 1.36 and 1.40.
+constexpr int kFrontCells = 1 << 23;
+// Rounds too narrow for the GPU's threads end when more than so many would
+// follow: 10000^2 with n = 2, 65 levels, takes 7.26 ms a timestep at 4 and 8 and
+// 7.00 at 16; ended by width alone, 7.21 below 2048 cells and 7.24 below 131072,
+// with n = 1.5 and 12 levels 36.5 below 131072 (35.7 at 4 to 16).
+constexpr int kFrontRounds = 16;
+// n != 1: a tile's levels narrower than this are left to k_tile_front, which
+// has full warps for them: with n = 1.5 35.7 -> 34.8 ms, with n = 2 7.00 -> 6.85
+// (96: 6.80, but 13.5 instead of 12.7 at 515 levels; 192: 7.07).
+constexpr int kRootedFew = 48;
+static_assert(kWalkW == 64 && kWalkH == 32, "a cell's tile: x >> 6, y >> 5");
 constexpr uint32_t kNoSink = 0xFFFFu;
 constexpr int kFinished = 1 << 30;
 constexpr int kTileQueued = 1, kTileAgain = 2;
@@ -131,6 +148,7 @@ __global__ void __launch_bounds__(kDrainThreads) k_tile_drain(StepArgs a) {
       a.ctl->amb = 0;
       a.ctl->left = a.ctl->progress = 0;
       a.ctl->qtail = a.ctl->qhead = 0;
+      a.ctl->bar = a.ctl->front[0] = a.ctl->front[1] = 0;
     }
   }
   __shared__ __align__(16) uint32_t s_w[kPadded];
@@ -1040,11 +1058,12 @@ __global__ void __launch_bounds__(kRootedThreads, 6) k_tile_rooted(StepArgs a) {
   const RealDesc &d = a.tb.desc[tl.r];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wt = (int)threadIdx.x - 32;
   constexpr int kWarps = kRootedThreads / 32, kErode = kRootedThreads - 32;
+  constexpr bool kRounds = NMODE != kNOne;  // what is left is k_tile_front's
   const uint64_t udt = (uint64_t)__double_as_longlong(d.u_dt);
   const Tolerance tol = d.tol;
   tile_stage<kRootedThreads>(a, tl, d, s.h);
   Front f;
-  unsigned long long F = 0, final = 0;
+  unsigned long long F = 0, F1 = 0, final = 0;  // the last level found, the one before, all
   int pos = 0;
   if (wid == 0) {  // levels 0 to 2
     front_load(f, a.tb.planes + (size_t)t * 256, lane);
@@ -1053,6 +1072,7 @@ __global__ void __launch_bounds__(kRootedThreads, 6) k_tile_rooted(StepArgs a) {
     reinterpret_cast<unsigned long long *>(s.words[0])[lane] = pits;
 #pragma unroll
     for (int q = 0; q < 2; q++) {
+      if (kRounds) F1 = F;
       F = front_next(f, F, lane);
       final |= F;
       const int nl = __popc((uint32_t)F), n = nl + __popc((uint32_t)(F >> 32));
@@ -1102,7 +1122,12 @@ __global__ void __launch_bounds__(kRootedThreads, 6) k_tile_rooted(StepArgs a) {
   for (int L = 1;; ++L) {
     const int lo = s.end[(L - 1) & 3], hi = s.end[L & 3], hi2 = s.end[(L + 1) & 3];
     if (lo == hi) break;
+    if (kRounds && hi - lo < kRootedFew) {  // k_tile_front's from here on
+      if (wid == 0) final &= ~(F | F1);
+      break;
+    }
     if (wid == 0) {  // level L + 2
+      if (kRounds) F1 = F;
       F = front_next(f, F, lane);
       final |= F;
       pos = front_emit(F, lane, s.list, pos);
@@ -1119,19 +1144,20 @@ __global__ void __launch_bounds__(kRootedThreads, 6) k_tile_rooted(StepArgs a) {
   }
   tile_store<kRootedThreads>(a, tl, d, s.h);
   // The cells of trees that leave the tile: a few for k_tile_pull, many for
-  // the queue. Only their counts go to memory (the others': k_tile_counts,
-  // when a caller asks).
+  // the queue, or all for k_tile_front. Only their counts go to memory (the
+  // others': k_tile_counts, when a caller asks).
   const TileRest rest = tile_rest(a, t);
   if (wid == 0) {
     a.tb.done[(size_t)t * kWalkH + lane] = final;
     const unsigned long long rows = f.flow & ~final;
     int at;
     const int left = front_emit(rows, lane, s.list, 0, &at);
-    rest.row[lane] = (uint16_t)at;
+    if (!kRounds) rest.row[lane] = (uint16_t)at;
     if (lane == 0) {
-      const bool pull = left <= kPullMost;
+      const bool pull = kRounds || left <= kPullMost;
       s.left = left;
       a.tb.nstart[t] = pull ? left : 0;
+      if (kRounds && left) atomicAdd(&a.ctl->left, left);
       if (!pull) {
         atomicAdd(&a.ctl->left, left);
         a.tb.state[t] = kTileQueued;
@@ -1144,7 +1170,7 @@ __global__ void __launch_bounds__(kRootedThreads, 6) k_tile_rooted(StepArgs a) {
   for (int i = threadIdx.x; i < left; i += kRootedThreads) {
     const int c = s.list[i];
     a.tb.count[d.off + (size_t)(tl.y0 + (c >> 6)) * d.W + tl.x0 + (c & 63)] = s.acc[c];
-    if (left <= kPullMost) {
+    if (!kRounds && left <= kPullMost) {
       rest.cell[i] = (uint16_t)(c | (s.code[c] & 7) << 11);
       rest.h0[i] = uplift_bits(s.h[c], udt);
       rest.count[i] = s.acc[c];
@@ -1369,14 +1395,132 @@ __global__ void __launch_bounds__(kWalkThreads, 7) k_tile_queue(StepArgs a) {
   }
 }
 
-enum Kernel { kKernelRooted, kKernelPull, kKernelQueue, kKernelResident };  // + width
+// ---------------------------------------------------------------------------
+// 5. Rounds of the whole GPU, where many cells are left or a cell takes long
+// (n != 1): the cells whose receivers are final, then their donors, and so on,
+// from one list that grows. Full warps are what counts there. k_tile_pull's lanes
+// follow paths of their own and erode shared cells again (10000^2 with n = 1.5,
+// 12 levels: 7.1 ms for 4% of the cells, 1.7 in rounds), and a tile from the
+// queue is visited for few ready cells at a time. A round lasts as long as its
+// slowest cell and a barrier, 20 us with n = 2, so the narrow rounds of long paths
+// are left to k_tile_queue, whose tiles do not wait for one another's.
+// ---------------------------------------------------------------------------
+template <int NMODE, int VAR>
+__global__ void __launch_bounds__(kFrontThreads, 2) k_tile_front(StepArgs a) {
+  Ctl *ctl = a.ctl;
+  if (stopped(ctl)) return;
+  const int lane = threadIdx.x & 31;
+  const int warp = (int)(blockIdx.x * kFrontThreads + threadIdx.x) >> 5;
+  const int warps = (int)gridDim.x * (kFrontThreads / 32);
+  const int all = ld_volatile_i32(&ctl->left);  // before the first barrier: written after it
+  if (NMODE == kNOne && all < kFrontCells) return;
+  // the list: cells numbered in their tile, and tiles
+  int32_t *cell = a.amb, *tile = a.amb_r;
+  // places for n entries of this lane (whole warps)
+  auto places = [&](unsigned *count, int n) -> int {
+    int incl = n;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+      const int v = __shfl_up_sync(kFull, incl, s);
+      if (lane >= s) incl += v;
+    }
+    int at = 0;
+    if (lane == 31 && incl) at = (int)atomicAdd(count, (unsigned)incl);
+    return __shfl_sync(kFull, at, 31) + incl - n;
+  };
+  for (int w = warp; w < a.tb.n; w += warps) {
+    const int t = tile_of(a, w);
+    if (NMODE != kNOne && a.tb.nstart[t] == 0) continue;  // nothing left
+    const Tile tl = a.tb.tiles[t];
+    const RealDesc &d = a.tb.desc[tl.r];
+    Front f;
+    front_load(f, a.tb.planes + (size_t)t * 256, lane);
+    const unsigned long long own = a.tb.done[(size_t)t * kWalkH + lane];
+    unsigned long long F =
+        (ready_exits(a, t, tl, d.W, d.H, f, lane) | front_next(f, own, lane)) & ~own;
+    int at = places(&ctl->front[0], __popcll(F));
+    for (; F; F &= F - 1, ++at) {
+      cell[at] = 64 * lane + __ffsll((long long)F) - 1;
+      tile[at] = t;
+    }
+  }
+  unsigned epoch = 0;
+  int lo = 0;
+  for (unsigned r = 0;; ++r) {
+    if (!grid_barrier(ctl, epoch, a.timeout_ns)) return;
+    const int n = ld_volatile_i32(reinterpret_cast<const int *>(&ctl->front[r % 3]));
+    if (n == 0 || (n < 32 * warps && all - lo > kFrontRounds * n)) break;
+    unsigned *next = &ctl->front[(r + 1) % 3];
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->front[(r + 2) % 3] = 0;
+    const int hi = lo + n;
+    for (int i = lo + 32 * warp; i < hi; i += 32 * warps) {
+      unsigned donors = 0;
+      int c = 0, t = 0;
+      Tile tl;
+      if (i + lane < hi) {
+        c = __ldcg(cell + i + lane);
+        t = __ldcg(tile + i + lane);
+        tl = a.tb.tiles[t];
+        const RealDesc &d = a.tb.desc[tl.r];
+        const int g = (tl.y0 + (c >> 6)) * d.W + tl.x0 + (c & 63);
+        const int8_t *rec = a.rec + d.off + g;
+        unsigned long long *h = reinterpret_cast<unsigned long long *>(a.h + d.off) + g;
+        const int dir = __ldg(rec);
+        const uint64_t h0 = __ldcg(h), hn = __ldcg(h + nbr_off(dir, d.W));
+        Cell e;
+        cell_table<NMODE, VAR>(e, d, __ldcg(a.tb.count + d.off + g), dir);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          if (__ldg(rec + nbr_off(k, d.W)) == ((k + 4) & 7)) donors |= 1u << k;
+        e.h0 = uplift_bits(h0, (uint64_t)__double_as_longlong(d.u_dt));
+        *h = cell_erode<NMODE, VAR>(e, d.tol, a.neq, ctl, hn);
+      }
+      int at = hi + places(next, __popc(donors));
+      for (; donors; donors &= donors - 1, ++at) {
+        const int k = __ffs(donors) - 1;
+        const int x = (c & 63) + dir_dx(k), y = (c >> 6) + dir_dy(k);
+        cell[at] = (y & (kWalkH - 1)) << 6 | (x & (kWalkW - 1));
+        tile[at] = t + (y >> 5) * tl.ntx + (x >> 6);
+      }
+    }
+    lo = hi;
+  }
+  // For the queue, in place of what k_tile_rooted and k_tile_pull put there:
+  // what is final, and the tiles with cells left.
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->left = all - lo;
+    ctl->qtail = 0;
+  }
+  for (int i = 32 * warp + lane; i < a.tb.n; i += 32 * warps) a.tb.queue[i] = 0;
+  if (lo == all) return;
+  for (int i = 32 * warp + lane; i < lo; i += 32 * warps) {
+    const int c = __ldcg(cell + i);
+    atomicOr(a.tb.done + (size_t)__ldcg(tile + i) * kWalkH + (c >> 6), 1ull << (c & 63));
+  }
+  if (!grid_barrier(ctl, epoch, a.timeout_ns)) return;
+  for (int w = warp; w < a.tb.n; w += warps) {
+    const int t = tile_of(a, w);
+    const unsigned long long flow =
+        __ldg(reinterpret_cast<const unsigned long long *>(a.tb.planes + (size_t)t * 256 + 192) + lane);
+    if (!__any_sync(kFull, (flow & ~ld_relaxed_u64(a.tb.done + (size_t)t * kWalkH + lane)) != 0))
+      continue;
+    if (lane == 0) {
+      a.tb.state[t] = kTileQueued;
+      a.tb.queue[atomicAdd(&ctl->qtail, 1u)] = t + 1;
+    }
+  }
+}
+
+enum Kernel { kKernelRooted, kKernelPull, kKernelQueue, kKernelFront, kKernelResident };  // + width
 
 template <int NMODE, int VAR>
 const void *kernel_of_nv(int k) {
+  if constexpr (NMODE == kNOne)
+    if (k == kKernelPull) return reinterpret_cast<const void *>(&k_tile_pull<NMODE, VAR>);
   switch (k) {
-    case kKernelRooted: return reinterpret_cast<const void *>(&k_tile_rooted<NMODE, VAR>);
-    case kKernelPull: return reinterpret_cast<const void *>(&k_tile_pull<NMODE, VAR>);
+    case kKernelFront: return reinterpret_cast<const void *>(&k_tile_front<NMODE, VAR>);
     case kKernelQueue: return reinterpret_cast<const void *>(&k_tile_queue<NMODE, VAR>);
+    case kKernelRooted: return reinterpret_cast<const void *>(&k_tile_rooted<NMODE, VAR>);
     case kKernelResident:
       return reinterpret_cast<const void *>(&k_tile_resident<NMODE, VAR, kResidentThreads[0]>);
     case kKernelResident + 1:
@@ -1481,12 +1625,20 @@ cudaError_t launch_tile_rest(const StepArgs &a, const TileRoom &room, cudaStream
   StepArgs args = a;
   void *params[] = {&args};
   const int var = variant(a);
-  cudaError_t e = cudaLaunchKernel(kernel_of(kKernelPull, a.nmode, var), dim3(a.tb.n),
-                                   dim3(kPullThreads), params, 0, s);
-  if (e != cudaSuccess) return e;
-  k_tile_mark<<<(a.tb.n + 7) / 8, 256, 0, s>>>(a);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  if (a.nmode == kNOne) {
+    cudaError_t e = cudaLaunchKernel(kernel_of(kKernelPull, a.nmode, var), dim3(a.tb.n),
+                                     dim3(kPullThreads), params, 0, s);
+    if (e != cudaSuccess) return e;
+    k_tile_mark<<<(a.tb.n + 7) / 8, 256, 0, s>>>(a);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  if (a.nmode != kNOne || a.tb.n >= kFrontCells / kWalkCells) {  // its blocks wait for one another
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel(kernel_of(kKernelFront, a.nmode, var), dim3(room.front),
+                                    dim3(kFrontThreads), params, 0, s);
+    if (e != cudaSuccess) return e;
+  }
   const int n = a.tb.n < room.queued ? a.tb.n : room.queued;
   return cudaLaunchKernel(kernel_of(kKernelQueue, a.nmode, var), dim3(n), dim3(kWalkThreads), params,
                           sizeof(TileSmem), s);
@@ -1495,8 +1647,12 @@ cudaError_t launch_tile_rest(const StepArgs &a, const TileRoom &room, cudaStream
 cudaError_t prepare_tile_kernels(int nmode, int sms, TileRoom *room) {
   for (int k = 0; k < kKernelResident + kResidentWidths; k++) {
     if (k == kKernelPull) continue;
-    const int threads = k < kKernelResident ? kWalkThreads : kResidentThreads[k - kKernelResident];
-    const size_t bytes = k == kKernelRooted ? sizeof(RootedSmem) : sizeof(TileSmem);
+    const int threads = k >= kKernelResident ? kResidentThreads[k - kKernelResident]
+                        : k == kKernelFront  ? kFrontThreads
+                                             : kWalkThreads;
+    const size_t bytes = k == kKernelRooted ? sizeof(RootedSmem)
+                         : k == kKernelFront ? 0
+                                             : sizeof(TileSmem);
     int least = 1 << 20;
     for (int var = 0; var < 3; var++) {
       const void *f = kernel_of(k, nmode, var);
@@ -1509,6 +1665,7 @@ cudaError_t prepare_tile_kernels(int nmode, int sms, TileRoom *room) {
       least = occ < least ? occ : least;
     }
     if (k == kKernelQueue) room->queued = least * sms;
+    if (k == kKernelFront) room->front = least * sms;
     if (k >= kKernelResident) room->resident[k - kKernelResident] = least * sms;
   }
   return cudaSuccess;

@@ -112,3 +112,32 @@ def test_steeper_exponents_against_the_oracle(pkg, oracle, n, kind):
             assert np.array_equal(m.accumulation(), ref["accum"]), s
             np.testing.assert_allclose(m.getH(), ref["h"], rtol=1e-12, atol=0)
             h = ref["h"]
+
+
+@pytest.mark.parametrize("int_sub", [0, 1])
+def test_rounds_of_the_whole_gpu(pkg, oracle, int_sub):
+    """n = 1 with more than 8.4e6 cells in trees that leave their tile: nearly
+    all of the deep part's 13e6, beside young ground whose cells are pulled. A
+    batch's subset and the oracle."""
+    from oracle.pyoracle import Params
+    W, H = 4500, 3600
+    p = pkg.workload_params()
+    h = field(W, H, "young", 41)
+    hh = h.reshape(H, W)
+    hh[:, :3700] = field(3700, H, "deep", 42).reshape(H, 3700)
+    ref = h.copy()
+    for _ in range(2):
+        ref = oracle.phases(ref, W, H, Params(*p.as_tuple()))["h"]
+    small = field(70, 90, "deep", 43)
+    with pkg.FastScapeBatch([70, W], [90, H], [p, p], init=pkg.INIT_ZERO) as b:
+        b.use_int_sub(int_sub)
+        b.setH(0, small)
+        b.setH(1, h)
+        b.set_active([1])
+        b.step(2)
+        assert np.array_equal(b.getH(0), small)
+        assert np.array_equal(b.getH(1), ref)
+        b.setH(1, h)
+        b.set_active(None)
+        b.step(2)
+        assert np.array_equal(b.getH(1), ref)
