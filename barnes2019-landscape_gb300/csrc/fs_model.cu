@@ -326,10 +326,17 @@ cudaError_t reset_walk(fs_batch *b, const fs::StepArgs &a) {
 
 // The per-realization walk is on: always where the caller asked for it; where
 // the autotuner chose it, for tiles that the GPU cannot hold at once (resident
-// ones are faster: 8 realizations of eroded 512^2 0.35 against 1.6 ms).
+// ones are faster: 8 realizations of eroded 512^2 0.35 against 1.6 ms). With
+// n != 1 and realizations of at most eight tiles, the line is at blocks of 128
+// threads, whose levels of a few cells waste the FP64 pipe that a CTA's of a
+// whole realization fill: 112 of eroded 122 x 98, 896 tiles, take 0.60 against
+// 0.66 ms with n = 2 and 1.6 against 2.1 with n = 1.5 (n = 1: 0.27, 0.22); 62 of
+// them 0.60 and 0.54, 1.60 and 1.56; 37 of 250 x 190 1.9 and 1.0, 5.8 and 2.6.
 bool cta_on(const fs_batch *b) {
   const int tiles = b->act_n > 0 ? b->nwt_act : b->tb.n;
-  return b->cta_walk && (!b->cta_auto || tiles > b->room.resident[0]);
+  const bool small = b->nmode != fs::kNOne &&
+                     *std::max_element(b->size.begin(), b->size.end()) <= 8 * fs::kWalkCells;
+  return b->cta_walk && (!b->cta_auto || tiles > b->room.resident[small ? 1 : 0]);
 }
 
 // It runs for the timesteps of more than one realization.

@@ -244,8 +244,9 @@ int fs_batch_use_int_sub(fs_batch *b, int enable);
  * versions), chosen[1] = graph (fs_batch_launch_config reports every choice).
  * The per-realization walk (fs_batch_use_cta_walk) is chosen when the batch
  * has more than one realization and none has more than 2^19 cells, for
- * launches whose tiles do not all fit the GPU at once. Results do not depend
- * on the configuration. */
+ * launches whose tiles do not all fit the GPU at once (n != 1 and none of more
+ * than 2^14 cells: or fill two thirds of it). Results do not depend on the
+ * configuration. */
 int fs_batch_autotune(fs_batch *b, int probe_steps, int *chosen);
 /* The launch configuration in use: 2 and 2 (once the blocks per SM of kernels
  * that are gone), graph replay (0/1), integer subtractions in the

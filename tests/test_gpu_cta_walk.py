@@ -105,3 +105,23 @@ def test_the_autotuners_choice(pkg):
     with pkg.FastScapeBatch([256] * few, [256] * few, [p] * few, seeds=list(range(few))) as b:
         b.autotune(1)
         assert not b.launch_config()["cta_walk"]
+
+
+@pytest.mark.parametrize("w,n,cta", [(122, 1.0, False), (122, 2.0, True), (122, 1.5, True),
+                                     (300, 2.0, False)])
+def test_the_autotuners_line_for_small_realizations(pkg, w, n, cta):
+    """Tiles that fit the GPU in blocks of 128 threads only, five to an SM: for
+    n != 1 the per-realization walk if none has more than eight tiles."""
+    torch = pytest.importorskip("torch")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    per = (w + 63) // 64 * 4
+    reals = 5 * sms // per
+    p = pkg.workload_params(neq=n)
+    with pkg.FastScapeBatch([w] * reals, [98] * reals, [p] * reals, init=pkg.INIT_PHILOX,
+                            seeds=list(range(reals))) as b, \
+            pkg.FastScape_RBP(w, 98, params=p, init=pkg.INIT_PHILOX, seed=1) as m:
+        b.autotune(1)
+        assert b.launch_config()["cta_walk"] == cta
+        b.step(3)
+        m.step(3)
+        assert np.array_equal(b.getH(1), m.getH())
