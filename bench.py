@@ -70,6 +70,16 @@ ALG_BYTES = {
     # k_tile_rooted / k_tile_resident: counts, codes, planes, h read, h write
     "rest": 0.04 * (2 + 8 + 4 + 8 + 8),     # k_tile_pull: the cells left, 4%
 }
+# The same of the per-realization walk.
+CTA_ALG_BYTES = {
+    "receivers": 8 + 1,
+    "donors_level0": 1 + 1,                 # rec read, mask write (+ pit list)
+    "order": 4 + 1 + 4 + 1 + 4 + 4 + 4 + 4 + 4,
+    # k_cta_order_accum: entry and mask read, entry, direction, receiver's place
+    # and count written; count and place read, reduction into the receiver's
+    "erode": 4 + 1 + 4 + 8 + 8,
+    # k_cta_erode: entry, direction, count, h read, h write
+}
 # The erosion uses the FP64 pipe: per eroded cell fact*dh and the
 # division's one multiplication (its residual and rounding run in integer
 # arithmetic), plus h0 - hn and h0 - q unless those run in integer
@@ -84,15 +94,28 @@ FP64_PEAK_TFLOPS = 1.59 * 152 * 2.07e9 / 1e12
 STEP_ALG_BYTES = 79        # compulsory streaming bytes per cell-step with int32 receivers
 
 
-def kernel_split(t, nsteps: int) -> dict:
+def kernel_split(t, nsteps: int, cta: bool = False) -> dict:
     """Milliseconds per timestep and kernel from fs_get_phase_times."""
+    if cta:
+        return {"receivers": t[0] / nsteps, "donors_level0": t[1] / nsteps,
+                "order": t[7] / nsteps, "erode": t[8] / nsteps}
     return {"receivers": t[0] / nsteps, "drain": t[1] / nsteps, "links": t[7] / nsteps,
             "erode": t[8] / nsteps, "rest": t[9] / nsteps}
 
 
-# launches a timestep: receivers, fix-up, drain, links, then one kernel where
-# the tiles fit the GPU at once, else rooted, pull, mark, queue
-LAUNCHES_LARGE, LAUNCHES_RESIDENT = 8, 5
+def launches_per_step(shapes, n: float = 1.0, cta: bool = False) -> int:
+    """Kernels of one timestep of realizations of these (width, height):
+    receivers and fix-up, then donors, order and erosion of the
+    per-realization walk, or drain, links and one kernel where the tiles fit the
+    GPU at once (six to an SM), else rooted, pull and mark (n = 1), front (other
+    n, and from 4096 tiles on) and queue."""
+    import torch
+    tiles = sum(-(-w // 64) * -(-h // 32) for w, h in shapes if min(w, h) > 4)
+    if cta or tiles <= 6 * torch.cuda.get_device_properties(0).multi_processor_count:
+        return 5
+    if n != 1.0:
+        return 7
+    return 9 if tiles >= 4096 else 8
 
 
 def grid_config(side: int) -> dict:
@@ -397,7 +420,7 @@ def ensemble_result(pkg, n, side, nsteps, seed, rank, ws, dist, local, walk="aut
     seeds = list(range(1000 * rank, 1000 * rank + len(sides)))
     b = pkg.FastScapeBatch(sides, sides, params, init=pkg.INIT_PHILOX, seeds=seeds)
     cells = b.cells()
-    # warm-up: the autotuner's probe timesteps (9 launch configurations x 3),
+    # warm-up: the autotuner's probe timesteps (3 launch configurations x 3),
     # after which it restores the initial fields
     tune = b.autotune(probe_steps=2)
     if walk != "auto":
@@ -427,13 +450,15 @@ def ensemble_result(pkg, n, side, nsteps, seed, rank, ws, dist, local, walk="aut
     shape = "equal-size" if side > 0 else "ragged"
     side_desc = f"{side}" if side > 0 else "log-U[256,2048]"
     peak, peak_kind = load_peaks()
-    kern = kernel_split(t, 1)
-    dom = max(("receivers", "drain", "erode"), key=kern.get)
-    achieved = ALG_BYTES[dom] * cells / (kern[dom] * 1e-3) / 1e9
+    cta = bool(tune.get("cta_walk"))
+    kern = kernel_split(t, 1, cta)
+    alg = CTA_ALG_BYTES if cta else ALG_BYTES
+    dom = max((k for k in kern if k not in ("links", "rest")), key=kern.get)
+    achieved = alg[dom] * cells / (kern[dom] * 1e-3) / 1e9
     return {
         "metric": f"ensemble realizations/s ({nsteps}-timestep runs)",
         "value": ws * len(sides) / (nsteps * per_step),
-        "unit": "realizations/s", "n_gpus": ws, "steps": nsteps, "warmup": 9 * 3,
+        "unit": "realizations/s", "n_gpus": ws, "steps": nsteps, "warmup": 3 * 3,
         "ms_per_step": 1e3 * per_step, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": {"workload": f"{shape} ensemble of {len(sides)} realizations, sides "
@@ -448,9 +473,9 @@ def ensemble_result(pkg, n, side, nsteps, seed, rank, ws, dist, local, walk="aut
                    "levels_at_end": levels},
         "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "traffic": None,
-                     "alg_bytes_per_cell": ALG_BYTES[dom],
+                     "alg_bytes_per_cell": alg[dom],
                      "peak_source": f"{peak_kind} hbm_gbs", "kernel_ms": kern},
-        "gpu_launches": (LAUNCHES_RESIDENT if tune.get("cta_walk") else LAUNCHES_LARGE) * nsteps,
+        "gpu_launches": launches_per_step([(s, s) for s in sides], cta=cta) * nsteps,
         "clocks": clk.summary(),
     }
 
@@ -830,7 +855,7 @@ def run_refconst(args, dist, rank, ws, local):
                                    "field, K 2e-6 n 2 m 0.8 U 2e-3 dt 1000 dr {1, sqrt 2}",
                        "levels": levels, "launch": tune},
             "kernel_ms": kernel_split(t, args.steps),
-            "gpu_launches": LAUNCHES_LARGE * args.steps,
+            "gpu_launches": launches_per_step([(side, side)], n=2.0) * args.steps,
             "cpu_baseline": cpu,
             "clocks": clk.summary(),
         }), flush=True)
@@ -847,7 +872,7 @@ def run_deep(args, dist, rank, ws, local):
     """Long-run regime: a 512^2 grid after 2000 timesteps of strong uplift and
     erosion (K 1e-5, m 0.6, U 5e-3: ~290 levels of at most a few thousand
     cells each), where a timestep is dominated by the per-level latency of
-    the three level walks rather than by bandwidth or FP64 throughput.
+    the walk rather than by bandwidth or FP64 throughput.
     Device cell-steps/s over 10 x --steps timesteps of that state (CUDA
     events; the spin-up is untimed), with the CPU restatement of
     fastscape_RB+P timed from the same elevations."""
@@ -896,7 +921,7 @@ def run_deep(args, dist, rank, ws, local):
                                    "untimed timesteps", "levels": levels, "launch": tune},
             "kernel_ms": kernel_split(t, nsteps),
             "per_level_us": {"erode": 1e3 * t[8] / nsteps / levels},
-            "gpu_launches": LAUNCHES_RESIDENT * nsteps,
+            "gpu_launches": launches_per_step([(side, side)]) * nsteps,
             "cpu_baseline": cpu,
             "clocks": clk.summary(),
         }), flush=True)
@@ -1019,7 +1044,7 @@ def main():
     split_total_ms = float(t[3])
     cells = side * side
     value = ws * cells * args.steps / (total_ms * 1e-3)
-    launches = LAUNCHES_LARGE * args.steps
+    launches = launches_per_step([(side, side)]) * args.steps
 
     # ---- roofline of the dominant kernel ----------------------------------
     peak, peak_kind = load_peaks()
