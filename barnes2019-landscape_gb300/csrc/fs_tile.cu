@@ -1657,8 +1657,8 @@ cudaError_t prepare_tile_kernels(int nmode, int sms, TileRoom *room) {
     int least = 1 << 20;
     for (int var = 0; var < 3; var++) {
       const void *f = kernel_of(k, nmode, var);
-      cudaError_t e =
-          cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      cudaError_t e = cudaSuccess;
+      if (bytes) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
       if (e != cudaSuccess) return e;
       int occ = 0;
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, threads, bytes);

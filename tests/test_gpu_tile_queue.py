@@ -141,3 +141,22 @@ def test_rounds_of_the_whole_gpu(pkg, oracle, int_sub):
         b.set_active(None)
         b.step(2)
         assert np.array_equal(b.getH(1), ref)
+
+
+@pytest.mark.parametrize("W,H", [(8, 32000), (5, 52000)])
+@pytest.mark.parametrize("n", [1.0, 2.0])
+def test_narrow_grids_on_the_callers_buffer(pkg, W, H, n):
+    """The static scratch at its most tiles: as an allocating model."""
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    assert tiles([(W, H)]) > most_resident()
+    p = pkg.workload_params(neq=n)
+    h = field(W, H, "deep", 51)
+    d = torch.from_numpy(h.copy()).cuda()
+    f = pkg.library().fs_step_noalloc
+    f.argtypes = [C.c_void_p, C.c_int, C.c_int, C.POINTER(pkg.Params), C.c_int, C.c_void_p]
+    assert f(C.c_void_p(d.data_ptr()), W, H, C.byref(p), 3, None) == 0, pkg.last_error()
+    with pkg.FastScape_RBP(W, H, params=p, init=pkg.INIT_ZERO) as m:
+        m.setH(h)
+        m.step(3)
+        assert np.array_equal(d.cpu().numpy(), m.getH())
