@@ -930,9 +930,8 @@ fs_batch *batch_create(int n, const int *widths, const int *heights, const fs_pa
     }
   }
   if (!cu(cudaDeviceGetAttribute(&b->walk_sms, cudaDevAttrMultiProcessorCount, b->device), "attr") ||
-      !cu(fs::prepare_tile_kernels(b->nmode, b->walk_sms, &b->room), "tile kernels"))
+      !cu(fs::prepare_tile_kernels(b->nmode, b->walk_sms, b->tb.n, &b->room), "tile kernels"))
     return fail(*status);
-  if (b->room.queued < 1) return fail(set_error(FS_ERR_CUDA, "tile kernel cannot be resident"));
   b->rmap_ok = n == 1 && fs::make_receiver_map(&b->rmap, b->h, b->W[0], b->H[0], b->rrows);
   if (!cu(cudaStreamSynchronize(b->stream), "sync")) return fail(*status);
   return b;

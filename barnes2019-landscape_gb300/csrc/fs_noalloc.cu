@@ -115,9 +115,8 @@ int setup_device(int dev, DeviceState &d) {
   e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
   for (int nm = 0; nm < 3; nm++) {
-    e = fs::prepare_tile_kernels(nm, sms, &d.room[nm]);
+    e = fs::prepare_tile_kernels(nm, sms, static_cast<int>(kMaxWalkTiles), &d.room[nm]);
     if (e != cudaSuccess) return cuda_fail(e, "tile kernels");
-    if (d.room[nm].queued < 1) return fail(FS_ERR_CUDA, "tile kernel cannot be resident");
   }
   d.base = static_cast<unsigned char *>(ptr);
   d.ready = true;

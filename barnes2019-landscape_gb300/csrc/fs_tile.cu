@@ -1645,15 +1645,9 @@ cudaError_t launch_tile_rest(const StepArgs &a, const TileRoom &room, cudaStream
                           sizeof(TileSmem), s);
 }
 
-cudaError_t prepare_tile_kernels(int nmode, int sms, TileRoom *room) {
-  for (int k = 0; k < kKernelResident + kResidentWidths; k++) {
-    if (k == kKernelPull) continue;
-    const int threads = k >= kKernelResident ? kResidentThreads[k - kKernelResident]
-                        : k == kKernelFront  ? kFrontThreads
-                                             : kWalkThreads;
-    const size_t bytes = k == kKernelRooted ? sizeof(RootedSmem)
-                         : k == kKernelFront ? 0
-                                             : sizeof(TileSmem);
+cudaError_t prepare_tile_kernels(int nmode, int sms, int tiles, TileRoom *room) {
+  // blocks of kernel k on the GPU at once, whichever its arithmetic
+  auto fit = [&](int k, int threads, size_t bytes, int *blocks) -> cudaError_t {
     int least = 1 << 20;
     for (int var = 0; var < 3; var++) {
       const void *f = kernel_of(k, nmode, var);
@@ -1665,11 +1659,24 @@ cudaError_t prepare_tile_kernels(int nmode, int sms, TileRoom *room) {
       if (e != cudaSuccess) return e;
       least = occ < least ? occ : least;
     }
-    if (k == kKernelQueue) room->queued = least * sms;
-    if (k == kKernelFront) room->front = least * sms;
-    if (k >= kKernelResident) room->resident[k - kKernelResident] = least * sms;
+    *blocks = least * sms;
+    return *blocks > 0 ? cudaSuccess : cudaErrorLaunchOutOfResources;
+  };
+  for (int w = kResidentWidths - 1; w >= 0; w--) {
+    const cudaError_t e =
+        fit(kKernelResident + w, kResidentThreads[w], sizeof(TileSmem), &room->resident[w]);
+    if (e != cudaSuccess) return e;
+    if (tiles <= room->resident[w]) {  // no launch needs narrower blocks, or the kernels below
+      for (int v = 0; v < w; v++) room->resident[v] = room->resident[w];
+      return cudaSuccess;
+    }
   }
-  return cudaSuccess;
+  int any = 0;
+  cudaError_t e = fit(kKernelRooted, kRootedThreads, sizeof(RootedSmem), &any);
+  if (e == cudaSuccess && (nmode != kNOne || tiles >= kFrontCells / kWalkCells))
+    e = fit(kKernelFront, kFrontThreads, 0, &room->front);
+  if (e == cudaSuccess) e = fit(kKernelQueue, kWalkThreads, sizeof(TileSmem), &room->queued);
+  return e;
 }
 
 }  // namespace fs
