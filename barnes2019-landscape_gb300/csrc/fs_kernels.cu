@@ -585,9 +585,9 @@ __global__ void __launch_bounds__(256) k_donors_level0(StepArgs a) {
 // Per-realization level walk, the timestep of batches of many small
 // realizations late in a long run, whose tiles do not fit the GPU at once.
 // There the tile walk (fs_tile.cu) finds narrow levels, some 30 cells of a
-// tile, and revisits each tile five times from its queue (256 realizations of
-// eroded 512^2: 9.4 ms); one CTA that walks a whole realization's levels, some
-// 1000 cells wide, with block barriers only, keeps its threads busy. Same
+// tile, and takes most cells in rounds of the whole GPU (256 realizations of
+// eroded 512^2: 7.5 ms); one CTA that walks a whole realization's levels, some
+// 1000 cells wide, with block barriers only, keeps its threads busy (3.6). Same
 // per-cell arithmetic, counts and elevations bit for bit.
 //   k_cta_order_accum: level ordering (fastscape_RB.cpp:213-254: level k+1 =
 //     the donors of level k, each entry's donors contiguous in direction

@@ -152,7 +152,7 @@ struct fs_batch {
   cudaGraphExec_t graph = nullptr;
   bool graph_dirty = true;
   std::vector<cudaEvent_t> ev;
-  double phase_ms[FS_NUM_TIMERS] = {};  // event timers (indices 0-3, 7, 8)
+  double phase_ms[FS_NUM_TIMERS] = {};  // event timers (harvest_events)
   // Active subset (fs_batch_set_active): act_n > 0 steps only the
   // realizations act_idx through descriptors and tile lists of their own
   // (the per-cell arrays are shared); act_n == 0 steps all.

@@ -458,8 +458,8 @@ __global__ void __launch_bounds__(256) k_tile_links(StepArgs a) {
 // meet at a barrier of their own. On young ground one level holds half of a
 // tile: where the SMs have room for wider blocks, more warps sleep at another
 // barrier and help with the levels wider than two rounds of the first three
-// (100^2: 70 -> 57 us a timestep, 1000^2: 96 -> 87), which deep ground's narrow
-// levels do not wait for. What takes time is the chain of one cell's
+// (100^2: 70 -> 57 us a timestep, 1000^2: 96 -> 87; with the steps after it 54
+// and 82), which deep ground's narrow levels do not wait for. What takes time is the chain of one cell's
 // arithmetic after its receiver's elevation is known (64 clocks for an FP64
 // operation, four to eight of them, and the quotient's integer steps), once a
 // level: everything else of a cell -- its elevation, count, table record, an
