@@ -70,8 +70,10 @@ constexpr int kFrontRounds = 16;
 // n != 1: a tile's levels narrower than this are left to k_tile_front, which
 // has full warps for them. n = 2: 7.00 -> 6.85 ms at 48 (96: 6.80, but 13.5
 // instead of 12.7 at 515 levels; 192: 7.07). Other n, whose cells take five times
-// as long: 35.7 -> 34.5 at 192 (48: 34.8, 400: 34.6, every level: 35.1).
-constexpr int kRootedFewTwo = 48, kRootedFewGeneral = 192;
+// as long: 35.7 -> 34.5 at 192 (48: 34.8, 400: 34.6, every level: 35.1), and
+// every level where the tiles come in few waves (672 x 4422, 1518 tiles, 1.44 ->
+// 1.39; 1500^2 1.15 -> 1.09; 3000^2, 4418 tiles, 3.41 -> 3.52).
+constexpr int kRootedFewTwo = 48, kRootedFewGeneral = 192, kRootedWaves = 4096;
 static_assert(kWalkW == 64 && kWalkH == 32, "a cell's tile: x >> 6, y >> 5");
 constexpr uint32_t kNoSink = 0xFFFFu;
 constexpr int kFinished = 1 << 30;
@@ -1123,7 +1125,9 @@ __global__ void __launch_bounds__(kRootedThreads, 6) k_tile_rooted(StepArgs a) {
   for (int L = 1;; ++L) {
     const int lo = s.end[(L - 1) & 3], hi = s.end[L & 3], hi2 = s.end[(L + 1) & 3];
     if (lo == hi) break;
-    if (kRounds && hi - lo < (NMODE == kNTwo ? kRootedFewTwo : kRootedFewGeneral)) {  // k_tile_front's from here on
+    if (kRounds && (hi - lo < (NMODE == kNTwo ? kRootedFewTwo : kRootedFewGeneral) ||
+                    (NMODE == kNGeneral && gridDim.x < kRootedWaves))) {
+      // k_tile_front's from here on
       if (wid == 0) final &= ~(F | F1);
       break;
     }

@@ -114,6 +114,21 @@ def test_steeper_exponents_against_the_oracle(pkg, oracle, n, kind):
             h = ref["h"]
 
 
+def test_general_exponent_on_many_tiles(pkg, oracle):
+    """From 4096 tiles on, a general n's wide levels are eroded in their tiles."""
+    from oracle.pyoracle import Params
+    W, H = 2100, 4100
+    assert tiles([(W, H)]) > 4096
+    p = pkg.workload_params(neq=1.5)
+    h = field(W, H, "young", 33)
+    ref = oracle.phases(h.copy(), W, H, Params(*p.as_tuple()))
+    with pkg.FastScape_RBP(W, H, params=p, init=pkg.INIT_ZERO) as m:
+        m.setH(h)
+        m.step(1)
+        assert np.array_equal(m.accumulation(), ref["accum"])
+        np.testing.assert_allclose(m.getH(), ref["h"], rtol=1e-12, atol=0)
+
+
 @pytest.mark.parametrize("int_sub", [0, 1])
 def test_rounds_of_the_whole_gpu(pkg, oracle, int_sub):
     """n = 1 with more than 8.4e6 cells in trees that leave their tile: nearly
